@@ -456,7 +456,7 @@ PP_API int pp_set_medium(pp_ctx* ctx, const pp_medium* m) {
   cudaFree(ctx->d_es_table);
   ctx->d_es_table = nullptr;
   if (phase.kind == PP_PHASE_HG_ES && m->hg_weight < 1.0f) {
-    std::vector<float2> es(pp::kEsTable);
+    std::vector<float2> es(pp::kEsTable + 1);
     pp::make_es_table(phase.es_b, es.data());
     PP_CUDA(cudaMalloc(&ctx->d_es_table, sizeof(float2) * es.size()), "cudaMalloc(ES table)");
     PP_CUDA(cudaMemcpy(ctx->d_es_table, es.data(), sizeof(float2) * es.size(),

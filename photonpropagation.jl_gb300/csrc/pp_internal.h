@@ -106,9 +106,11 @@ struct PhaseDev {
   float es_b;       // Einstein-Smoluchowski b
   int kind;         // PP_PHASE_*
   float sl_exp;     // simplified Liu: (1 - g) / (1 + g)
+  // u = ((w >> 8) + 1) 2^-24 < hg_weight as a compare of the random word: w < hg_words
+  uint32_t hg_words;
   // Einstein-Smoluchowski inverse CDF for the fast kernel: kEsTable intervals
-  // of eta on [0, 1], entry i = {q(i / N), q((i + 1) / N) - q(i / N)} (set by
-  // pp_set_medium; null: the Cardano formula)
+  // of eta on [0, 1], entry i = {q(i / N), q((i + 1) / N) - q(i / N)}, then one
+  // entry {q(1), 0} (set by pp_set_medium; null: the Cardano formula)
   const float2* es_table;
 };
 
@@ -116,9 +118,11 @@ struct PhaseDev {
 // smooth on [0, 1] (its derivative is 1 / pdf, and pdf ~ 1 + b cos^2 is
 // bounded away from 0), so linear interpolation on 1024 intervals is exact to
 // ~1e-7, below the SFU cube roots of the formula it replaces.
-constexpr int kEsTable = 1024;
+constexpr int kEsTableBits = 10;
+constexpr int kEsTable = 1 << kEsTableBits;
 
-// The table of PhaseDev::es_table for parameter b, in double and rounded once:
+// The table of PhaseDev::es_table for parameter b (kEsTable + 1 entries), in
+// double and rounded once:
 // q = cbrt(Q + D) + cbrt(Q - D), Q = (b + 3)(eta - 1/2) / b, D = sqrt(Q^2 + 1/b^3)
 // (the Cardano root of the ES CDF's cubic, as the replay kernel evaluates it).
 inline void make_es_table(float b, float2* out) {
@@ -131,6 +135,9 @@ inline void make_es_table(float b, float2* out) {
     if (i > 0) out[i - 1] = make_float2((float)prev, (float)(v - prev));
     prev = v;
   }
+  // eta = 1: the last interval's end, as its interpolation rounds
+  const float2 e = out[kEsTable - 1];
+  out[kEsTable] = make_float2((float)((double)e.x + (double)e.y), 0.0f);
 }
 
 // The phase function of a medium, validated: nullptr on success, else the
@@ -157,6 +164,9 @@ inline const char* make_phase(const pp_medium* m, PhaseDev* p) {
   p->es_b = b;
   p->kind = m->phase_kind;
   p->sl_exp = (1.0f - g) / (1.0f + g);
+  // k 2^-24 < hg_weight, k = (w >> 8) + 1 in 1 .. 2^24
+  const double c = std::ceil((double)m->hg_weight * 16777216.0);
+  p->hg_words = c >= 1.0 ? ((uint32_t)c - 1u) << 8 : 0u;
   return nullptr;
 }
 

@@ -199,9 +199,9 @@ __device__ __forceinline__ int check_queue(WarpQueue& q, int n2, int n1, const G
     d = make_float3(q.dx[src], q.dy[src], q.dz[src]);
     L = q.len[src];
     // slab test against the grid box (the same one the walk clips to)
-    const float ix = approx_rcp(fabsf(d.x) > 1e-20f ? d.x : 1e-20f);
-    const float iy = approx_rcp(fabsf(d.y) > 1e-20f ? d.y : 1e-20f);
-    const float iz = approx_rcp(fabsf(d.z) > 1e-20f ? d.z : 1e-20f);
+    const float ix = ftz_rcp(fabsf(d.x) > 1e-20f ? d.x : 1e-20f);
+    const float iy = ftz_rcp(fabsf(d.y) > 1e-20f ? d.y : 1e-20f);
+    const float iz = ftz_rcp(fabsf(d.z) > 1e-20f ? d.z : 1e-20f);
     const float tx0 = (g.lo[0] - p.x) * ix, tx1 = (g.hi[0] - p.x) * ix;
     const float ty0 = (g.lo[1] - p.y) * iy, ty1 = (g.hi[1] - p.y) * iy;
     const float tz0 = (g.lo[2] - p.z) * iz, tz1 = (g.hi[2] - p.z) * iz;
@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(kMaxBlockThreads, PP_PROPAGATE_MIN_BLOCKS)
           comp = (t - dist) - y;
           dist = t;
         }
-        dir = update_direction<kPrecise>(a.phase, dir, u01(r.y), u01(r.z), u01(r.w));
+        dir = update_direction<kPrecise>(a.phase, dir, r.y, r.z, r.w);
       }
       if (kShapes) break;
       if (flush && n1 > 0) {

@@ -261,7 +261,7 @@ extern "C" PP_API int pp_propagate_static(
   // the fast kernel's tabulated ES inverse CDF, as pp_set_medium makes it
   std::vector<float2> es;
   if (phase.kind == PP_PHASE_HG_ES && medium->hg_weight < 1.0f) {
-    es.resize(pp::kEsTable);
+    es.resize(pp::kEsTable + 1);
     pp::make_es_table(phase.es_b, es.data());
   }
 
