@@ -237,15 +237,11 @@ int rebuild_grid(pp_ctx* ctx, float cell_size) {
   ctx->grid = g;
   ctx->d_blob = blob;
   ctx->n_items = n_items;
-  // Safety field over the same box; automatic cell: about 32k cells (32 KiB).
+  // Safety field over the same box.
   cudaFree(ctx->d_safety);
   ctx->d_safety = nullptr;
   float hs = ctx->tuning.safety_cell;
-  if (!(hs > 0.0f)) {
-    double vol = 1.0;
-    for (int a = 0; a < 3; ++a) vol *= std::max(1e-6, (double)g.hi[a] - (double)g.lo[a]);
-    hs = (float)std::max(1e-3, std::cbrt(vol / 32768.0));
-  }
+  if (!(hs > 0.0f)) hs = (float)pp::SafetyDev::auto_cell(g.lo, g.hi);
   pp::SafetyDev sg{};
   unsigned char* field = nullptr;
   if (pp::build_safety(ctx->d_targets, n, g, hs, ctx->stream, &sg, &field, &err) != 0)

@@ -132,7 +132,7 @@ __global__ void pack_kernel(const unsigned* __restrict__ counts, const unsigned*
   }
 }
 
-// One thread per safety cell: min over spheres of |c - s| - r - margin,
+// One thread per safety node: min over spheres of |c - s| - r - margin,
 // floored to the quantum.  Targets are staged through shared memory.
 __global__ void safety_kernel(const SafetyDev sg, const pp_sphere* __restrict__ t, int n,
                               unsigned char* __restrict__ out) {
@@ -143,9 +143,9 @@ __global__ void safety_kernel(const SafetyDev sg, const pp_sphere* __restrict__ 
     const int x = i % sg.dims[0];
     const int y = (i / sg.dims[0]) % sg.dims[1];
     const int z = i / (sg.dims[0] * sg.dims[1]);
-    cx = sg.lo[0] + (x + 0.5f) * sg.cell;
-    cy = sg.lo[1] + (y + 0.5f) * sg.cell;
-    cz = sg.lo[2] + (z + 0.5f) * sg.cell;
+    cx = sg.lo[0] + x * sg.cell;
+    cy = sg.lo[1] + y * sg.cell;
+    cz = sg.lo[2] + z * sg.cell;
   }
   float best = 1e30f;
   for (int base = 0; base < n; base += 256) {
@@ -351,26 +351,7 @@ int build_safety(const pp_sphere* targets_dev, int n, const GridDev& grid, float
                  cudaStream_t stream, SafetyDev* out, unsigned char** field_out, std::string* err) {
   *field_out = nullptr;
   SafetyDev sg{};
-  double h = cell > 0.0f ? cell : 12.5;
-  double ext[3];
-  for (int a = 0; a < 3; ++a) ext[a] = (double)grid.hi[a] - (double)grid.lo[a];
-  for (int guard = 0; guard < 64; ++guard) {
-    double cells = 1.0;
-    for (int a = 0; a < 3; ++a) cells *= std::max(1.0, std::ceil(ext[a] / h));
-    if (cells <= 16.0 * 1024 * 1024) break;
-    h *= 1.25;
-  }
-  sg.n_cells = 1;
-  for (int a = 0; a < 3; ++a) {
-    sg.dims[a] = (int)std::max(1.0, std::ceil(ext[a] / h));
-    sg.lo[a] = grid.lo[a];
-    sg.hi[a] = (float)((double)grid.lo[a] + sg.dims[a] * h);
-    sg.n_cells *= sg.dims[a];
-  }
-  sg.cell = (float)h;
-  sg.inv_cell = (float)(1.0 / h);
-  sg.bytes = (uint32_t)(((size_t)sg.n_cells + 15) & ~(size_t)15);
-  sg.set_derived();
+  sg.set_shape(grid.lo, grid.hi, cell > 0.0f ? cell : 12.5);
   unsigned char* f = nullptr;
   if (cudaMalloc(&f, (size_t)sg.bytes) != cudaSuccess) {
     if (err) *err = "cudaMalloc(safety field) failed";

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <string>
@@ -32,39 +33,78 @@ struct GridDev {
   uint32_t blob_bytes;   // multiple of 16
 };
 
-// Safety field: a coarser-or-finer uniform grid over the same box whose cell
-// value is a lower bound on the distance from the cell centre to the nearest
-// (inflated) sphere surface, quantised down in kSafetyQuantum steps (uint8).
-// A step segment lies inside the ball of radius L/2 about its midpoint m; if
-// D(centre) - |m - centre| > L/2 (1-Lipschitz) no sphere can be hit.
+// Safety field: a uniform grid of nodes lo + i * cell over a box that contains
+// every (inflated) sphere; a node holds a lower bound of its distance to the
+// nearest sphere surface, quantised down in kSafetyQuantum steps (uint8).  For
+// a point m with projection m' onto the box and the node c nearest to m',
+// every sphere is at least sqrt(|m - m'|^2 + w^2) away, w = max(D(c) - |m' - c|, 0):
+// the distance to the spheres is 1-Lipschitz, and a convex box seen from
+// outside lies behind its nearest point.
 struct SafetyDev {
   float lo[3];
   float hi[3];
-  float cell;      // edge (m), cubic cells
+  float cell;      // node spacing (m), the same on every axis
   float inv_cell;
-  int dims[3];
-  int n_cells;
+  int dims[3];     // nodes per axis, >= 2
+  int n_cells;     // nodes, < 2^23
   uint32_t bytes;  // allocation, n_cells rounded up to 16 (padding bytes are 0)
   // Derived on the host (set_derived) so that the kernel's tests read them
-  // as constant operands instead of converting dims or re-adding offsets.
+  // as constant operands; the tests work in units of the spacing.
   float fdims[3];  // dims as float
-  float fmaxc[3];  // dims - 1 as float (largest cell coordinate)
+  float fmaxc[3];  // dims - 1 as float (largest node coordinate)
   float lo_sc[3];  // lo * inv_cell
-  float c_lo[3];   // centre of cell 0: lo + cell / 2
-  float bc[3];     // centre of the field's box
-  float he[3];     // half extents of the field's box
-  void set_derived() {
-    for (int a = 0; a < 3; ++a) {
-      fdims[a] = (float)dims[a];
-      fmaxc[a] = (float)(dims[a] - 1);
-      lo_sc[a] = lo[a] * inv_cell;
-      c_lo[a] = lo[a] + 0.5f * cell;
-      bc[a] = 0.5f * (lo[a] + hi[a]);
-      he[a] = 0.5f * (hi[a] - lo[a]);
-    }
-  }
+  float quantum;   // kSafetyQuantum * inv_cell
+  float r_scale;   // ball radius in spacings = r_scale * (half the segment) + r_slack:
+  float r_slack;   // 1e-4 relative and 0.1 mm above it
+  void set_derived();
+  // Nodes of spacing h (m, made coarser if they would be too many) over the
+  // box [blo, bhi].
+  void set_shape(const float* blo, const float* bhi, double h);
+  // The automatic spacing: about 32k nodes (32 KiB).
+  static double auto_cell(const float* blo, const float* bhi);
 };
 constexpr float kSafetyQuantum = 0.5f;  // m per uint8 step (saturates at 127.5 m)
+
+inline void SafetyDev::set_derived() {
+  for (int a = 0; a < 3; ++a) {
+    fdims[a] = (float)dims[a];
+    fmaxc[a] = (float)(dims[a] - 1);
+    lo_sc[a] = lo[a] * inv_cell;
+  }
+  quantum = kSafetyQuantum * inv_cell;
+  r_scale = 1.0001f * inv_cell;
+  r_slack = 1e-4f * inv_cell;
+}
+
+inline double safety_nodes(const float* blo, const float* bhi, double h) {
+  double n = 1.0;
+  for (int a = 0; a < 3; ++a)
+    n *= std::ceil(std::max(1e-6, (double)bhi[a] - (double)blo[a]) / h) + 1.0;
+  return n;
+}
+
+inline void SafetyDev::set_shape(const float* blo, const float* bhi, double h) {
+  for (int guard = 0; guard < 64 && safety_nodes(blo, bhi, h) > 8.0e6; ++guard) h *= 1.25;
+  n_cells = 1;
+  for (int a = 0; a < 3; ++a) {
+    dims[a] = (int)std::ceil(std::max(1e-6, (double)bhi[a] - (double)blo[a]) / h) + 1;
+    lo[a] = blo[a];
+    hi[a] = (float)((double)blo[a] + (dims[a] - 1) * h);
+    n_cells *= dims[a];
+  }
+  cell = (float)h;
+  inv_cell = (float)(1.0 / h);
+  bytes = (uint32_t)(((size_t)n_cells + 15) & ~(size_t)15);
+  set_derived();
+}
+
+inline double SafetyDev::auto_cell(const float* blo, const float* bhi) {
+  double vol = 1.0;
+  for (int a = 0; a < 3; ++a) vol *= std::max(1e-6, (double)bhi[a] - (double)blo[a]);
+  double h = std::max(1e-3, std::cbrt(vol / 32768.0));
+  for (int guard = 0; guard < 512 && safety_nodes(blo, bhi, h) > 34000.0; ++guard) h *= 1.02;
+  return h;
+}
 
 // Per-warp shared-memory state of the propagation kernel: the queue of
 // deferred step segments and, per lane, the earliest hit found so far.

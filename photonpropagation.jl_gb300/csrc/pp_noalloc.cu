@@ -92,7 +92,7 @@ long long scaled_photons(long long photons, float scaling) {
   return (long long)floorf(x);
 }
 
-// Grid and safety-field shapes from the host copy of the targets, with the
+// Grid shape from the host copy of the targets, with the
 // same box, automatic cell sizes and limits as pp_set_targets.
 void grid_shape(const pp_sphere* t, int n, float cell_size, pp::GridDev* g) {
   *g = pp::GridDev{};
@@ -133,33 +133,6 @@ void grid_shape(const pp_sphere* t, int n, float cell_size, pp::GridDev* g) {
     g->hi[a] = (float)((double)bb[a] + g->dims[a] * h);
     g->n_cells *= g->dims[a];
   }
-}
-
-void safety_shape(const pp::GridDev& g, pp::SafetyDev* s) {
-  *s = pp::SafetyDev{};
-  double ext[3], vol = 1.0;
-  for (int a = 0; a < 3; ++a) {
-    ext[a] = std::max(1e-6, (double)g.hi[a] - (double)g.lo[a]);
-    vol *= ext[a];
-  }
-  double h = std::max(1e-3, std::cbrt(vol / 32768.0));
-  for (int guard = 0; guard < 64; ++guard) {
-    double cells = 1.0;
-    for (int a = 0; a < 3; ++a) cells *= std::max(1.0, std::ceil(ext[a] / h));
-    if (cells <= 16.0 * 1024 * 1024) break;
-    h *= 1.25;
-  }
-  s->n_cells = 1;
-  for (int a = 0; a < 3; ++a) {
-    s->dims[a] = (int)std::max(1.0, std::ceil(ext[a] / h));
-    s->lo[a] = g.lo[a];
-    s->hi[a] = (float)((double)g.lo[a] + s->dims[a] * h);
-    s->n_cells *= s->dims[a];
-  }
-  s->cell = (float)h;
-  s->inv_cell = (float)(1.0 / h);
-  s->bytes = (uint32_t)(((size_t)s->n_cells + 15) & ~(size_t)15);
-  s->set_derived();
 }
 
 // Upper bound of the grid's item count from the host copy of the targets.
@@ -241,7 +214,7 @@ extern "C" PP_API int pp_propagate_static(
   pp::GridDev gshape;
   grid_shape(targets, n_targets, cell_size, &gshape);
   pp::SafetyDev sshape;
-  safety_shape(gshape, &sshape);
+  sshape.set_shape(gshape.lo, gshape.hi, pp::SafetyDev::auto_cell(gshape.lo, gshape.hi));
   const int ppt = 8, block = 1024;
   const long long chunk = 32LL * ppt;
   std::vector<unsigned long long> prefix(n_src + 1, 0);
