@@ -55,6 +55,91 @@ __device__ __forceinline__ uint4 philox(uint4 c, const uint32_t* __restrict__ rk
   return c;
 }
 
+// The steps of one photon share most of rounds 1 and 2: with counter (plo,
+// phi, k, s), the products with plo and s-mixed words do not depend on the
+// step k, and those with k and phi not on the photon's low word.  A photon
+// keeps three words, a step computes three for the whole warp (phi is equal
+// in a group of photons), and each (photon, step) starts at round 3.
+struct PhiloxPhoton {
+  uint32_t a, b, c;
+};
+struct PhiloxStep {
+  uint32_t lo1, hi, lo;
+};
+__device__ __forceinline__ PhiloxPhoton philox_photon(uint32_t plo, uint32_t s,
+                                                      const uint32_t* __restrict__ rk) {
+  const unsigned long long p0 = (unsigned long long)kPhiloxM0 * plo;
+  const unsigned long long p1 =
+      (unsigned long long)kPhiloxM1 * ((uint32_t)(p0 >> 32) ^ s ^ rk[1]);
+  return {(uint32_t)(p1 >> 32) ^ rk[2], (uint32_t)p1, (uint32_t)p0 ^ rk[3]};
+}
+__device__ __forceinline__ PhiloxStep philox_step(uint32_t k, uint32_t phi,
+                                                  const uint32_t* __restrict__ rk) {
+  const unsigned long long p1 = (unsigned long long)kPhiloxM1 * k;
+  const unsigned long long p0 =
+      (unsigned long long)kPhiloxM0 * ((uint32_t)(p1 >> 32) ^ phi ^ rk[0]);
+  return {(uint32_t)p1, (uint32_t)(p0 >> 32), (uint32_t)p0};
+}
+// philox(make_uint4(plo, phi, k, s), rk)
+__device__ __forceinline__ uint4 philox_words(const PhiloxPhoton& p, const PhiloxStep& t,
+                                              const uint32_t* __restrict__ rk) {
+  uint4 c = make_uint4(p.a ^ t.lo1, p.b, t.hi ^ p.c, t.lo);
+#pragma unroll
+  for (int r = 2; r < 10; ++r) {
+    const unsigned long long p0 = (unsigned long long)kPhiloxM0 * c.x;
+    const unsigned long long p1 = (unsigned long long)kPhiloxM1 * c.z;
+    c = make_uint4((uint32_t)(p1 >> 32) ^ c.y ^ rk[2 * r], (uint32_t)p1,
+                   (uint32_t)(p0 >> 32) ^ c.w ^ rk[2 * r + 1], (uint32_t)p0);
+  }
+  return c;
+}
+
+// ---- two photons at a time ---------------------------------------------------
+// A lane of the propagation kernel carries two photons, and their FP32 sums
+// and products go through the packed f32x2 instructions: each half rounds as
+// the scalar instruction does, at the same FP32 rate, in half the issue slots
+// (measured on the GB300: 16 FFMA + 16 LOP3 take 37.4 issue cycles, 8 packed
+// FFMA + 16 LOP3 28.8).
+__device__ __forceinline__ unsigned long long pack2(float2 v) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(v.x), "f"(v.y));
+  return d;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(v));
+  return d;
+}
+__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(pack2(a)), "l"(pack2(b)), "l"(pack2(c)));
+  return unpack2(d);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pack2(a)), "l"(pack2(b)));
+  return unpack2(d);
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pack2(a)), "l"(pack2(b)));
+  return unpack2(d);
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pack2(a)), "l"(pack2(b)));
+  return unpack2(d);
+}
+struct Vec2 {  // the two photons' vectors
+  float2 x, y, z;
+};
+__device__ __forceinline__ float3 first(const Vec2& v) { return make_float3(v.x.x, v.y.x, v.z.x); }
+__device__ __forceinline__ float3 second(const Vec2& v) { return make_float3(v.x.y, v.y.y, v.z.y); }
+__device__ __forceinline__ Vec2 both(float3 a, float3 b) {
+  return {make_float2(a.x, b.x), make_float2(a.y, b.y), make_float2(a.z, b.z)};
+}
+
 // 24-bit uniform in (0, 1] (exact: integer <= 2^24 times 2^-24).
 __device__ __forceinline__ float u01(uint32_t x) {
   return __uint2float_rn((x >> 8) + 1u) * 5.9604644775390625e-8f;
@@ -282,38 +367,46 @@ __device__ __forceinline__ float scatter_cos_precise(const pp::PhaseDev& ph, uin
   return u_choice < ph.hg_weight ? hg : other;
 }
 
-// The fast variant works on the 24-bit integers of the uniforms where that is
-// exact and cheaper than forming u = k 2^-24 first: the choice is one integer
-// compare (PhaseDev::hg_words), 2 eta - 1 = k 2^-23 - 1, and the interval and
-// fraction of the tabulated Einstein-Smoluchowski root (PhaseDev::es_table)
-// are k's upper and lower bits (no float-to-integer conversions, which take
-// the quarter-rate pipe).  Same values bit for bit.
-__device__ __forceinline__ float scatter_cos_fast(const pp::PhaseDev& ph, uint32_t wc,
-                                                  uint32_t we) {
-  const uint32_t ke = (we >> 8) + 1u;  // eta = ke 2^-24
-  const float kf = __uint2float_rn(ke);
+// The fast variant takes two photons (words we.x and we.y are theirs) and
+// works on the 24-bit integers of the uniforms where that is exact and cheaper
+// than forming u = k 2^-24 first: the choice is one integer compare
+// (PhaseDev::hg_words), 2 eta - 1 = k 2^-23 - 1, and the interval and fraction
+// of the tabulated Einstein-Smoluchowski root (PhaseDev::es_table) are k's
+// upper and lower bits (no float-to-integer conversions, which take the
+// quarter-rate pipe).  Same values bit for bit.
+__device__ __forceinline__ float es_root(const pp::PhaseDev& ph, uint32_t ke) {
+  constexpr int kShift = 24 - pp::kEsTableBits;
+  const float2 e = __ldg(reinterpret_cast<const float2*>(
+      reinterpret_cast<const char*>(ph.es_table) + ((ke >> kShift) << 3)));
+  // low bits as a fraction: 2^23 + l through the bit pattern, then l 2^-shift
+  const float l = __uint_as_float(0x4B000000u | (ke & ((1u << kShift) - 1u)));
+  constexpr float kFrac = 1.0f / (float)(1 << kShift);
+  return fmaf(fmaf(l, kFrac, -8388608.0f * kFrac), e.y, e.x);
+}
+__device__ __forceinline__ float second_component(const pp::PhaseDev& ph, float kf) {
+  const float eta = kf * 5.9604644775390625e-8f;
+  // (a subnormal power and its logarithm round away against the 1)
+  if (ph.kind == PP_PHASE_HG_SL) return fmaf(2.0f, ftz_ex2(ph.sl_exp * ftz_lg2(eta)), -1.0f);
+  const float q = ph.es_k1 * (eta - 0.5f);
+  const float d = approx_sqrt(fmaf(q, q, ph.es_k2));
+  return f_cbrt_pos<false>(q + d) - f_cbrt_pos<false>(d - q);
+}
+__device__ __forceinline__ float2 scatter_cos_fast(const pp::PhaseDev& ph, uint2 wc, uint2 we) {
+  const uint32_t k0 = (we.x >> 8) + 1u, k1 = (we.y >> 8) + 1u;  // eta = k 2^-24
+  const float2 kf = make_float2(__uint2float_rn(k0), __uint2float_rn(k1));
   // (1 + g (2 eta - 1) lies in [1 - |g|, 1 + |g|]: normal)
-  const float t =
-      ph.hg_1mg2 * ftz_rcp(fmaf(ph.hg_g, fmaf(kf, 1.1920928955078125e-7f, -1.0f), 1.0f));
-  const float hg = fminf(fmaxf(fmaf(-t, t, ph.hg_1pg2) * ph.hg_inv2g, -1.0f), 1.0f);
-  float other;
-  if (ph.kind == PP_PHASE_HG_SL) {
-    // (a subnormal power and its logarithm round away against the 1)
-    other = fmaf(2.0f, ftz_ex2(ph.sl_exp * ftz_lg2(kf * 5.9604644775390625e-8f)), -1.0f);
-  } else if (ph.es_table) {
-    constexpr int kShift = 24 - pp::kEsTableBits;
-    const float2 e = __ldg(reinterpret_cast<const float2*>(
-        reinterpret_cast<const char*>(ph.es_table) + ((ke >> kShift) << 3)));
-    // low bits as a fraction: 2^23 + l through the bit pattern, then l 2^-shift
-    const float l = __uint_as_float(0x4B000000u | (ke & ((1u << kShift) - 1u)));
-    constexpr float kFrac = 1.0f / (float)(1 << kShift);
-    other = fmaf(fmaf(l, kFrac, -8388608.0f * kFrac), e.y, e.x);
-  } else {
-    const float q = ph.es_k1 * (kf * 5.9604644775390625e-8f - 0.5f);
-    const float d = approx_sqrt(fmaf(q, q, ph.es_k2));
-    other = f_cbrt_pos<false>(q + d) - f_cbrt_pos<false>(d - q);
-  }
-  return wc < ph.hg_words ? hg : other;
+  const float2 v = fma2(dup2(ph.hg_g), fma2(kf, dup2(1.1920928955078125e-7f), dup2(-1.0f)),
+                        dup2(1.0f));
+  const float2 t = mul2(dup2(ph.hg_1mg2), make_float2(ftz_rcp(v.x), ftz_rcp(v.y)));
+  // (1 + g^2 - t^2) / 2g with both factors' signs turned
+  const float2 h = mul2(fma2(t, t, dup2(ph.hg_n1pg2)), dup2(ph.hg_ninv2g));
+  float2 other;
+  if (ph.es_table)
+    other = make_float2(es_root(ph, k0), es_root(ph, k1));
+  else
+    other = make_float2(second_component(ph, kf.x), second_component(ph, kf.y));
+  return make_float2(wc.x < ph.hg_words ? fminf(fmaxf(h.x, -1.0f), 1.0f) : other.x,
+                     wc.y < ph.hg_words ? fminf(fmaxf(h.y, -1.0f), 1.0f) : other.y);
 }
 
 // Back onto the unit sphere, for the fast variant: its SFU sine, cosine and
@@ -329,23 +422,58 @@ __device__ __forceinline__ float3 renormalise(float3 d) {
 }
 
 // The new direction from the step's three random words (choice, eta, azimuth).
-template <bool P>
-__device__ __forceinline__ float3 update_direction(const pp::PhaseDev& ph, float3 dir, uint32_t wc,
-                                                   uint32_t we, uint32_t wp) {
-  if (P) {
-    const float c = scatter_cos_precise(ph, wc, we);
-    const float s2 = 1.0f - c * c;
-    const float st = f_sqrt<true>(s2 > 0.0f ? s2 : 0.0f);
-    const float phi = uniform_ab(0.0f, kTwoPi, u01(wp));
-    return rot_from_ez<true>(dir, make_float3(cosf(phi) * st, sinf(phi) * st, c));
-  }
-  const float c = scatter_cos_fast(ph, wc, we);
-  // 1 - c^2 is 0 or at least 2^-24
-  const float st = ftz_sqrt(fmaxf(fmaf(-c, c, 1.0f), 0.0f));
+// Replay variant.
+__device__ __forceinline__ float3 update_direction_precise(const pp::PhaseDev& ph, float3 dir,
+                                                           uint32_t wc, uint32_t we, uint32_t wp) {
+  const float c = scatter_cos_precise(ph, wc, we);
+  const float s2 = 1.0f - c * c;
+  const float st = f_sqrt<true>(s2 > 0.0f ? s2 : 0.0f);
+  const float phi = uniform_ab(0.0f, kTwoPi, u01(wp));
+  return rot_from_ez<true>(dir, make_float3(cosf(phi) * st, sinf(phi) * st, c));
+}
+
+// Fast variant, two photons: each half rounds as renormalise(rot_from_ez<false>(
+// dir, (cos(2 pi u) st, sin(2 pi u) st, c))) of that photon; where a packed
+// operand is needed negated, an exact sign change takes the place of the scalar
+// instruction's operand modifier.
+__device__ __forceinline__ Vec2 update_direction_fast(const pp::PhaseDev& ph, const Vec2& a,
+                                                      uint2 wc, uint2 we, uint2 wp) {
+  const float2 c = scatter_cos_fast(ph, wc, we);
+  // 1 - c^2 (with its sign turned; it is 0 or at least 2^-24)
+  const float2 n2 = fma2(c, c, dup2(-1.0f));
+  const float2 st = make_float2(ftz_sqrt(fmaxf(-n2.x, 0.0f)), ftz_sqrt(fmaxf(-n2.y, 0.0f)));
   // 2 pi u - pi with u = k 2^-24, the scale folded into the constant (f_sincos_2pi)
-  float ss, cc;
-  __sincosf(fmaf(kTwoPi * 5.9604644775390625e-8f, __uint2float_rn((wp >> 8) + 1u), -kPi), &ss, &cc);
-  return renormalise(rot_from_ez<false>(dir, make_float3(-cc * st, -ss * st, c)));
+  const float2 ang = fma2(dup2(kTwoPi * 5.9604644775390625e-8f),
+                          make_float2(__uint2float_rn((wp.x >> 8) + 1u),
+                                      __uint2float_rn((wp.y >> 8) + 1u)),
+                          dup2(-kPi));
+  float2 ss, cc;
+  __sincosf(ang.x, &ss.x, &cc.x);
+  __sincosf(ang.y, &ss.y, &cc.y);
+  // the azimuth's sine and cosine are -ss and -cc
+  const float2 nst = make_float2(-st.x, -st.y);
+  const float2 bx = mul2(cc, nst), by = mul2(ss, nst), nbx = mul2(cc, st);
+  // 1 / (1 + a.z), or (1 - a.z) / (a.x^2 + a.y^2) in the lower hemisphere; 0 on
+  // the lower axis, where the rotation is -1
+  const float2 s2 = fma2(a.y, a.y, mul2(a.x, a.x));
+  const float2 up = add2(a.z, dup2(1.0f)), down = sub2(dup2(1.0f), a.z);
+  float2 f;
+  {
+    const bool u0 = a.z.x >= 0.0f, u1 = a.z.y >= 0.0f;
+    const float d0 = u0 ? up.x : s2.x, d1 = u1 ? up.y : s2.y;
+    f = mul2(make_float2(u0 ? 1.0f : down.x, u1 ? 1.0f : down.y),
+             make_float2(ftz_rcp(d0), ftz_rcp(d1)));
+    if (d0 < 1.17549435e-38f) f.x = 0.0f;
+    if (d1 < 1.17549435e-38f) f.y = 0.0f;
+  }
+  const float2 k = mul2(fma2(a.x, by, mul2(a.y, nbx)), f);
+  const float2 nk = make_float2(-k.x, -k.y);
+  const float2 ox = fma2(a.x, c, fma2(bx, a.z, mul2(a.y, nk)));
+  const float2 oy = fma2(a.y, c, fma2(by, a.z, mul2(a.x, k)));
+  const float2 w = fma2(a.x, bx, mul2(a.y, by));
+  const float2 oz = fma2(c, a.z, make_float2(-w.x, -w.y));
+  const float2 s = fma2(dup2(-0.5f), fma2(oz, oz, fma2(oy, oy, mul2(ox, ox))), dup2(1.5f));
+  return {mul2(ox, s), mul2(oy, s), mul2(oz, s)};
 }
 
 // ---- ray-sphere test (_intersect_nsphere, src/photon_prop_cuda.jl:309-343) --

@@ -106,27 +106,42 @@ inline double SafetyDev::auto_cell(const float* blo, const float* bhi) {
   return h;
 }
 
-// Per-warp shared-memory state of the propagation kernel: the queue of
-// deferred step segments and, per lane, the earliest hit found so far.
-// Entries [0, checked) of the queue have been clipped by the safety field and
-// wait for the grid walk over [t0, t1]; entries from `checked` on wait to be
-// clipped (at most 32 of them at a time).
-constexpr int kQueueCap = 64;
-constexpr int kMaxBlockThreads = 1024;
+// A lane of the propagation kernel carries two photons, so a CTA of
+// block_threads "photon lanes" (pp_tuning) has half as many threads.
+constexpr int kPhotonsPerLane = 2;
+constexpr int kGroup = 32 * kPhotonsPerLane;  // photons a warp carries at a time
+constexpr int kMaxBlockThreads = 1024 / kPhotonsPerLane;
+inline int propagate_warps(int block_threads) { return (block_threads + kGroup - 1) / kGroup; }
+
+// Per-warp shared-memory state of the propagation kernel: the step segments
+// whose hit test is deferred (two stacks: those not yet clipped by the safety
+// field, and those clipped, which wait for the grid walk over [t0, t1]) and,
+// per photon, the earliest hit found so far.
+constexpr int kRawCap = 32 - 1 + kGroup;  // clipped as soon as 32 wait
+constexpr int kClippedCap = 32 - 1 + 32;  // walked as soon as 32 wait
 struct WarpQueue {
-  float px[kQueueCap], py[kQueueCap], pz[kQueueCap];
-  float dx[kQueueCap], dy[kQueueCap], dz[kQueueCap];
-  float len[kQueueCap];
-  float dist0[kQueueCap];     // compensated path length at the segment start
-  uint32_t meta[kQueueCap];   // owner lane | step << 8
-  float t0[kQueueCap];        // part of the segment the grid walk must cover
-  float t1[kQueueCap];
+  struct {
+    float px[kRawCap], py[kRawCap], pz[kRawCap];
+    float dx[kRawCap], dy[kRawCap], dz[kRawCap];
+    float len[kRawCap];
+    float dist0[kRawCap];     // compensated path length at the segment start
+    uint32_t meta[kRawCap];   // owner (lane + 32 * photon) | step << 8
+  } raw;
+  struct {
+    float px[kClippedCap], py[kClippedCap], pz[kClippedCap];
+    float dx[kClippedCap], dy[kClippedCap], dz[kClippedCap];
+    float len[kClippedCap];
+    float dist0[kClippedCap];
+    uint32_t meta[kClippedCap];
+    float t0[kClippedCap];    // part of the segment the grid walk must cover
+    float t1[kClippedCap];
+  } clip;
 };
 struct WarpBest {
-  uint32_t key[32];           // step << 16 | target index; ~0 = none
-  float hx[32], hy[32], hz[32];
-  float ox[32], oy[32], oz[32];
-  float dist[32];
+  uint32_t key[kGroup];       // step << 16 | target index; ~0 = none
+  float hx[kGroup], hy[kGroup], hz[kGroup];
+  float ox[kGroup], oy[kGroup], oz[kGroup];
+  float dist[kGroup];
 };
 
 constexpr uint32_t kCellStartBits = 20;                    // first item index
@@ -139,8 +154,8 @@ struct PhaseDev {
   float hg_weight;  // P(Henyey-Greenstein)
   float hg_g;
   float hg_1mg2;    // 1 - g^2
-  float hg_1pg2;    // 1 + g^2
-  float hg_inv2g;   // 1 / (2 g)
+  float hg_n1pg2;   // -(1 + g^2)
+  float hg_ninv2g;  // -1 / (2 g)
   float es_k1;      // (b + 3) / b
   float es_k2;      // 1 / b^3
   float es_b;       // Einstein-Smoluchowski b
@@ -197,8 +212,8 @@ inline const char* make_phase(const pp_medium* m, PhaseDev* p) {
   p->hg_weight = m->hg_weight;
   p->hg_g = g;
   p->hg_1mg2 = 1.0f - g * g;
-  p->hg_1pg2 = 1.0f + g * g;
-  p->hg_inv2g = m->hg_weight > 0.0f ? 1.0f / (2.0f * g) : 0.0f;
+  p->hg_n1pg2 = -(1.0f + g * g);
+  p->hg_ninv2g = m->hg_weight > 0.0f ? -1.0f / (2.0f * g) : 0.0f;
   p->es_k1 = (b + 3.0f) / b;
   p->es_k2 = 1.0f / (b * b * b);
   p->es_b = b;
@@ -218,7 +233,7 @@ struct LaunchArgs {
   const long long* src_photons;            // [n_src] photons after scaling
   unsigned long long total_chunks;
   int n_src;
-  int chunk_photons;                       // 32 * photons_per_thread
+  int chunk_photons;                       // photons per queued chunk
 
   const unsigned char* blob;               // grid blob (global memory)
   GridDev grid;
@@ -288,7 +303,7 @@ inline size_t propagate_smem_bytes(uint32_t blob_bytes, uint32_t safety_bytes, b
   const size_t off = smem_tables ? blob + field : 0;
   if (safety_offset) *safety_offset = (uint32_t)blob;
   if (state_offset) *state_offset = (uint32_t)off;
-  return off + (size_t)(block_threads / 32) * (sizeof(WarpQueue) + sizeof(WarpBest));
+  return off + (size_t)propagate_warps(block_threads) * (sizeof(WarpQueue) + sizeof(WarpBest));
 }
 // Largest dynamic shared memory per CTA for which CTAs of block_threads
 // still fill an SM with 1024 threads (the 64-register cap of the kernel): the

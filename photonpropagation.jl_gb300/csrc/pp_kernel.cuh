@@ -1,29 +1,35 @@
 // pp_kernel.cuh -- the persistent photon-propagation kernel template.
 //
 // Included by two translation units: pp_propagate.cu instantiates the fast
-// variant (SFU approximations, FMA contraction), pp_propagate_precise.cu the
+// variant (SFU approximations, packed pairs), pp_propagate_precise.cu the
 // replay variant (IEEE math library, compiled with -fmad=false so that every
 // FP32 expression rounds exactly as the CPU oracle's does).
 //
 // Replaces cuda_propagate_photons! (PhotonPropagation.jl v0.9.3,
 // src/photon_prop_cuda.jl:429-549) and its one-launch-per-source host loop
 // (:927-943).  Design:
-//   * persistent CTAs; every warp pulls chunks of 32 * photons_per_thread
-//     photons of one source from a device work queue, so one launch covers any
-//     number of sources with uneven photon counts;
+//   * persistent CTAs; every warp pulls chunks of photons of one source from a
+//     device work queue, so one launch covers any number of sources with
+//     uneven photon counts;
 //   * photon i of source s draws its random numbers from Philox4x32-10 at
 //     counter (i, call, s) and key = seed: results do not depend on the launch
 //     shape and any photon range can be replayed;
+//   * two photons per lane.  The kernel is bound by instruction issue, and the
+//     packed f32x2 instructions do the two photons' sums and products in one
+//     issue slot; the 64 photons of a warp also fill its clip and walk passes
+//     twice as well.  16 warps of 104 registers replace 32 of 64: per photon step
+//     8.7 warp instructions instead of 11.4 (1e8 photons, 400 modules: 16.66 ->
+//     15.75 ms; 256 emitters 5.51 -> 4.97; histogram tables 6.22 -> 5.37);
 //   * speculative stepping with deferred hit tests.  Each lane runs all
-//     n_steps of its photon without waiting for the target test.  A step
+//     n_steps of its photons without waiting for the target test.  A step
 //     segment is cleared cheaply when the safety field proves that no target
 //     lies within the ball around its midpoint; the rare uncleared segments
-//     go to a per-warp queue in shared memory.  When 32 of them wait, the warp
+//     go to a per-warp stack in shared memory.  When 32 of them wait, the warp
 //     clips them, one per lane, by sphere tracing the safety field from both
-//     ends (most vanish); the survivors stay queued with the part of the
-//     segment that may come near a target, and whenever 32 survivors wait the
+//     ends (most vanish); the survivors wait on a second stack with the part
+//     of the segment that may come near a target, and whenever 32 wait the
 //     warp walks them, one per lane, through the uniform-grid DDA over that
-//     part only.  The photon's hit is the earliest step with an intersection
+//     part only.  A photon's hit is the earliest step with an intersection
 //     and, within it, the lowest target index -- the reference's "first
 //     target in index order" (:497-506).  Steps after the hit were computed
 //     speculatively and are discarded;
@@ -113,7 +119,7 @@ __device__ bool stage_tables(unsigned char* dst0, const unsigned char* src0, uin
   }
 }
 
-// A point against the safety field, in units of the node spacing: q, the
+// Two points against the safety field, in units of the node spacing: q, the
 // squared distance of m from the field's box, and w, the lower bound
 // max(D(c) - |m' - c|, 0) at m's projection m' onto the box, c the nearest node.
 // Adding and subtracting 2^23 rounds to the nearest node and leaves the node's
@@ -121,54 +127,54 @@ __device__ bool stage_tables(unsigned char* dst0, const unsigned char* src0, uin
 // 45 instructions against 55-60 for floor, clamp and a Chebyshev box test,
 // and sqrt(q + w^2) clears more than the larger of two bounds did.
 constexpr float kRoundMagic = 8388608.0f;
-struct FieldPoint {
-  float q, w;
+struct FieldPoint2 {
+  float2 q, w;
 };
 template <bool kShared>
-__device__ __forceinline__ FieldPoint field_point(const SafetyDev& s,
-                                                  const unsigned char* __restrict__ f, float3 m) {
-  const float ux = fmaf(m.x, s.inv_cell, -s.lo_sc[0]);
-  const float uy = fmaf(m.y, s.inv_cell, -s.lo_sc[1]);
-  const float uz = fmaf(m.z, s.inv_cell, -s.lo_sc[2]);
-  const float cx = fminf(fmaxf(ux, 0.0f), s.fmaxc[0]);
-  const float cy = fminf(fmaxf(uy, 0.0f), s.fmaxc[1]);
-  const float cz = fminf(fmaxf(uz, 0.0f), s.fmaxc[2]);
-  const float ex = ux - cx, ey = uy - cy, ez = uz - cz;
-  const float gx = cx + kRoundMagic;
-  const float fx = gx - kRoundMagic;
-  const float fy = (cy + kRoundMagic) - kRoundMagic, fz = (cz + kRoundMagic) - kRoundMagic;
-  const float rx = cx - fx, ry = cy - fy, rz = cz - fz;
-  // 2^23 + index, exact (fewer than 2^23 nodes)
-  const uint32_t idx =
-      __float_as_uint(fmaf(fmaf(fz, s.fdims[1], fy), s.fdims[0], gx)) - 0x4B000000u;
-  const uint32_t b = kShared ? f[idx] : __ldg(f + idx);
-  // the byte as a float through its bit pattern (2^23 + b), exactly
-  const float D = fmaf(__uint_as_float(0x4B000000u | b), s.quantum, -kRoundMagic * s.quantum);
-  FieldPoint p;
-  p.q = fmaf(ez, ez, fmaf(ey, ey, ex * ex));
-  p.w = fmaxf(D - ftz_sqrt(fmaf(rz, rz, fmaf(ry, ry, rx * rx))), 0.0f);
+__device__ __forceinline__ FieldPoint2 field_point2(const SafetyDev& s,
+                                                    const unsigned char* __restrict__ f,
+                                                    const Vec2& m) {
+  const float2 inv = dup2(s.inv_cell), magic = dup2(kRoundMagic), nmagic = dup2(-kRoundMagic);
+  const float2 ux = fma2(m.x, inv, dup2(-s.lo_sc[0]));
+  const float2 uy = fma2(m.y, inv, dup2(-s.lo_sc[1]));
+  const float2 uz = fma2(m.z, inv, dup2(-s.lo_sc[2]));
+  auto clamp = [](float2 u, float hi) {
+    return make_float2(fminf(fmaxf(u.x, 0.0f), hi), fminf(fmaxf(u.y, 0.0f), hi));
+  };
+  const float2 cx = clamp(ux, s.fmaxc[0]), cy = clamp(uy, s.fmaxc[1]), cz = clamp(uz, s.fmaxc[2]);
+  const float2 ex = sub2(ux, cx), ey = sub2(uy, cy), ez = sub2(uz, cz);
+  const float2 gx = add2(cx, magic);
+  const float2 fx = add2(gx, nmagic);
+  const float2 fy = add2(add2(cy, magic), nmagic), fz = add2(add2(cz, magic), nmagic);
+  const float2 rx = sub2(cx, fx), ry = sub2(cy, fy), rz = sub2(cz, fz);
+  const float2 id = fma2(fma2(fz, dup2(s.fdims[1]), fy), dup2(s.fdims[0]), gx);
+  const uint32_t i0 = __float_as_uint(id.x) - 0x4B000000u, i1 = __float_as_uint(id.y) - 0x4B000000u;
+  const uint32_t b0 = kShared ? f[i0] : __ldg(f + i0), b1 = kShared ? f[i1] : __ldg(f + i1);
+  const float2 D = fma2(make_float2(__uint_as_float(0x4B000000u | b0),
+                                    __uint_as_float(0x4B000000u | b1)),
+                        dup2(s.quantum), dup2(-kRoundMagic * s.quantum));
+  const float2 rr = fma2(rz, rz, fma2(ry, ry, mul2(rx, rx)));
+  const float2 w = sub2(D, make_float2(ftz_sqrt(rr.x), ftz_sqrt(rr.y)));
+  FieldPoint2 p;
+  p.q = fma2(ez, ez, fma2(ey, ey, mul2(ex, ex)));
+  p.w = make_float2(fmaxf(w.x, 0.0f), fmaxf(w.y, 0.0f));
   return p;
 }
 
-// The segment pos + t*dir, t in [0, L], provably misses every target: it lies
-// inside the ball of radius L/2 about its midpoint, and no (inflated) sphere
-// comes that near.
+// Do the segments pos + t*dir, t in [0, L], of the two photons provably miss
+// every target?  A segment lies inside the ball of radius L/2 about its
+// midpoint, and no (inflated) sphere comes that near.
 template <bool kShared>
-__device__ __forceinline__ bool segment_clear(const SafetyDev& s, const unsigned char* f,
-                                              float3 pos, float3 dir, float L) {
-  const float h = 0.5f * L;
-  const FieldPoint p = field_point<kShared>(
-      s, f, make_float3(fmaf(dir.x, h, pos.x), fmaf(dir.y, h, pos.y), fmaf(dir.z, h, pos.z)));
-  const float r = fmaf(h, s.r_scale, s.r_slack);
-  return fmaf(p.w, p.w, p.q) > r * r;
-}
-
-// Lower bound (m) on the distance from a point to every (inflated) target
-// sphere (weak outside the field's box: its distance from the box is left out).
-template <bool kShared>
-__device__ __forceinline__ float field_bound(const SafetyDev& s, const unsigned char* __restrict__ f,
-                                             float3 m) {
-  return field_point<kShared>(s, f, m).w * s.cell;
+__device__ __forceinline__ void segments_clear(const SafetyDev& s, const unsigned char* f,
+                                               const Vec2& pos, const Vec2& dir, float2 L,
+                                               bool* clear0, bool* clear1) {
+  const float2 h = mul2(L, dup2(0.5f));
+  const FieldPoint2 p = field_point2<kShared>(
+      s, f, {fma2(dir.x, h, pos.x), fma2(dir.y, h, pos.y), fma2(dir.z, h, pos.z)});
+  const float2 r = fma2(h, dup2(s.r_scale), dup2(s.r_slack));
+  const float2 bound = fma2(p.w, p.w, p.q), r2 = mul2(r, r);
+  *clear0 = bound.x > r2.x;
+  *clear1 = bound.y > r2.y;
 }
 
 // Slack (m) taken off each clipped end: covers the rounding of the traced
@@ -176,26 +182,26 @@ __device__ __forceinline__ float field_bound(const SafetyDev& s, const unsigned 
 // spheres are inflated.
 constexpr float kClipSlack = 5e-3f;
 
-// Clip the unchecked queue entries [n2, n2 + n1) (n1 <= 32, one per lane):
-// first to the grid's box (no target lies outside it), then by sphere tracing
-// the safety field twice from each end of what is left -- no target lies
-// within field_bound(p) of a point p -- so the walk can skip [0, t0) and
-// (t1, L].  Entries left with t0 < t1 are compacted (in place) to
-// [n2, n2 + kept) with their interval; the others cannot hit anything and are
-// dropped.  Returns the new number of checked entries.
+// Clip the raw entries [base, base + c) (c <= 32, one per lane): first to the
+// grid's box (no target lies outside it), then by sphere tracing the safety
+// field twice from each end of what is left, both ends in one packed test --
+// no target lies within w of a point p -- so the walk can skip [0, t0) and
+// (t1, L].  Entries left with t0 < t1 go on top of the clipped stack with
+// their interval; the others cannot hit anything and are dropped.  Returns the
+// new height of the clipped stack.
 template <bool kShared>
-__device__ __forceinline__ int check_queue(WarpQueue& q, int n2, int n1, const GridDev& g,
-                                           const SafetyDev& s, const unsigned char* __restrict__ f,
-                                           int lane) {
-  const int src = n2 + lane;
+__device__ __forceinline__ int clip_entries(WarpQueue& q, int base, int c, int n2,
+                                            const GridDev& g, const SafetyDev& s,
+                                            const unsigned char* __restrict__ f, int lane) {
+  const int src = base + lane;
   bool keep = false;
   float3 p = make_float3(0.0f, 0.0f, 0.0f), d = p;
   float L = 0.0f, d0 = 0.0f, t0 = 0.0f, t1 = 0.0f;
   uint32_t meta = 0;
-  if (lane < n1) {
-    p = make_float3(q.px[src], q.py[src], q.pz[src]);
-    d = make_float3(q.dx[src], q.dy[src], q.dz[src]);
-    L = q.len[src];
+  if (lane < c) {
+    p = make_float3(q.raw.px[src], q.raw.py[src], q.raw.pz[src]);
+    d = make_float3(q.raw.dx[src], q.raw.dy[src], q.raw.dz[src]);
+    L = q.raw.len[src];
     // slab test against the grid box (the same one the walk clips to)
     const float ix = ftz_rcp(fabsf(d.x) > 1e-20f ? d.x : 1e-20f);
     const float iy = ftz_rcp(fabsf(d.y) > 1e-20f ? d.y : 1e-20f);
@@ -207,43 +213,44 @@ __device__ __forceinline__ int check_queue(WarpQueue& q, int n2, int n1, const G
     t1 = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fminf(fmaxf(tz0, tz1), L));
 #pragma unroll
     for (int it = 0; it < 2; ++it) {
-      t0 += field_bound<kShared>(
-          s, f, make_float3(fmaf(d.x, t0, p.x), fmaf(d.y, t0, p.y), fmaf(d.z, t0, p.z)));
-      t1 -= field_bound<kShared>(
-          s, f, make_float3(fmaf(d.x, t1, p.x), fmaf(d.y, t1, p.y), fmaf(d.z, t1, p.z)));
+      const float2 t = make_float2(t0, t1);
+      const float2 w =
+          field_point2<kShared>(s, f, {fma2(dup2(d.x), t, dup2(p.x)), fma2(dup2(d.y), t, dup2(p.y)),
+                                       fma2(dup2(d.z), t, dup2(p.z))}).w;
+      t0 = fmaf(w.x, s.cell, t0);
+      t1 = fmaf(-w.y, s.cell, t1);
     }
     t0 = fmaxf(t0 - kClipSlack, 0.0f);
     t1 = fminf(t1 + kClipSlack, L);
     keep = t0 < t1;
-    d0 = q.dist0[src];
-    meta = q.meta[src];
+    d0 = q.raw.dist0[src];
+    meta = q.raw.meta[src];
   }
   const unsigned m = __ballot_sync(0xffffffffu, keep);
-  __syncwarp();  // every entry is read before any is overwritten
   if (keep) {
     const int dst = n2 + __popc(m & ((1u << lane) - 1u));
-    q.px[dst] = p.x;
-    q.py[dst] = p.y;
-    q.pz[dst] = p.z;
-    q.dx[dst] = d.x;
-    q.dy[dst] = d.y;
-    q.dz[dst] = d.z;
-    q.len[dst] = L;
-    q.dist0[dst] = d0;
-    q.meta[dst] = meta;
-    q.t0[dst] = t0;
-    q.t1[dst] = t1;
+    q.clip.px[dst] = p.x;
+    q.clip.py[dst] = p.y;
+    q.clip.pz[dst] = p.z;
+    q.clip.dx[dst] = d.x;
+    q.clip.dy[dst] = d.y;
+    q.clip.dz[dst] = d.z;
+    q.clip.len[dst] = L;
+    q.clip.dist0[dst] = d0;
+    q.clip.meta[dst] = meta;
+    q.clip.t0[dst] = t0;
+    q.clip.t1[dst] = t1;
   }
   __syncwarp();
   return n2 + __popc(m);
 }
 
-// Test the checked entries [base, base + c) (c <= 32): lane e walks entry
+// Test the clipped entries [base, base + c) (c <= 32): lane e walks entry
 // base + e through the grid DDA over its clipped interval -- or, when at most
 // 16 (10) entries are left, two (three) lanes walk an equal slice of each
 // entry's interval, overlapping by the clip slack, so that the longest walk
 // sets the pass's length less often; the earliest
-// (step, target) per owner lane wins via a shared atomicMin on the key
+// (step, target) per photon wins via a shared atomicMin on the key
 // (step << 16 | target), and the winning lane writes the hit state into the
 // owner's slot.
 template <bool P>
@@ -259,16 +266,16 @@ __device__ __forceinline__ void test_queue(WarpQueue& q, WarpBest& b, int base, 
   float d = 0.0f, d0 = 0.0f;
   float3 p = make_float3(0.0f, 0.0f, 0.0f), dir = p;
   if (el < c) {
-    p = make_float3(q.px[e], q.py[e], q.pz[e]);
-    dir = make_float3(q.dx[e], q.dy[e], q.dz[e]);
-    d0 = q.dist0[e];
-    const uint32_t meta = q.meta[e];
-    owner = (int)(meta & 31u);
-    const float t0 = q.t0[e], t1 = q.t1[e];
+    p = make_float3(q.clip.px[e], q.clip.py[e], q.clip.pz[e]);
+    dir = make_float3(q.clip.dx[e], q.clip.dy[e], q.clip.dz[e]);
+    d0 = q.clip.dist0[e];
+    const uint32_t meta = q.clip.meta[e];
+    owner = (int)(meta & (kGroup - 1u));
+    const float t0 = q.clip.t0[e], t1 = q.clip.t1[e];
     const float w = (t1 - t0) * (m == 1 ? 1.0f : (m == 2 ? 0.5f : 0.33333334f));
     const float ta = piece == 0 ? t0 : fmaxf(fmaf((float)piece, w, t0) - kClipSlack, t0);
     const float tb = piece == m - 1 ? t1 : fminf(fmaf((float)(piece + 1), w, t0) + kClipSlack, t1);
-    j = first_hit<P>(g, cells, items, sph, p, dir, q.len[e], ta, tb, &d);
+    j = first_hit<P>(g, cells, items, sph, p, dir, q.clip.len[e], ta, tb, &d);
     if (j >= 0) {
       key = ((meta >> 8) << 16) | (uint32_t)j;
       atomicMin(&b.key[owner], key);
@@ -423,14 +430,74 @@ __device__ __noinline__ PhotonInit init_photon_again(const LaunchArgs& a, int s,
   return init_photon<kPrecise>(a, s, plo, phi);
 }
 
-// One CTA of kMaxBlockThreads per SM caps the kernel at 64 registers.
+// One CTA of kMaxBlockThreads per SM caps the kernel at 128 registers.
 #ifndef PP_PROPAGATE_MIN_BLOCKS
 #define PP_PROPAGATE_MIN_BLOCKS 1
 #endif
 
+// Put a step segment on the raw stack (visible to the warp after a __syncwarp).
+__device__ __forceinline__ void push_raw(WarpQueue& q, int e, float3 pos, float3 dir, float step,
+                                         float dist0, uint32_t meta) {
+  q.raw.px[e] = pos.x;
+  q.raw.py[e] = pos.y;
+  q.raw.pz[e] = pos.z;
+  q.raw.dx[e] = dir.x;
+  q.raw.dy[e] = dir.y;
+  q.raw.dz[e] = dir.z;
+  q.raw.len[e] = step;
+  q.raw.dist0[e] = dist0;
+  q.raw.meta[e] = meta;
+}
+
+// Shaped targets: test one step segment against every target in index order and
+// keep the first hit as photon `own`'s; a list of detector lines is searched
+// line by line (src/photon_prop_cuda.jl:611-634): the 2-D test of the line, then
+// its modules; the first crossed line ends the search.
+template <bool kPrecise>
+__device__ __forceinline__ bool search_shapes(const LaunchArgs& a, float3 pos, float3 dir,
+                                              float step, float dist0, uint32_t k, WarpBest& best,
+                                              int own) {
+  int hit = -1;  // 0-based module index to report
+  float d = 0.0f;
+  int line_no = 0;
+  for (int j = 0; j < a.n_shapes; ++j) {
+    const float4 h = __ldg(a.shapes + 2 * j + 1);
+    if (__float_as_int(h.y) == PP_TARGET_LINE) {
+      const int nm = __float_as_int(h.x);
+      ++line_no;
+      float dl;
+      if (!sphere_hit<kPrecise>(__ldg(a.shapes + 2 * j), make_float3(pos.x, pos.y, 0.0f),
+                                make_float3(dir.x, dir.y, 0.0f), step, &dl)) {
+        j += nm;
+        continue;
+      }
+      for (int m = 1; m <= nm; ++m) {
+        if (shape_hit<kPrecise>(a.shapes, j + m, pos, dir, step, &d)) {
+          hit = m + nm * line_no - 1;
+          break;
+        }
+      }
+      break;
+    }
+    if (shape_hit<kPrecise>(a.shapes, j, pos, dir, step, &d)) {
+      hit = j;
+      break;
+    }
+  }
+  if (hit < 0) return false;
+  best.key[own] = (k << 16) | (uint32_t)hit;
+  best.hx[own] = madd<kPrecise>(dir.x, d, pos.x);
+  best.hy[own] = madd<kPrecise>(dir.y, d, pos.y);
+  best.hz[own] = madd<kPrecise>(dir.z, d, pos.z);
+  best.ox[own] = dir.x;
+  best.oy[own] = dir.y;
+  best.oz[own] = dir.z;
+  best.dist[own] = dist0 + d;
+  return true;
+}
+
 // kShapes: shaped targets (a.shapes), every target tested at every step in
-// index order (no grid, no deferred queue); a list of detector lines is
-// searched line by line (src/photon_prop_cuda.jl:611-634).
+// index order (no grid, no deferred queue).
 template <bool kPrecise, bool kSmemGrid, bool kShapes = false>
 __global__ void __launch_bounds__(kMaxBlockThreads, PP_PROPAGATE_MIN_BLOCKS)
     propagate_kernel(const __grid_constant__ LaunchArgs a) {
@@ -486,169 +553,160 @@ __global__ void __launch_bounds__(kMaxBlockThreads, PP_PROPAGATE_MIN_BLOCKS)
     const int s = lo;
     const long long p0 = (long long)(c - __ldg(a.chunk_prefix + s)) * a.chunk_photons;
     const long long pend = min(p0 + (long long)a.chunk_photons, __ldg(a.src_photons + s));
-    const long long first = __ldg(&a.sources[s].first_photon);
+    const long long first_photon = __ldg(&a.sources[s].first_photon);
 
-    for (long long base = p0; base < pend; base += 32) {
-      const bool active = base + lane < pend;
-      // Lanes past the end replay the first photon of the round (never recorded).
-      const long long p = first + (active ? base + lane : base);
-      const uint32_t plo = (uint32_t)p, phi = (uint32_t)((unsigned long long)p >> 32);
-      float3 pos, dir;
-      float sca_len;
-      {
-        const PhotonInit in = init_photon<kPrecise>(a, s, plo, phi);
-        pos = in.pos;
-        dir = in.dir;
-        sca_len = in.med.x;
+    int count;
+    for (long long base = p0; base < pend; base += count) {
+      // A group: up to 64 photons, lane l carrying the l-th and the (32 + l)-th,
+      // all with the same high counter word.
+      const long long pb = first_photon + base;
+      count = (int)min(min(pend - base, (long long)kGroup),
+                       0x100000000ll - (long long)(uint32_t)pb);
+      const uint32_t phi = (uint32_t)((unsigned long long)pb >> 32);
+      const bool active0 = lane < count, active1 = lane + 32 < count;
+      // Lanes past the end replay the group's first photon (never recorded).
+      const uint32_t plo0 = (uint32_t)pb + (active0 ? (uint32_t)lane : 0u);
+      const uint32_t plo1 = (uint32_t)pb + (active1 ? (uint32_t)lane + 32u : 0u);
+      Vec2 pos, dir;
+      float2 sca_len;
+#pragma unroll 1
+      for (int j = 0; j < 2; ++j) {
+        const PhotonInit in = init_photon<kPrecise>(a, s, j ? plo1 : plo0, phi);
+        if (j == 0) {
+          pos.x.x = in.pos.x; pos.y.x = in.pos.y; pos.z.x = in.pos.z;
+          dir.x.x = in.dir.x; dir.y.x = in.dir.y; dir.z.x = in.dir.z;
+          sca_len.x = in.med.x;
+        } else {
+          pos.x.y = in.pos.x; pos.y.y = in.pos.y; pos.z.y = in.pos.z;
+          dir.x.y = in.dir.x; dir.y.y = in.dir.y; dir.z.y = in.dir.z;
+          sca_len.y = in.med.x;
+        }
       }
-      float dist = 0.0f, comp = 0.0f;  // Kahan-compensated path length
+      const PhiloxPhoton ph0 = philox_photon(plo0, (uint32_t)s, a.round_keys);
+      const PhiloxPhoton ph1 = philox_photon(plo1, (uint32_t)s, a.round_keys);
+      float2 dist = dup2(0.0f), comp = dup2(0.0f);  // Kahan-compensated path lengths
       best.key[lane] = 0xffffffffu;
+      best.key[lane + 32] = 0xffffffffu;
       __syncwarp();
-      // warp-uniform queue state: [0, n2) clipped, [n2, n2 + n1) not yet
+      // heights of the raw and the clipped stack (warp-uniform)
       int n1 = 0, n2 = 0;
-      bool found = false;  // shaped targets: the photon has hit
-      // The step loop holds no grid walk: when more than 31 checked entries
-      // wait, it stops before appending step k's entries, the walk below takes
-      // 32 of them, and the loop resumes at step k (recomputing its random
-      // numbers and ball test, which are the same).  At the end of the steps
-      // the same walk takes everything left.
+      bool found0 = false, found1 = false;  // shaped targets: the photon has hit
+      // The step loop holds neither the clip nor the walk: it stops when 32 raw
+      // entries wait, they are clipped, 32 clipped ones are walked as soon as
+      // they wait, and the loop resumes; after the last step the same code
+      // takes what is left.
       int k = 1;
       while (true) {
-      bool flush = true;
-      for (; k <= a.n_steps; ++k) {
-        const uint4 r = philox(make_uint4(plo, phi, (uint32_t)k, (uint32_t)s), a.round_keys);
-        const float step = -f_log<kPrecise>(u01(r.x)) * sca_len;
-        if constexpr (kShapes) {
-          if (active && !found) {
-            int hit = -1;  // 0-based module index to report
-            float d = 0.0f;
-            int line_no = 0;
-            for (int j = 0; j < a.n_shapes; ++j) {
-              const float4 h = __ldg(a.shapes + 2 * j + 1);
-              if (__float_as_int(h.y) == PP_TARGET_LINE) {
-                // DetectorLines: the 2-D test of the line, then its modules;
-                // the first crossed line ends the search
-                const int nm = __float_as_int(h.x);
-                ++line_no;
-                float dl;
-                if (!sphere_hit<kPrecise>(__ldg(a.shapes + 2 * j), make_float3(pos.x, pos.y, 0.0f),
-                                          make_float3(dir.x, dir.y, 0.0f), step, &dl)) {
-                  j += nm;
-                  continue;
-                }
-                for (int m = 1; m <= nm; ++m) {
-                  if (shape_hit<kPrecise>(a.shapes, j + m, pos, dir, step, &d)) {
-                    hit = m + nm * line_no - 1;
-                    break;
-                  }
-                }
-                break;
-              }
-              if (shape_hit<kPrecise>(a.shapes, j, pos, dir, step, &d)) {
-                hit = j;
-                break;
-              }
-            }
-            if (hit >= 0) {
-              found = true;
-              best.key[lane] = ((uint32_t)k << 16) | (uint32_t)hit;
-              best.hx[lane] = madd<kPrecise>(dir.x, d, pos.x);
-              best.hy[lane] = madd<kPrecise>(dir.y, d, pos.y);
-              best.hz[lane] = madd<kPrecise>(dir.z, d, pos.z);
-              best.ox[lane] = dir.x;
-              best.oy[lane] = dir.y;
-              best.oz[lane] = dir.z;
-              best.dist[lane] = (dist - comp) + d;
-            }
+        for (; k <= a.n_steps && n1 < 32; ++k) {
+          const PhiloxStep pt = philox_step((uint32_t)k, phi, a.round_keys);
+          const uint4 r0 = philox_words(ph0, pt, a.round_keys);
+          const uint4 r1 = philox_words(ph1, pt, a.round_keys);
+          float2 step;
+          if constexpr (kPrecise)
+            step = make_float2(-f_log<true>(u01(r0.x)) * sca_len.x,
+                               -f_log<true>(u01(r1.x)) * sca_len.y);
+          else
+            step = mul2(mul2(make_float2(ftz_lg2(u01(r0.x)), ftz_lg2(u01(r1.x))),
+                             dup2(-0.693147182f)), sca_len);
+          if constexpr (kShapes) {
+            if (active0 && !found0)
+              found0 = search_shapes<kPrecise>(a, first(pos), first(dir), step.x, dist.x - comp.x,
+                                               (uint32_t)k, best, lane);
+            if (active1 && !found1)
+              found1 = search_shapes<kPrecise>(a, second(pos), second(dir), step.y,
+                                               dist.y - comp.y, (uint32_t)k, best, lane + 32);
+          } else {
+            bool clear0, clear1;
+            segments_clear<kSmemGrid>(a.sgrid, field, pos, dir, step, &clear0, &clear1);
+            const bool need0 = have_grid && active0 && !clear0;
+            const bool need1 = have_grid && active1 && !clear1;
+            const unsigned m0 = __ballot_sync(0xffffffffu, need0);
+            const unsigned m1 = __ballot_sync(0xffffffffu, need1);
+            if (need0)
+              push_raw(q, n1 + __popc(m0 & lanemask_lt), first(pos), first(dir), step.x,
+                       dist.x - comp.x, (uint32_t)lane | ((uint32_t)k << 8));
+            n1 += __popc(m0);
+            if (need1)
+              push_raw(q, n1 + __popc(m1 & lanemask_lt), second(pos), second(dir), step.y,
+                       dist.y - comp.y, (uint32_t)(lane + 32) | ((uint32_t)k << 8));
+            n1 += __popc(m1);
           }
-        } else {
-        const bool need = have_grid && active && !segment_clear<kSmemGrid>(a.sgrid, field, pos, dir, step);
-        const unsigned m = __ballot_sync(0xffffffffu, need);
-        if (m) {
-          const int nn = __popc(m);
-          if (n1 + nn > 32) {
-            // clip the unchecked entries; walk the grid once 32 checked ones wait
-            n2 = check_queue<kSmemGrid>(q, n2, n1, a.grid, a.sgrid, field, lane);
-            n1 = 0;
-            if (n2 >= 32) {
-              flush = false;
-              break;
-            }
+          if constexpr (kPrecise) {
+            const float3 q0 = first(pos), q1 = second(pos), e0 = first(dir), e1 = second(dir);
+            pos = both(make_float3(madd<true>(e0.x, step.x, q0.x), madd<true>(e0.y, step.x, q0.y),
+                                   madd<true>(e0.z, step.x, q0.z)),
+                       make_float3(madd<true>(e1.x, step.y, q1.x), madd<true>(e1.y, step.y, q1.y),
+                                   madd<true>(e1.z, step.y, q1.z)));
+          } else {
+            pos = {fma2(dir.x, step, pos.x), fma2(dir.y, step, pos.y), fma2(dir.z, step, pos.z)};
           }
-          if (need) {
-            const int e = n2 + n1 + __popc(m & lanemask_lt);
-            q.px[e] = pos.x;
-            q.py[e] = pos.y;
-            q.pz[e] = pos.z;
-            q.dx[e] = dir.x;
-            q.dy[e] = dir.y;
-            q.dz[e] = dir.z;
-            q.len[e] = step;
-            q.dist0[e] = dist - comp;
-            q.meta[e] = (uint32_t)lane | ((uint32_t)k << 8);
+          {
+            const float2 y = sub2(step, comp), t = add2(dist, y);
+            comp = sub2(sub2(t, dist), y);
+            dist = t;
           }
-          n1 += nn;
-          __syncwarp();
+          if constexpr (kPrecise)
+            dir = both(update_direction_precise(a.phase, first(dir), r0.y, r0.z, r0.w),
+                       update_direction_precise(a.phase, second(dir), r1.y, r1.z, r1.w));
+          else
+            dir = update_direction_fast(a.phase, dir, make_uint2(r0.y, r1.y),
+                                        make_uint2(r0.z, r1.z), make_uint2(r0.w, r1.w));
         }
-        }  // kShapes
-        pos = make_float3(madd<kPrecise>(dir.x, step, pos.x), madd<kPrecise>(dir.y, step, pos.y),
-                          madd<kPrecise>(dir.z, step, pos.z));
-        {
-          const float y = step - comp, t = dist + y;
-          comp = (t - dist) - y;
-          dist = t;
+        if (kShapes) break;
+        __syncwarp();  // the raw entries are visible
+        if (n1 > 0) {  // 32 wait, or the steps are done
+          const int take = min(n1, 32);
+          n1 -= take;
+          n2 = clip_entries<kSmemGrid>(q, n1, take, n2, a.grid, a.sgrid, field, lane);
         }
-        dir = update_direction<kPrecise>(a.phase, dir, r.y, r.z, r.w);
+        const bool last = k > a.n_steps && n1 == 0;
+        if (n2 >= 32 || (last && n2 > 0)) {
+          const int take = min(n2, 32);
+          n2 -= take;
+          test_queue<kPrecise>(q, best, n2, take, a.grid, cells, items, sph, lane);
+        }
+        if (last && n2 == 0) break;
       }
-      if (kShapes) break;
-      if (flush && n1 > 0) {
-        n2 = check_queue<kSmemGrid>(q, n2, n1, a.grid, a.sgrid, field, lane);
-        n1 = 0;
-      }
-      while (n2 > 0) {
-        const int c = n2 < 32 ? n2 : 32;
-        n2 -= c;
-        test_queue<kPrecise>(q, best, n2, c, a.grid, cells, items, sph, lane);
-        if (!flush) break;
-      }
-      if (flush) break;
-      }  // resume the steps after a walk
       __syncwarp();
 
-      const uint32_t key = best.key[lane];
-      bool overflowed = false;
-      int steps_taken = a.n_steps;
-      if (active && key != 0xffffffffu) {
-        steps_taken = (int)(key >> 16);
-        const PhotonInit in = init_photon_again<kPrecise>(a, s, plo, phi);
-        const float wl = in.wl;
-        const float3 idir = in.dir;
-        const float t0 = in.t0;
-        const float4 med = in.med;
-        const float3 hpos = make_float3(best.hx[lane], best.hy[lane], best.hz[lane]);
-        const float3 hdir = make_float3(best.ox[lane], best.oy[lane], best.oz[lane]);
-        const float hdist = best.dist[lane];
-        const double time = (double)t0 + (double)hdist / (double)med.y;
-        const float abs_w = f_exp<kPrecise>(-f_div<kPrecise>(hdist, med.z));
-        if (a.hist) {
-          // arrival-time histogram of this source, weighted by absorption
-          const float tres = (float)(time - (double)__ldg(a.hist_tgeo + s));
-          const float u = log10f(fmaxf(tres + a.hist_t_offset, 1e-30f));
-          const int bin =
-              min(max((int)floorf((u - a.hist_log_lo) * a.hist_inv_log_width), 0), a.hist_bins - 1);
-          float* row = a.hist + (size_t)s * (size_t)(a.hist_bins + 1);
-          atomicAdd(row, abs_w);
-          atomicAdd(row + 1 + bin, abs_w);
-          atomicAdd(u64(&a.counters->n_hits), 1ull);
-        } else {
-          record_hit(a, hpos, wl, hdir, hdist, idir, abs_w, time, p, (int)(key & 0xffffu) + 1,
-                     steps_taken, s, &overflowed);
+#pragma unroll 1
+      for (int j = 0; j < 2; ++j) {
+        const int own = lane + 32 * j;
+        const bool active = own < count;
+        const uint32_t key = best.key[own];
+        bool overflowed = false;
+        int steps_taken = a.n_steps;
+        if (active && key != 0xffffffffu) {
+          steps_taken = (int)(key >> 16);
+          const uint32_t plo = j ? plo1 : plo0;
+          const PhotonInit in = init_photon_again<kPrecise>(a, s, plo, phi);
+          const float4 med = in.med;
+          const float hdist = best.dist[own];
+          const double time = (double)in.t0 + (double)hdist / (double)med.y;
+          const float abs_w = f_exp<kPrecise>(-f_div<kPrecise>(hdist, med.z));
+          if (a.hist) {
+            // arrival-time histogram of this source, weighted by absorption
+            const float tres = (float)(time - (double)__ldg(a.hist_tgeo + s));
+            const float u = log10f(fmaxf(tres + a.hist_t_offset, 1e-30f));
+            const int bin = min(max((int)floorf((u - a.hist_log_lo) * a.hist_inv_log_width), 0),
+                                a.hist_bins - 1);
+            float* row = a.hist + (size_t)s * (size_t)(a.hist_bins + 1);
+            atomicAdd(row, abs_w);
+            atomicAdd(row + 1 + bin, abs_w);
+            atomicAdd(u64(&a.counters->n_hits), 1ull);
+          } else {
+            record_hit(a, make_float3(best.hx[own], best.hy[own], best.hz[own]), in.wl,
+                       make_float3(best.ox[own], best.oy[own], best.oz[own]), hdist, in.dir, abs_w,
+                       time, (long long)(((unsigned long long)phi << 32) | plo),
+                       (int)(key & 0xffffu) + 1, steps_taken, s, &overflowed);
+          }
+        }
+        if (active) {
+          steps_acc += (unsigned long long)steps_taken;
+          if (!overflowed) sim_acc += 1;
         }
       }
-      if (active) {
-        steps_acc += (unsigned long long)steps_taken;
-        if (!overflowed) sim_acc += 1;
-      }
+      __syncwarp();  // the hits are read before the next group clears them
     }
   }
 

@@ -28,7 +28,8 @@ int propagate_occupancy(int block_threads, bool precise, bool smem_tables, uint3
   if (smem_bytes > 48 * 1024)
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
   int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, block_threads, smem_bytes) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, propagate_warps(block_threads) * 32,
+                                                    smem_bytes) != cudaSuccess)
     return 0;
   return n;
 }
@@ -39,29 +40,31 @@ cudaError_t launch_propagate(const LaunchArgs& args, int block_threads, int ctas
   const bool shapes = args.shapes != nullptr;
   if (shapes) smem_grid = false;
   const void* k = select_kernel(precise, smem_grid, shapes);
-  if (block_threads > kMaxBlockThreads || block_threads % 32) return cudaErrorInvalidValue;
+  if (block_threads > kMaxBlockThreads * kPhotonsPerLane || block_threads % 32)
+    return cudaErrorInvalidValue;
+  const int threads = propagate_warps(block_threads) * 32;
   LaunchArgs a = args;
   const size_t smem = propagate_smem_bytes(args.grid.blob_bytes, args.sgrid.bytes, smem_grid,
                                            block_threads, &a.safety_offset, &a.state_offset);
-  a.warps_per_block = block_threads / 32;
+  a.warps_per_block = threads / 32;
   cudaError_t e;
   if (smem > 48 * 1024) {
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
   int occ = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, block_threads, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, threads, smem);
   if (e != cudaSuccess) return e;
   if (occ < 1) return cudaErrorInvalidConfiguration;
   const int per_sm = ctas_per_sm > 0 ? (ctas_per_sm < occ ? ctas_per_sm : occ) : occ;
   int grid = per_sm * num_sms;
   // Never launch more warps than there are chunks of work.
-  const unsigned long long warps_per_cta = (unsigned long long)(block_threads / 32);
+  const unsigned long long warps_per_cta = (unsigned long long)(threads / 32);
   const unsigned long long need = (args.total_chunks + warps_per_cta - 1) / warps_per_cta;
   if (need < (unsigned long long)grid) grid = (int)(need > 0 ? need : 1);
   if (grid_out) *grid_out = grid;
   void* params[] = {&a};
-  return cudaLaunchKernel(k, dim3(grid), dim3(block_threads), params, smem, stream);
+  return cudaLaunchKernel(k, dim3(grid), dim3(threads), params, smem, stream);
 }
 
 }  // namespace pp
