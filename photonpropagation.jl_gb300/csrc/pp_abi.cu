@@ -189,7 +189,7 @@ int build_queue(pp_ctx* ctx) {
   // that a 1e5-photon call is not run by a tenth of the warps.  Photons draw
   // their random numbers by index, so the chunking changes no result.
   int ppt = ctx->tuning.photons_per_thread;
-  const long long resident_warps = 1024LL / pp::kGroup * std::max(ctx->num_sms, 1);
+  const long long resident_warps = (long long)pp::kSmWarps * std::max(ctx->num_sms, 1);
   while (ppt > 1 && total / (32LL * ppt) < 2 * resident_warps) ppt /= 2;
   const long long chunk = 32LL * ppt;
   for (int i = 0; i < n; ++i)

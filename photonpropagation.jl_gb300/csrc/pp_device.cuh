@@ -527,33 +527,25 @@ __device__ __forceinline__ bool shape_hit(const float4* __restrict__ shapes, int
 
 // First target in index order intersected within (0, step): the candidates
 // come from a 3-D DDA walk over the uniform grid cells the segment crosses
-// between t_lo and t_hi (0 <= t_lo, t_hi <= step: the part of the segment
-// that may come near a target; the sphere test itself always uses the whole
-// segment) (Amanatides & Woo); among all intersected candidates the smallest index
+// between t_lo and t_hi (0 <= t_lo < t_hi <= step: the part of the segment
+// that may come near a target, inside the grid's box up to rounding; the sphere
+// test itself always uses the whole segment) (Amanatides & Woo); among all intersected candidates the smallest index
 // wins, which is exactly the reference's "first target in index order"
 // (src/photon_prop_cuda.jl:497-506).  Returns the 0-based index or -1.
 template <bool P>
 __device__ __forceinline__ int first_hit(const pp::GridDev& g, const uint32_t* __restrict__ cells,
                                          const uint16_t* __restrict__ items,
                                          const float4* __restrict__ sph, float3 pos, float3 dir,
-                                         float step, float t_lo, float t_hi, float* d_out) {
+                                         float step, float t_lo, float t_hi) {
   // Reciprocal direction; zero components become a huge value of the same
   // sign as the step direction chosen below (+ for +0 and -0 alike).
   const float ix = ftz_rcp(fabsf(dir.x) > 1e-20f ? dir.x : 1e-20f);
   const float iy = ftz_rcp(fabsf(dir.y) > 1e-20f ? dir.y : 1e-20f);
   const float iz = ftz_rcp(fabsf(dir.z) > 1e-20f ? dir.z : 1e-20f);
-  // Clip the segment to the grid box (slab test).
-  const float tx0 = (g.lo[0] - pos.x) * ix, tx1 = (g.hi[0] - pos.x) * ix;
-  const float ty0 = (g.lo[1] - pos.y) * iy, ty1 = (g.hi[1] - pos.y) * iy;
-  const float tz0 = (g.lo[2] - pos.z) * iz, tz1 = (g.hi[2] - pos.z) * iz;
-  const float tmin = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), t_lo));
-  const float tmax = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fminf(fmaxf(tz0, tz1), t_hi));
-  if (!(tmin <= tmax)) return -1;
-
   const int nx = g.dims[0], ny = g.dims[1], nz = g.dims[2];
-  int cx = (int)floorf((fmaf(dir.x, tmin, pos.x) - g.lo[0]) * g.inv_cell[0]);
-  int cy = (int)floorf((fmaf(dir.y, tmin, pos.y) - g.lo[1]) * g.inv_cell[1]);
-  int cz = (int)floorf((fmaf(dir.z, tmin, pos.z) - g.lo[2]) * g.inv_cell[2]);
+  int cx = (int)floorf((fmaf(dir.x, t_lo, pos.x) - g.lo[0]) * g.inv_cell[0]);
+  int cy = (int)floorf((fmaf(dir.y, t_lo, pos.y) - g.lo[1]) * g.inv_cell[1]);
+  int cz = (int)floorf((fmaf(dir.z, t_lo, pos.z) - g.lo[2]) * g.inv_cell[2]);
   cx = min(max(cx, 0), nx - 1);
   cy = min(max(cy, 0), ny - 1);
   cz = min(max(cz, 0), nz - 1);
@@ -570,7 +562,6 @@ __device__ __forceinline__ int first_hit(const pp::GridDev& g, const uint32_t* _
   int cidx = (cz * ny + cy) * nx + cx;
 
   int best = 0x7fffffff;
-  float best_d = 0.0f;
   const int max_iter = nx + ny + nz + 3;
   for (int it = 0; it < max_iter; ++it) {
     const uint32_t w = cells[cidx];
@@ -582,7 +573,6 @@ __device__ __forceinline__ int first_hit(const pp::GridDev& g, const uint32_t* _
         float d;
         if (j < best && sphere_hit<P>(sph[j], pos, dir, step, &d)) {
           best = j;
-          best_d = d;
         }
       }
     }
@@ -592,7 +582,7 @@ __device__ __forceinline__ int first_hit(const pp::GridDev& g, const uint32_t* _
     const bool ay = !ax && tny <= tnz;
     const bool az = !ax && !ay;
     const float tn = ax ? tnx : (ay ? tny : tnz);
-    if (tn > tmax) break;
+    if (tn > t_hi) break;
     cx += ax ? sx : 0;
     cy += ay ? sy : 0;
     cz += az ? sz : 0;
@@ -604,9 +594,7 @@ __device__ __forceinline__ int first_hit(const pp::GridDev& g, const uint32_t* _
     tnz += az ? tdz : 0.0f;
     cidx += ax ? strx : (ay ? stry : strz);
   }
-  if (best == 0x7fffffff) return -1;
-  *d_out = best_d;
-  return best;
+  return best == 0x7fffffff ? -1 : best;
 }
 
 // ---- emitters (initialize_photon_state, src/photon_prop_cuda.jl:158-276) ----

@@ -257,7 +257,9 @@ int build_grid(const pp_sphere* targets_dev, int n, float cell_size, cudaStream_
     vol *= ext[a];
   }
   double h = cell_size;
-  if (!(h > 0.0)) h = std::cbrt(vol / (16.0 * n));  // about 16 cells per target
+  // (400 modules: 8 cells per target 15.0 ms per 1e8 photons, 16 15.7, 4 15.2:
+  // fewer cells to cross against more spheres per cell)
+  if (!(h > 0.0)) h = std::cbrt(vol / (8.0 * n));  // about 8 cells per target
   // Keep the cell count bounded.
   const double kMaxCells = 4.0 * 1024 * 1024;
   for (int guard = 0; guard < 64; ++guard) {

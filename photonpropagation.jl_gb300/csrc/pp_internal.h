@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -106,12 +107,17 @@ inline double SafetyDev::auto_cell(const float* blo, const float* bhi) {
   return h;
 }
 
-// A lane of the propagation kernel carries two photons, so a CTA of
-// block_threads "photon lanes" (pp_tuning) has half as many threads.
-constexpr int kPhotonsPerLane = 2;
-constexpr int kGroup = 32 * kPhotonsPerLane;  // photons a warp carries at a time
-constexpr int kMaxBlockThreads = 1024 / kPhotonsPerLane;
-inline int propagate_warps(int block_threads) { return (block_threads + kGroup - 1) / kGroup; }
+// A lane of the propagation kernel carries two photons.  pp_tuning's
+// block_threads counts 1024 for all the warps an SM holds: that many, or the
+// same share of them, make a CTA.
+constexpr int kGroup = 64;     // photons a warp carries at a time
+// (16 warps of 104 registers: 24 of 80 issue 73% of the time against 68%, but
+// spill, and both take 13.6 ms per 1e8 photons; the FMA and ALU pipes bound both.)
+constexpr int kSmWarps = 16;
+constexpr int kMaxBlockThreads = 32 * kSmWarps;
+inline int propagate_warps(int block_threads) {
+  return (block_threads * kSmWarps + 1023) / 1024;
+}
 
 // Per-warp shared-memory state of the propagation kernel: the step segments
 // whose hit test is deferred (two stacks: those not yet clipped by the safety
@@ -119,26 +125,16 @@ inline int propagate_warps(int block_threads) { return (block_threads + kGroup -
 // per photon, the earliest hit found so far.
 constexpr int kRawCap = 32 - 1 + kGroup;  // clipped as soon as 32 wait
 constexpr int kClippedCap = 32 - 1 + 32;  // walked as soon as 32 wait
-struct WarpQueue {
-  struct {
-    float px[kRawCap], py[kRawCap], pz[kRawCap];
-    float dx[kRawCap], dy[kRawCap], dz[kRawCap];
-    float len[kRawCap];
-    float dist0[kRawCap];     // compensated path length at the segment start
-    uint32_t meta[kRawCap];   // owner (lane + 32 * photon) | step << 8
-  } raw;
-  struct {
-    float px[kClippedCap], py[kClippedCap], pz[kClippedCap];
-    float dx[kClippedCap], dy[kClippedCap], dz[kClippedCap];
-    float len[kClippedCap];
-    float dist0[kClippedCap];
-    uint32_t meta[kClippedCap];
-    float t0[kClippedCap];    // part of the segment the grid walk must cover
-    float t1[kClippedCap];
-  } clip;
+struct alignas(16) WarpQueue {
+  float4 raw_a[kRawCap];       // segment start, length
+  float4 raw_b[kRawCap];       // direction, owner (lane + 32 * photon) | step << 8
+  float4 clip_a[kClippedCap];
+  float4 clip_b[kClippedCap];
+  float2 clip_t[kClippedCap];  // part of the segment the grid walk must cover
+  uint32_t key[kGroup];        // step << 16 | target index; ~0 = none
 };
+// Shaped targets (no queue): per photon, the hit itself.
 struct WarpBest {
-  uint32_t key[kGroup];       // step << 16 | target index; ~0 = none
   float hx[kGroup], hy[kGroup], hz[kGroup];
   float ox[kGroup], oy[kGroup], oz[kGroup];
   float dist[kGroup];
@@ -294,7 +290,8 @@ struct LaunchArgs {
 };
 
 // Dynamic shared memory of one CTA: [grid blob | safety field] when staged,
-// then the per-warp state.
+// then the per-warp state (the queues, whose room the shaped targets' hits use).
+static_assert(sizeof(WarpBest) <= offsetof(WarpQueue, key), "shares the stacks' room");
 inline size_t propagate_smem_bytes(uint32_t blob_bytes, uint32_t safety_bytes, bool smem_tables,
                                    int block_threads, uint32_t* safety_offset,
                                    uint32_t* state_offset) {
@@ -303,10 +300,10 @@ inline size_t propagate_smem_bytes(uint32_t blob_bytes, uint32_t safety_bytes, b
   const size_t off = smem_tables ? blob + field : 0;
   if (safety_offset) *safety_offset = (uint32_t)blob;
   if (state_offset) *state_offset = (uint32_t)off;
-  return off + (size_t)propagate_warps(block_threads) * (sizeof(WarpQueue) + sizeof(WarpBest));
+  return off + (size_t)propagate_warps(block_threads) * sizeof(WarpQueue);
 }
 // Largest dynamic shared memory per CTA for which CTAs of block_threads
-// still fill an SM with 1024 threads (the 64-register cap of the kernel): the
+// still fill an SM: the
 // SM's 228 KB less 1 KB reserved per CTA and the static barrier, at most the
 // 227 KB one CTA may opt into.
 inline size_t smem_budget(int block_threads) {

@@ -117,7 +117,7 @@ void grid_shape(const pp_sphere* t, int n, float cell_size, pp::GridDev* g) {
     vol *= ext[a];
   }
   double h = cell_size;
-  if (!(h > 0.0)) h = std::cbrt(vol / (16.0 * n));
+  if (!(h > 0.0)) h = std::cbrt(vol / (8.0 * n));
   for (int guard = 0; guard < 64; ++guard) {
     double cells = 1.0;
     for (int a = 0; a < 3; ++a) cells *= std::max(1.0, std::ceil(ext[a] / h));

@@ -40,7 +40,7 @@ cudaError_t launch_propagate(const LaunchArgs& args, int block_threads, int ctas
   const bool shapes = args.shapes != nullptr;
   if (shapes) smem_grid = false;
   const void* k = select_kernel(precise, smem_grid, shapes);
-  if (block_threads > kMaxBlockThreads * kPhotonsPerLane || block_threads % 32)
+  if (block_threads > 1024 || block_threads % 32)
     return cudaErrorInvalidValue;
   const int threads = propagate_warps(block_threads) * 32;
   LaunchArgs a = args;
