@@ -241,7 +241,7 @@ int rebuild_grid(pp_ctx* ctx, float cell_size) {
   cudaFree(ctx->d_safety);
   ctx->d_safety = nullptr;
   float hs = ctx->tuning.safety_cell;
-  if (!(hs > 0.0f)) hs = (float)pp::SafetyDev::auto_cell(g.lo, g.hi);
+  if (!(hs > 0.0f)) hs = (float)pp::SafetyDev::auto_cell(g.lo, g.hi, n);
   pp::SafetyDev sg{};
   unsigned char* field = nullptr;
   if (pp::build_safety(ctx->d_targets, n, g, hs, ctx->stream, &sg, &field, &err) != 0)

@@ -453,9 +453,10 @@ __device__ __forceinline__ Vec2 update_direction_fast(const pp::PhaseDev& ph, co
   // the azimuth's sine and cosine are -ss and -cc
   const float2 nst = make_float2(-st.x, -st.y);
   const float2 bx = mul2(cc, nst), by = mul2(ss, nst), nbx = mul2(cc, st);
-  // 1 / (1 + a.z), or (1 - a.z) / (a.x^2 + a.y^2) in the lower hemisphere; 0 on
-  // the lower axis, where the rotation is -1
-  const float2 s2 = fma2(a.y, a.y, mul2(a.x, a.x));
+  // 1 / (1 + a.z), or (1 - a.z) / (a.x^2 + a.y^2) in the lower hemisphere.  The
+  // added 2^-126 (lost in any other sum) keeps it finite on the lower axis,
+  // where it meets zeros (emission directions are exact there, on_axis)
+  const float2 s2 = fma2(a.y, a.y, fma2(a.x, a.x, dup2(1.17549435e-38f)));
   const float2 up = add2(a.z, dup2(1.0f)), down = sub2(dup2(1.0f), a.z);
   float2 f;
   {
@@ -463,8 +464,6 @@ __device__ __forceinline__ Vec2 update_direction_fast(const pp::PhaseDev& ph, co
     const float d0 = u0 ? up.x : s2.x, d1 = u1 ? up.y : s2.y;
     f = mul2(make_float2(u0 ? 1.0f : down.x, u1 ? 1.0f : down.y),
              make_float2(ftz_rcp(d0), ftz_rcp(d1)));
-    if (d0 < 1.17549435e-38f) f.x = 0.0f;
-    if (d1 < 1.17549435e-38f) f.y = 0.0f;
   }
   const float2 k = mul2(fma2(a.x, by, mul2(a.y, nbx)), f);
   const float2 nk = make_float2(-k.x, -k.y);

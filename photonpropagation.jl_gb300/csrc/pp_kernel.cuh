@@ -440,6 +440,12 @@ __device__ __forceinline__ float2 step_lengths(uint32_t w0, uint32_t w1, float2 
                 sca_len);
 }
 
+// An emission direction nearer to the z axis than FP32 can square counts as on
+// it, exactly, so that the step's rotation divides nothing by zero.
+__device__ __forceinline__ float3 on_axis(float3 d) {
+  return fmaf(d.y, d.y, d.x * d.x) < 1.17549435e-38f ? make_float3(0.0f, 0.0f, d.z) : d;
+}
+
 // The two photons' state, moved over one step.
 struct Walk2 {
   Vec2 pos, dir;
@@ -536,7 +542,8 @@ __device__ __noinline__ void replay_hit(const LaunchArgs& a, int s, uint32_t plo
                                         int k_hit, float4 target, Hit* out) {
   const PhotonInit in = init_photon<kPrecise>(a, s, plo, phi);
   const PhiloxPhoton ph = philox_photon(plo, (uint32_t)s, a.round_keys);
-  Walk2 w = {both(in.pos, in.pos), both(in.dir, in.dir), dup2(0.0f), dup2(0.0f)};
+  const float3 d0 = on_axis(in.dir);
+  Walk2 w = {both(in.pos, in.pos), both(d0, d0), dup2(0.0f), dup2(0.0f)};
   float2 step;
 #pragma unroll 1
   for (int k = 1;; ++k) {
@@ -632,11 +639,13 @@ __global__ void __launch_bounds__(kMaxBlockThreads, PP_PROPAGATE_MIN_BLOCKS)
         const PhotonInit in = init_photon<kPrecise>(a, s, j ? plo1 : plo0, phi);
         if (j == 0) {
           w.pos.x.x = in.pos.x; w.pos.y.x = in.pos.y; w.pos.z.x = in.pos.z;
-          w.dir.x.x = in.dir.x; w.dir.y.x = in.dir.y; w.dir.z.x = in.dir.z;
+          const float3 d = on_axis(in.dir);
+          w.dir.x.x = d.x; w.dir.y.x = d.y; w.dir.z.x = d.z;
           sca_len.x = in.med.x;
         } else {
           w.pos.x.y = in.pos.x; w.pos.y.y = in.pos.y; w.pos.z.y = in.pos.z;
-          w.dir.x.y = in.dir.x; w.dir.y.y = in.dir.y; w.dir.z.y = in.dir.z;
+          const float3 d = on_axis(in.dir);
+          w.dir.x.y = d.x; w.dir.y.y = d.y; w.dir.z.y = d.z;
           sca_len.y = in.med.x;
         }
       }

@@ -214,7 +214,7 @@ extern "C" PP_API int pp_propagate_static(
   pp::GridDev gshape;
   grid_shape(targets, n_targets, cell_size, &gshape);
   pp::SafetyDev sshape;
-  sshape.set_shape(gshape.lo, gshape.hi, pp::SafetyDev::auto_cell(gshape.lo, gshape.hi));
+  sshape.set_shape(gshape.lo, gshape.hi, pp::SafetyDev::auto_cell(gshape.lo, gshape.hi, n_targets));
   const int ppt = 8, block = 1024;
   const long long chunk = 32LL * ppt;
   std::vector<unsigned long long> prefix(n_src + 1, 0);
