@@ -184,14 +184,15 @@ int build_queue(pp_ctx* ctx) {
     nph[i] = source_photons(ctx->h_sources[i].photons, ctx->scaling);
     total += nph[i];
   }
-  // Small workloads: halve the photons per lane and chunk until there are at
-  // least two chunks for every warp the GPU holds at once (32 per SM), so
-  // that a 1e5-photon call is not run by a tenth of the warps.  Photons draw
-  // their random numbers by index, so the chunking changes no result.
+  // Small workloads: halve the photons per lane and chunk, down to one group of
+  // 64 per chunk, until there are at least two chunks for every warp the GPU
+  // holds at once, so that a 1e5-photon call is not run by a tenth of the warps.
+  // Photons draw their random numbers by index, so the chunking changes no
+  // result.
   int ppt = ctx->tuning.photons_per_thread;
   const long long resident_warps = (long long)pp::kSmWarps * std::max(ctx->num_sms, 1);
-  while (ppt > 1 && total / (32LL * ppt) < 2 * resident_warps) ppt /= 2;
-  const long long chunk = 32LL * ppt;
+  while (ppt > 2 && total / (32LL * ppt) < 2 * resident_warps) ppt /= 2;
+  const long long chunk = std::max<long long>(32LL * ppt, pp::kGroup);
   for (int i = 0; i < n; ++i)
     prefix[i + 1] = prefix[i] + (unsigned long long)((nph[i] + chunk - 1) / chunk);
   ctx->chunk_photons = (int)chunk;

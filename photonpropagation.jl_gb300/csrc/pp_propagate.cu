@@ -58,10 +58,9 @@ cudaError_t launch_propagate(const LaunchArgs& args, int block_threads, int ctas
   if (occ < 1) return cudaErrorInvalidConfiguration;
   const int per_sm = ctas_per_sm > 0 ? (ctas_per_sm < occ ? ctas_per_sm : occ) : occ;
   int grid = per_sm * num_sms;
-  // Never launch more warps than there are chunks of work.
-  const unsigned long long warps_per_cta = (unsigned long long)(threads / 32);
-  const unsigned long long need = (args.total_chunks + warps_per_cta - 1) / warps_per_cta;
-  if (need < (unsigned long long)grid) grid = (int)(need > 0 ? need : 1);
+  // Never launch more CTAs than there are chunks of work.
+  if (args.total_chunks < (unsigned long long)grid)
+    grid = (int)(args.total_chunks > 0 ? args.total_chunks : 1);
   if (grid_out) *grid_out = grid;
   void* params[] = {&a};
   return cudaLaunchKernel(k, dim3(grid), dim3(threads), params, smem, stream);
