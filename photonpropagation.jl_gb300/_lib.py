@@ -11,6 +11,8 @@ import os
 from ctypes import (POINTER, Structure, c_char_p, c_double, c_float, c_int32, c_int64,
                     c_uint32, c_uint64, c_void_p)
 
+import numpy as np
+
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG_DIR, "_lib", "libpp_gb300.so")
 
@@ -156,6 +158,24 @@ class pp_hits(Structure):
         ("abs_weight", c_void_p), ("module_index", c_void_p), ("n_steps", c_void_p),
         ("source_index", c_void_p), ("photon_index", c_void_p),
     ]
+
+
+def fill(dst, values) -> None:
+    """Copy an array into the leading elements of a structure's array member,
+    converted to its type as element-wise assignment would."""
+    a = np.ctypeslib.as_array(dst)
+    v = np.asarray(values, a.dtype)
+    if len(v) > len(a):
+        raise IndexError("invalid index")  # what assigning past the member's end raises
+    a[:len(v)] = v
+
+
+def records(dtype_struct, arr):
+    """A numpy structured array as the ctypes array of `dtype_struct` sharing its
+    memory."""
+    out = (dtype_struct * len(arr)).from_buffer(arr)
+    out._keep = arr
+    return out
 
 
 assert ctypes.sizeof(pp_source) == 96

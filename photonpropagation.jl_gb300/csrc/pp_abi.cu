@@ -147,11 +147,17 @@ struct pp_ctx {
   // sources and work queue
   std::vector<pp_source> h_sources;
   float scaling = 1.0f;
+  // one device buffer {sources, prefix, photons} and its host image (pinned when
+  // small), uploaded in one copy
+  unsigned char* d_queue = nullptr;
+  unsigned char* h_queue = nullptr;
+  std::vector<unsigned char> h_queue_big;
+  size_t queue_cap = 0;
+  bool queue_in_flight = false;  // the image may still be being read
   pp_source* d_sources = nullptr;
   unsigned long long* d_prefix = nullptr;
   long long* d_src_photons = nullptr;
   int n_src = 0;
-  int n_src_alloc = 0;
   unsigned long long total_chunks = 0;
   long long total_photons = 0;
   bool has_sources = false;
@@ -159,10 +165,14 @@ struct pp_ctx {
 
   pp_tuning tuning{1024, 8, 0, 0, 0.0f, 0, 0.0f, 0};
 
-  // scratch of pp_propagate
+  // scratch of pp_propagate: one device buffer {counters, hits} and a pinned
+  // host image of its first rows
+  unsigned char* d_result = nullptr;
   pp_hit_record* d_hits = nullptr;
   long long d_hits_cap = 0;
   pp_counters* d_ctr = nullptr;
+  unsigned char* h_result = nullptr;
+  long long h_rows = 0;  // hit rows of the last pp_propagate in h_result
   pp_hit_record* h_stage = nullptr;
   long long h_stage_cap = 0;
 
@@ -175,10 +185,41 @@ struct pp_ctx {
 
 namespace {
 
-int build_queue(pp_ctx* ctx) {
+// Results a pp_propagate call brings back with its counters in one copy: a small
+// call's hits all come with them, saving it a second round trip.
+constexpr size_t kHitsOffset = 128;  // of the hits in the result buffer
+constexpr long long kFirstRows = 256;
+constexpr size_t kPinnedQueue = 256 * 1024;
+
+// The work queue of ctx->h_sources on the device.  Without `wait` the upload is
+// only ordered before later work on ctx->stream.
+int build_queue(pp_ctx* ctx, bool wait = true) {
   const int n = (int)ctx->h_sources.size();
-  std::vector<unsigned long long> prefix(n + 1, 0);
-  std::vector<long long> nph(std::max(n, 1), 0);
+  auto up16 = [](size_t v) { return (v + 15) & ~(size_t)15; };
+  const size_t off_prefix = up16(sizeof(pp_source) * n);
+  const size_t off_photons = off_prefix + up16(sizeof(unsigned long long) * (n + 1));
+  const size_t bytes = off_photons + up16(sizeof(long long) * std::max(n, 1));
+  if (ctx->queue_in_flight) {
+    PP_CUDA(cudaStreamSynchronize(ctx->stream), "upload sources");
+    ctx->queue_in_flight = false;
+  }
+  if (bytes > ctx->queue_cap) {
+    cudaFree(ctx->d_queue);
+    ctx->d_queue = nullptr;
+    ctx->queue_cap = 0;
+    PP_CUDA(cudaMalloc(&ctx->d_queue, bytes), "cudaMalloc(sources)");
+    ctx->queue_cap = bytes;
+  }
+  // (pinning pays for small copies; a pageable one is taken before the call returns)
+  const bool pinned = bytes <= kPinnedQueue;
+  if (pinned && !ctx->h_queue)
+    PP_CUDA(cudaMallocHost(&ctx->h_queue, kPinnedQueue), "cudaMallocHost(sources)");
+  if (!pinned) ctx->h_queue_big.resize(bytes);
+  unsigned char* image = pinned ? ctx->h_queue : ctx->h_queue_big.data();
+  if (n > 0) memcpy(image, ctx->h_sources.data(), sizeof(pp_source) * n);
+  unsigned long long* prefix = reinterpret_cast<unsigned long long*>(image + off_prefix);
+  long long* nph = reinterpret_cast<long long*>(image + off_photons);
+  prefix[0] = 0;
   long long total = 0;
   for (int i = 0; i < n; ++i) {
     nph[i] = source_photons(ctx->h_sources[i].photons, ctx->scaling);
@@ -196,27 +237,16 @@ int build_queue(pp_ctx* ctx) {
   for (int i = 0; i < n; ++i)
     prefix[i + 1] = prefix[i] + (unsigned long long)((nph[i] + chunk - 1) / chunk);
   ctx->chunk_photons = (int)chunk;
-  if (n > ctx->n_src_alloc) {
-    cudaFree(ctx->d_sources);
-    cudaFree(ctx->d_prefix);
-    cudaFree(ctx->d_src_photons);
-    ctx->d_sources = nullptr;
-    ctx->d_prefix = nullptr;
-    ctx->d_src_photons = nullptr;
-    ctx->n_src_alloc = 0;
-    PP_CUDA(cudaMalloc(&ctx->d_sources, sizeof(pp_source) * n), "cudaMalloc(sources)");
-    PP_CUDA(cudaMalloc(&ctx->d_prefix, sizeof(unsigned long long) * (n + 1)), "cudaMalloc(prefix)");
-    PP_CUDA(cudaMalloc(&ctx->d_src_photons, sizeof(long long) * n), "cudaMalloc(photons)");
-    ctx->n_src_alloc = n;
-  }
+  ctx->d_sources = reinterpret_cast<pp_source*>(ctx->d_queue);
+  ctx->d_prefix = reinterpret_cast<unsigned long long*>(ctx->d_queue + off_prefix);
+  ctx->d_src_photons = reinterpret_cast<long long*>(ctx->d_queue + off_photons);
   if (n > 0) {
-    PP_CUDA(cudaMemcpyAsync(ctx->d_sources, ctx->h_sources.data(), sizeof(pp_source) * n,
-                            cudaMemcpyHostToDevice, ctx->stream), "upload sources");
-    PP_CUDA(cudaMemcpyAsync(ctx->d_prefix, prefix.data(), sizeof(unsigned long long) * (n + 1),
-                            cudaMemcpyHostToDevice, ctx->stream), "upload prefix");
-    PP_CUDA(cudaMemcpyAsync(ctx->d_src_photons, nph.data(), sizeof(long long) * n,
-                            cudaMemcpyHostToDevice, ctx->stream), "upload photon counts");
-    PP_CUDA(cudaStreamSynchronize(ctx->stream), "upload sources");
+    PP_CUDA(cudaMemcpyAsync(ctx->d_queue, image, bytes, cudaMemcpyHostToDevice, ctx->stream), "upload sources");
+    ctx->queue_in_flight = true;
+    if (wait) {
+      PP_CUDA(cudaStreamSynchronize(ctx->stream), "upload sources");
+      ctx->queue_in_flight = false;
+    }
   }
   ctx->n_src = n;
   ctx->total_chunks = prefix[n];
@@ -384,10 +414,12 @@ PP_API int pp_create(pp_ctx** out, int32_t device) {
   e = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->inflight, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaMalloc(&ctx->d_ctr, sizeof(pp_counters));
+  if (e == cudaSuccess)
+    e = cudaMallocHost(&ctx->h_result, kHitsOffset + sizeof(pp_hit_record) * kFirstRows);
   if (e != cudaSuccess) {
     int rc = cuda_error(e, "pp_create");
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
+    if (ctx->inflight) cudaEventDestroy(ctx->inflight);
     delete ctx;
     return rc;
   }
@@ -410,11 +442,10 @@ PP_API int pp_destroy(pp_ctx* ctx) {
   cudaFree(ctx->d_loop_spheres);
   cudaFree(ctx->d_blob);
   cudaFree(ctx->d_safety);
-  cudaFree(ctx->d_sources);
-  cudaFree(ctx->d_prefix);
-  cudaFree(ctx->d_src_photons);
-  cudaFree(ctx->d_hits);
-  cudaFree(ctx->d_ctr);
+  cudaFree(ctx->d_queue);
+  if (ctx->h_queue) cudaFreeHost(ctx->h_queue);
+  cudaFree(ctx->d_result);
+  if (ctx->h_result) cudaFreeHost(ctx->h_result);
   if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->inflight) cudaEventDestroy(ctx->inflight);
@@ -649,7 +680,7 @@ PP_API int pp_set_shaped_targets(pp_ctx* ctx, const pp_target* t, int32_t n) {
   return PP_OK;
 }
 
-PP_API int pp_set_sources(pp_ctx* ctx, const pp_source* s, int32_t n, float photon_scaling) {
+static int set_sources(pp_ctx* ctx, const pp_source* s, int32_t n, float photon_scaling, bool wait) {
   wait_launches(ctx);  // inputs of launches in flight are about to change
   if (!ctx || n < 0 || (n > 0 && !s)) return set_error(PP_ERR_INVALID, "bad source list");
   if (!(photon_scaling >= 0.0f) || !std::isfinite(photon_scaling))
@@ -677,9 +708,13 @@ PP_API int pp_set_sources(pp_ctx* ctx, const pp_source* s, int32_t n, float phot
   ctx->scaling = photon_scaling;
   ctx->needs_track = needs_track;
   ctx->max_smear_table = max_table;
-  int rc = build_queue(ctx);
+  int rc = build_queue(ctx, wait);
   ctx->has_sources = rc == PP_OK;
   return rc;
+}
+
+PP_API int pp_set_sources(pp_ctx* ctx, const pp_source* s, int32_t n, float photon_scaling) {
+  return set_sources(ctx, s, n, photon_scaling, true);
 }
 
 PP_API int pp_set_tuning(pp_ctx* ctx, const pp_tuning* t) {
@@ -852,28 +887,43 @@ PP_API int pp_propagate(pp_ctx* ctx, const pp_source* sources, int32_t n_src, in
   *n_hits = 0;
   *n_ph_sim = 0;
   ctx->last_hits = 0;
+  ctx->h_rows = 0;
   DeviceScope ds(ctx->device);
-  int rc = pp_set_sources(ctx, sources, n_src, photon_scaling);
-  if (rc != PP_OK) return rc;
-  rc = check_ready(ctx);
-  if (rc != PP_OK) return rc;
+  int rc = set_sources(ctx, sources, n_src, photon_scaling, false);
+  if (rc == PP_OK) rc = check_ready(ctx);
+  if (rc != PP_OK) {
+    cudaStreamSynchronize(ctx->stream);  // the sources are set all the same
+    return rc;
+  }
   // A photon hits at most once: the device buffer never needs more rows than
   // there are photons.
   const long long dev_cap = std::max<long long>(1, std::min<long long>(capacity, ctx->total_photons));
   if (dev_cap > ctx->d_hits_cap) {
-    cudaFree(ctx->d_hits);
-    ctx->d_hits = nullptr;
+    cudaFree(ctx->d_result);
+    ctx->d_result = nullptr;
     ctx->d_hits_cap = 0;
-    PP_CUDA(cudaMalloc(&ctx->d_hits, sizeof(pp_hit_record) * dev_cap), "cudaMalloc(hit buffer)");
+    const cudaError_t e =
+        cudaMalloc(&ctx->d_result, kHitsOffset + sizeof(pp_hit_record) * dev_cap);
+    if (e != cudaSuccess) {
+      cudaStreamSynchronize(ctx->stream);
+      return cuda_error(e, "cudaMalloc(hit buffer)");
+    }
+    ctx->d_ctr = reinterpret_cast<pp_counters*>(ctx->d_result);
+    ctx->d_hits = reinterpret_cast<pp_hit_record*>(ctx->d_result + kHitsOffset);
     ctx->d_hits_cap = dev_cap;
   }
   rc = enqueue(ctx, seed, n_steps, ctx->d_hits, std::min<long long>(capacity, dev_cap), ctx->d_ctr,
                ctx->stream);
   if (rc != PP_OK) return rc;
-  pp_counters c{};
-  PP_CUDA(cudaMemcpyAsync(&c, ctx->d_ctr, sizeof(c), cudaMemcpyDeviceToHost, ctx->stream),
+  const long long first = std::min<long long>(kFirstRows, ctx->d_hits_cap);
+  PP_CUDA(cudaMemcpyAsync(ctx->h_result, ctx->d_result,
+                          kHitsOffset + sizeof(pp_hit_record) * (size_t)first,
+                          cudaMemcpyDeviceToHost, ctx->stream),
           "read counters");
   PP_CUDA(cudaStreamSynchronize(ctx->stream), "propagate");
+  ctx->queue_in_flight = false;
+  pp_counters c;
+  memcpy(&c, ctx->h_result, sizeof(c));
   *n_hits = (int64_t)c.n_hits;
   *n_ph_sim = (int64_t)c.n_ph_sim;
   if (c.err_flags & PP_FLAG_TIMEOUT)
@@ -883,6 +933,7 @@ PP_API int pp_propagate(pp_ctx* ctx, const pp_source* sources, int32_t n_src, in
                      (unsigned long long)c.n_hits, (long long)capacity);
   const long long n = (long long)c.n_hits;
   ctx->last_hits = n;
+  ctx->h_rows = std::min(n, first);
   if (n == 0 || !out) return PP_OK;
   return fetch_hits(ctx, out, n);
 }
@@ -926,19 +977,23 @@ int fetch_hits(pp_ctx* ctx, const pp_hits* out, long long n) {
     if (e != cudaSuccess) return cuda_error(e, "hits_to_columns");
     return PP_OK;
   }
-  if (n > ctx->h_stage_cap) {
-    if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
-    ctx->h_stage = nullptr;
-    ctx->h_stage_cap = 0;
-    PP_CUDA(cudaMallocHost(&ctx->h_stage, sizeof(pp_hit_record) * n), "cudaMallocHost(stage)");
-    ctx->h_stage_cap = n;
+  const pp_hit_record* rows = reinterpret_cast<const pp_hit_record*>(ctx->h_result + kHitsOffset);
+  if (n > ctx->h_rows) {
+    if (n > ctx->h_stage_cap) {
+      if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
+      ctx->h_stage = nullptr;
+      ctx->h_stage_cap = 0;
+      PP_CUDA(cudaMallocHost(&ctx->h_stage, sizeof(pp_hit_record) * n), "cudaMallocHost(stage)");
+      ctx->h_stage_cap = n;
+    }
+    PP_CUDA(cudaMemcpyAsync(ctx->h_stage, ctx->d_hits, sizeof(pp_hit_record) * n,
+                            cudaMemcpyDeviceToHost, ctx->stream),
+            "copy hits");
+    PP_CUDA(cudaStreamSynchronize(ctx->stream), "copy hits");
+    rows = ctx->h_stage;
   }
-  PP_CUDA(cudaMemcpyAsync(ctx->h_stage, ctx->d_hits, sizeof(pp_hit_record) * n,
-                          cudaMemcpyDeviceToHost, ctx->stream),
-          "copy hits");
-  PP_CUDA(cudaStreamSynchronize(ctx->stream), "copy hits");
   for (long long i = 0; i < n; ++i) {
-    const pp_hit_record& h = ctx->h_stage[i];
+    const pp_hit_record& h = rows[i];
     for (int a = 0; a < 3; ++a) {
       if (out->position) out->position[3 * i + a] = h.position[a];
       if (out->direction) out->direction[3 * i + a] = h.direction[a];

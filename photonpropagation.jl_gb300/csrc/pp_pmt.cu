@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <cstring>
 #include <string>
+#include <vector>
 
 #include "pp_device.cuh"
 #include "pp_internal.h"
@@ -263,16 +264,15 @@ PP_API int pp_make_hits_from_photons_models(const pp_hit_record* d_records, int6
   const size_t ob_pom = tb, ob_dom = ob_pom + (pom ? up16(sizeof(pp_pom_model)) : 0);
   const size_t ob_mp = ob_dom + (dom ? up16(sizeof(pp_dom_model)) : 0);
   const size_t total = ob_mp + (mp ? up16(sizeof(pp_multipmt_model)) : 0);
+  std::vector<unsigned char> image(total);  // one copy (pageable: taken before the call returns)
+  if (n_targets > 0) memcpy(image.data(), targets, sizeof(pp_pmt_target) * n_targets);
+  if (pom) memcpy(image.data() + ob_pom, pom, sizeof(pp_pom_model));
+  if (dom) memcpy(image.data() + ob_dom, dom, sizeof(pp_dom_model));
+  if (mp) memcpy(image.data() + ob_mp, mp, sizeof(pp_multipmt_model));
   unsigned char* buf = nullptr;
   cudaError_t e = cudaMallocAsync((void**)&buf, total, s);
-  if (e == cudaSuccess && n_targets > 0)
-    e = cudaMemcpyAsync(buf, targets, sizeof(pp_pmt_target) * n_targets, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess && pom)
-    e = cudaMemcpyAsync(buf + ob_pom, pom, sizeof(pp_pom_model), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess && dom)
-    e = cudaMemcpyAsync(buf + ob_dom, dom, sizeof(pp_dom_model), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess && mp)
-    e = cudaMemcpyAsync(buf + ob_mp, mp, sizeof(pp_multipmt_model), cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(buf, image.data(), total, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) {
     if (buf) cudaFreeAsync(buf, s);
     return pp::report_error(PP_ERR_CUDA, std::string(kWho) + cudaGetErrorString(e));

@@ -44,25 +44,40 @@ def check_pmt_hit_opening_angle(rel_hit_position, pmt_positions, opening_angle) 
     return 0
 
 
+# the detection model of each module class, subclasses included
+_KINDS = ((POM, _lib.PP_PMT_POM), (DOM, _lib.PP_PMT_DOM),
+          (SphericalMultiPMTTarget, _lib.PP_PMT_MULTIPMT),
+          (HomogeneousDetector, _lib.PP_PMT_HOMOGENEOUS))
+_PMT_TARGET = np.dtype(_lib.pp_pmt_target)
+
+
+def _kind_of(cls):
+    for base, kind in _KINDS:
+        if issubclass(cls, base):
+            return kind
+    return None
+
+
 def pmt_targets(targets) -> "ctypes.Array":
     """pp_pmt_target per propagation target (index i -> module_index i + 1)."""
-    arr = (_lib.pp_pmt_target * max(1, len(targets)))()
-    for i, t in enumerate(targets):
-        p = np.asarray(t.shape.position, np.float32).reshape(3)
-        arr[i].position[:] = (float(p[0]), float(p[1]), float(p[2]))
-        arr[i].radius = float(np.float32(t.shape.radius))
-        arr[i].active_area = float(getattr(t, "pmt_area", 0.0))
-        if isinstance(t, POM):
-            arr[i].kind = _lib.PP_PMT_POM
-        elif isinstance(t, DOM):
-            arr[i].kind = _lib.PP_PMT_DOM
-        elif isinstance(t, SphericalMultiPMTTarget):
-            arr[i].kind = _lib.PP_PMT_MULTIPMT
-        elif isinstance(t, HomogeneousDetector):
-            arr[i].kind = _lib.PP_PMT_HOMOGENEOUS
-        else:
-            raise TypeError(f"target {i}: no detection model for {type(t).__name__}")
-    return arr
+    n = len(targets)
+    kind_of = {cls: _kind_of(cls) for cls in set(map(type, targets))}
+    for cls, kind in kind_of.items():
+        if kind is None:
+            i = next(i for i, t in enumerate(targets) if type(t) is cls)
+            raise TypeError(f"target {i}: no detection model for {cls.__name__}")
+    arr = np.zeros(max(1, n), _PMT_TARGET)
+    if n:
+        shapes = [t.shape for t in targets]
+        try:
+            pos = np.array([s.position for s in shapes], np.float32).reshape(n, 3)
+        except ValueError:  # positions of different array shapes
+            pos = np.stack([np.asarray(s.position, np.float32).reshape(3) for s in shapes])
+        arr["position"][:n] = pos
+        arr["radius"][:n] = [s.radius for s in shapes]
+        arr["active_area"][:n] = [getattr(t, "pmt_area", 0.0) for t in targets]
+        arr["kind"][:n] = [kind_of[type(t)] for t in targets]
+    return _lib.records(_lib.pp_pmt_target, arr)
 
 
 def detection_models(targets, orientation=None, apply_wl_acc: bool = True):
@@ -70,15 +85,16 @@ def detection_models(targets, orientation=None, apply_wl_acc: bool = True):
     present in `targets`; keep the second item alive for the call."""
     keep = []
     models = _lib.pp_detection_models()
-    if any(isinstance(t, POM) for t in targets):
+    present = {_kind_of(cls) for cls in set(map(type, targets))}
+    if _lib.PP_PMT_POM in present:
         keep.append(pom_model(orientation))
         models.pom = ctypes.pointer(keep[-1])
-    doms = [t for t in targets if isinstance(t, DOM)]
-    if doms:
-        keep.append(dom_model(doms[0].acceptance, orientation, apply_wl_acc))
+    if _lib.PP_PMT_DOM in present:
+        dom = next(t for t in targets if isinstance(t, DOM))
+        keep.append(dom_model(dom.acceptance, orientation, apply_wl_acc))
         models.dom = ctypes.pointer(keep[-1])
-    mps = [t for t in targets if isinstance(t, SphericalMultiPMTTarget)]
-    if mps:
+    if _lib.PP_PMT_MULTIPMT in present:
+        mps = [t for t in targets if isinstance(t, SphericalMultiPMTTarget)]
         keep.append(multipmt_model(mps, orientation))
         models.multipmt = ctypes.pointer(keep[-1])
     return models, keep

@@ -84,13 +84,12 @@ def dom_model(acceptance: DOMAcceptance | None = None, orientation=None,
     m = _lib.pp_dom_model()
     m.n_poly = len(a.poly)
     m.n_wl = len(a.wl)
-    for i, c in enumerate(np.asarray(a.poly, np.float32)):
-        m.poly[i] = float(c)
+    _lib.fill(m.poly, a.poly)
     m.polymax = float(a.polymax)
     R = np.eye(3) if orientation is None else np.asarray(orientation, np.float64)
     m.zenith_axis[:] = [float(v) for v in R[:, 2].astype(np.float32)]
-    for i, (x, y) in enumerate(zip(np.asarray(a.wl, np.float32), np.asarray(a.wl_acc, np.float32))):
-        m.wl[i] = float(x)
-        m.wl_acc[i] = float(y)
+    n = min(len(a.wl), len(a.wl_acc))
+    _lib.fill(m.wl, a.wl[:n])
+    _lib.fill(m.wl_acc, a.wl_acc[:n])
     m.apply_wl_acceptance = 1 if apply_wl_acc else 0
     return m

@@ -127,8 +127,12 @@ def multipmt_model(targets: Sequence[SphericalMultiPMTTarget],
     """pp_multipmt_model shared by the multi-PMT modules of one detection call
     (they must share PMT layout, area and QE table)."""
     t0 = targets[0]
-    key = _layout_key(t0)
-    if any(_layout_key(t) != key for t in targets[1:]):
+    # (modules usually share the very arrays; else they are compared by value)
+    other = [t for t in targets[1:] if not (t.pmt_area == t0.pmt_area and
+                                            t.pmt_coordinates is t0.pmt_coordinates and
+                                            t.wl_acceptance is t0.wl_acceptance)]
+    key = _layout_key(t0) if other else None
+    if any(_layout_key(t) != key for t in other):
         raise ValueError("multi-PMT modules of one call must share PMT layout, area and QE")
     n = get_pmt_count(t0)
     if not 1 <= n <= _lib.PP_MULTIPMT_MAX_PMTS:
@@ -142,10 +146,9 @@ def multipmt_model(targets: Sequence[SphericalMultiPMTTarget],
     m.pmt_area = float(t0.pmt_area)
     dm = get_pmt_positions(t0).astype(np.float32)
     do = get_pmt_positions(t0, orientation).astype(np.float32)
-    for i in range(n):
-        m.pmt_dir_module[i][:] = [float(v) for v in dm[i]]
-        m.pmt_dir[i][:] = [float(v) for v in do[i]]
-    for i, (x, y) in enumerate(zip(np.asarray(qwl, np.float32), np.asarray(qv, np.float32))):
-        m.qe_wavelength[i] = float(x)
-        m.qe[i] = float(y)
+    _lib.fill(m.pmt_dir_module, dm)
+    _lib.fill(m.pmt_dir, do)
+    k = min(len(qwl), len(qv))
+    _lib.fill(m.qe_wavelength, qwl[:k])
+    _lib.fill(m.qe, qv[:k])
     return m

@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import os
 from dataclasses import dataclass
+from functools import lru_cache
 from typing import Sequence
 
 import numpy as np
@@ -76,11 +77,17 @@ def make_pom_pmt_coordinates() -> np.ndarray:
     return c
 
 
+@lru_cache(maxsize=1)
+def _module_directions() -> np.ndarray:
+    """The 16 unit vectors in the module frame: a constant."""
+    c = make_pom_pmt_coordinates()
+    return np.stack([_sph_to_cart(c[0, i], c[1, i]) for i in range(16)])
+
+
 def pom_pmt_directions(orientation=None) -> np.ndarray:
     """16 x 3 PMT unit vectors in the detector frame (orientation * the module
     frame; identity by default, as the reference's RotMatrix3(I))."""
-    c = make_pom_pmt_coordinates()
-    d = np.stack([_sph_to_cart(c[0, i], c[1, i]) for i in range(16)])
+    d = _module_directions().copy()
     if orientation is not None:
         d = d @ np.asarray(orientation, float).T
     return d
@@ -97,10 +104,17 @@ class POMTables:
     qe: np.ndarray
 
 
-def load_pom_tables() -> POMTables:
+@lru_cache(maxsize=1)
+def _table_files():
+    """The packaged CSVs, parsed once."""
     a = np.loadtxt(os.path.join(_DATA, "pom_pmt_acceptance.csv"), delimiter=",", skiprows=1)
     s = np.loadtxt(os.path.join(_DATA, "pom_pmt_sigma.csv"), delimiter=",", skiprows=1)
     q = np.loadtxt(os.path.join(_DATA, "pom_rel_qe.csv"), delimiter=",", skiprows=1)
+    return a, s, q
+
+
+def load_pom_tables() -> POMTables:
+    a, s, q = (t.copy() for t in _table_files())
     return POMTables(a[:, 0], a[:, 1], a[:, 2], float(s[0]), float(s[1]), q[:, 0], q[:, 1])
 
 
@@ -112,16 +126,11 @@ def pom_model(orientation=None, tables: POMTables | None = None) -> "_lib.pp_pom
     for name, arr in (("acc_wavelength", t.acc_wavelength), ("acc_group1", t.acc_group1),
                       ("acc_group2", t.acc_group2), ("qe_wavelength", t.qe_wavelength),
                       ("qe", t.qe)):
-        dst = getattr(m, name)
-        for i, v in enumerate(np.asarray(arr, np.float32)):
-            dst[i] = float(v)
+        _lib.fill(getattr(m, name), arr)
     m.sigma_group1 = t.sigma_group1
     m.sigma_group2 = t.sigma_group2
-    d = pom_pmt_directions(orientation).astype(np.float32)
-    for i in range(16):
-        for k in range(3):
-            m.pmt_dir[i][k] = float(d[i, k])
-        m.pmt_group[i] = int(POM_PMT_GROUP[i])
+    _lib.fill(m.pmt_dir, pom_pmt_directions(orientation))
+    _lib.fill(m.pmt_group, POM_PMT_GROUP)
     return m
 
 

@@ -191,7 +191,9 @@ def generate_tables(pairs: Pairs, photons: int, seed: int = 1, ctx=None, medium=
     hists = torch.empty((n, N_BINS), dtype=torch.float32, device="cuda")
     ctr = torch.zeros(64, dtype=torch.uint8, device="cuda")
     tgeo_all = torch.tensor(geometric_time(pairs, medium), dtype=torch.float32, device="cuda")
-    table_setup(pairs.subset(slice(0, 1)), photons, seed, medium, spectrum).upload(ctx)
+    setup = table_setup(pairs.subset(slice(0, 1)), photons, seed, medium, spectrum)
+    if not setup.is_uploaded(ctx):  # by value: a context used for the last batch has it all
+        setup.upload(ctx)
     for lo in range(0, n, chunk):
         hi = min(n, lo + chunk)
         ctx.set_sources(cascade_records(pairs.subset(slice(lo, hi)), photons), hi - lo, 1.0)
