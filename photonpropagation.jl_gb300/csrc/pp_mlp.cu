@@ -26,6 +26,7 @@
 
 #include "pp_device.cuh"
 #include "pp_internal.h"
+#include "pp_mlp_rows.cuh"
 #include "pp_tc.cuh"
 
 using bf16 = __nv_bfloat16;
@@ -1228,6 +1229,15 @@ struct pp_mlp {
              total == o.total && B == o.B && lr0 == o.lr0 && lr1 == o.lr1 && seed == o.seed;
     }
   } graph_key{};
+  // The three-kernel training step (pp_mlp_rows.cuh), for the shapes it takes:
+  // the weight packs, the tiles of one batch and the accumulators between steps.
+  bool rows_path = false;
+  uint32_t rows_act = 0;                // bytes of one activation buffer
+  std::vector<uint32_t> wf_off, wb_off;
+  unsigned char *wf = nullptr, *wb = nullptr, *tiles = nullptr;
+  float* loss_acc = nullptr;
+  pprows::TrainCtl* ctl = nullptr;
+  bool g_dirty = false;                 // the gradient accumulators are not zero
 };
 
 namespace {
@@ -1237,6 +1247,7 @@ void mlp_free(pp_mlp* m) {
   cudaFree(m->X0); cudaFree(m->O); cudaFree(m->dO16);
   cudaFree(m->dZ[0]); cudaFree(m->dZ[1]); cudaFree(m->loss); cudaFree(m->err);
   cudaFree(m->wpack);
+  cudaFree(m->wf); cudaFree(m->wb); cudaFree(m->tiles); cudaFree(m->loss_acc); cudaFree(m->ctl);
   cudaFree(m->bx); cudaFree(m->bc); cudaFree(m->bh); cudaFree(m->d_step); cudaFree(m->d_sched);
   if (m->step_graph) cudaGraphExecDestroy(m->step_graph);
   if (m->cap_stream) cudaStreamDestroy(m->cap_stream);
@@ -1384,8 +1395,144 @@ int check_err(pp_mlp* m, cudaStream_t s) {
   if (e != cudaSuccess) return cuda_fail(e, "mlp");
   if (h) {
     cudaMemsetAsync(m->err, 0, sizeof(unsigned), s);
+    m->g_dirty = true;
     return fail(PP_ERR_TIMEOUT, "a tensor-core wait timed out");
   }
+  return PP_OK;
+}
+
+// ---- the three-kernel training step --------------------------------------------
+
+// The shapes rows_kernel takes: hidden widths that split into two halves of whole
+// 64-column chunks, one chunk of inputs, four 8-column blocks of outputs per
+// thread of the loss.  Others train layer by layer.
+void rows_setup(pp_mlp* m) {
+  m->rows_path = (m->hidden == 128 || m->hidden == 256) && m->in_pad <= pprows::kChunk &&
+                 m->out_pad <= 128;
+  m->rows_act = (uint32_t)(pprows::kRows * std::max(m->hidden, m->out_pad) * 2);
+}
+size_t rows_smem(const pp_mlp* m) {
+  return 2 * (size_t)m->rows_act + (size_t)(m->hidden / pprows::kChunk) * pprows::kSlotBytes;
+}
+size_t dw_smem() { return (size_t)pprows::kDwStages * pprows::kDwStageBytes; }
+cudaError_t rows_attributes(const pp_mlp* m) {
+  const void* k = m->hidden == 256 ? (const void*)pprows::rows_kernel<256>
+                                   : (const void*)pprows::rows_kernel<128>;
+  cudaError_t e =
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem(m));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(pprows::dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)dw_smem());
+  return e;
+}
+
+// Blocks of one batch, carved from m->tiles: inputs, the layers' activations,
+// pre-activations and their gradients, the head's gradient.
+struct RowsTiles {
+  unsigned char *x0, *y, *z, *dz, *dout;
+  size_t layer, total;
+};
+RowsTiles rows_tiles(const pp_mlp* m) {
+  const size_t rows = ((size_t)m->max_batch + pprows::kRows - 1) / pprows::kRows * pprows::kRows;
+  RowsTiles t{};
+  t.layer = rows * m->hidden * 2;
+  unsigned char* p = m->tiles;
+  t.x0 = p; p += rows * m->in_pad * 2;
+  t.dout = p; p += rows * m->out_pad * 2;
+  t.y = p; p += t.layer * m->n_layers;
+  t.z = p; p += t.layer * m->n_layers;
+  t.dz = p; p += t.layer * m->n_layers;
+  t.total = (size_t)(p - m->tiles);
+  return t;
+}
+
+// Forward, loss and all gradients of a batch into m->G and m->loss_acc (which
+// are zero before): rows 0 .. B - 1 of the arrays, or B rows drawn from n_table.
+// `schedule`: also the captured step's step size.
+int rows_gradients(pp_mlp* m, const float* x, const float* count, const float* hist,
+                   long long n_table, int B, bool schedule, cudaStream_t s) {
+  const RowsTiles t = rows_tiles(m);
+  const int L = m->n_layers;
+  pprows::RowsParams p{};
+  p.x = x; p.count = count; p.hist = hist; p.n_table = n_table; p.ctl = m->ctl;
+  p.B = B; p.n_in = m->n_in; p.in_pad = m->in_pad; p.hidden = m->hidden; p.n_layers = L;
+  p.out_pad = m->out_pad; p.n_bins = m->n_bins;
+  p.inv_b = 1.0f / (float)B; p.time_weight = m->time_weight;
+  p.wf = m->wf; p.wb = m->wb;
+  for (int l = 0; l <= L; ++l) {
+    p.wf_off[l] = m->wf_off[l];
+    p.wb_off[l] = m->wb_off[l];
+    p.bias[l] = m->P + m->off_b[l];
+  }
+  p.x0 = t.x0; p.y = t.y; p.z = t.z; p.dz = t.dz; p.dout = t.dout; p.layer_bytes = t.layer;
+  p.gbias = m->G + m->off_b[L]; p.loss = m->loss_acc;
+  p.act_bytes = m->rows_act; p.err = m->err; p.wait_ns = kWaitNs;
+  const dim3 grid((unsigned)((B + pprows::kRows - 1) / pprows::kRows));
+  auto* k = m->hidden == 256 ? pprows::rows_kernel<256> : pprows::rows_kernel<128>;
+  cudaError_t e = launch_pdl(k, grid, dim3(pprows::kRowsThreads), rows_smem(m), s, p);
+  if (e != cudaSuccess) return cuda_fail(e, "training rows");
+
+  pprows::DwParams d{};
+  const int cb = m->hidden / 128;  // 128-column tiles of a hidden layer
+  for (int l = 0; l <= L; ++l) {
+    const int mt = l < L ? cb : 1, nt = l == 0 ? 1 : cb;
+    for (int i = 0; i < mt; ++i)
+      for (int j = 0; j < nt; ++j) {
+        // (128 columns of a block of 8-row groups are 128 * 16 bytes apart)
+        pprows::DwTile& w = d.tile[d.n_tiles++];
+        w.a = l < L ? t.dz + (size_t)l * t.layer + (size_t)i * 2048 : t.dout;
+        w.a_cols = l < L ? m->hidden : m->out_pad;
+        w.rows = l < L ? 128 : m->out_pad;
+        w.b = l == 0 ? t.x0 : t.y + (size_t)(l - 1) * t.layer + (size_t)j * 2048;
+        w.b_cols = l == 0 ? m->in_pad : m->hidden;
+        w.cols = l == 0 ? m->in_pad : 128;
+        w.out = m->G + m->off_w[l] + (size_t)i * 128 * m->cols[l] + (size_t)j * 128;
+        w.ldc = m->cols[l];
+        w.bias = l < L && j == 0 ? m->G + m->off_b[l] + i * 128 : nullptr;
+      }
+  }
+  d.n_blocks = (int)grid.x;
+  const int splits = std::max(1, std::min(d.n_blocks, m->num_sms / d.n_tiles));
+  d.blocks_per_split = (d.n_blocks + splits - 1) / splits;
+  d.err = m->err; d.wait_ns = kWaitNs;
+  d.sched = schedule ? m->d_sched : nullptr; d.ctl = m->ctl; d.b1 = m->b1; d.b2 = m->b2;
+  const int used = (d.n_blocks + d.blocks_per_split - 1) / d.blocks_per_split;
+  e = launch_pdl(pprows::dw_kernel, dim3((unsigned)(d.n_tiles * used)), dim3(pprows::kDwThreads),
+                 dw_smem(), s, d);
+  if (e != cudaSuccess) return cuda_fail(e, "weight gradients");
+  return PP_OK;
+}
+
+pprows::AdamParams rows_adam(pp_mlp* m) {
+  pprows::AdamParams p{};
+  p.w = m->P; p.g = m->G; p.m = m->Mo; p.v = m->Vo; p.n = m->n_params;
+  p.b1 = m->b1; p.b2 = m->b2; p.eps = m->eps;
+  p.w16 = m->P16; p.wf = m->wf; p.wb = m->wb;
+  p.n_layers = m->n_layers;
+  for (int l = 0; l <= m->n_layers; ++l)
+    p.layer[l] = {m->off_w[l], m->off_b[l], m->rows[l], m->cols[l], m->wf_off[l], m->wb_off[l]};
+  p.loss_acc = m->loss_acc; p.loss = m->loss;
+  return p;
+}
+// The BF16 copies of the FP32 parameters.
+void refresh_bf16(pp_mlp* m) {
+  if (m->rows_path)
+    pprows::pack_kernel<<<(unsigned)((m->n_params + 1023) / 1024), 256>>>(rows_adam(m));
+  else
+    to_bf16_kernel<<<(unsigned)((m->n_params + 255) / 256), 256>>>(m->P, m->n_params, m->P16);
+}
+int rows_step(pp_mlp* m, const pprows::AdamParams& p, cudaStream_t s) {
+  const cudaError_t e = launch_pdl(pprows::adam_kernel,
+                                   dim3((unsigned)((m->n_params + 1023) / 1024)), dim3(256), 0, s,
+                                   p);
+  return e == cudaSuccess ? PP_OK : cuda_fail(e, "adam");
+}
+int rows_clear(pp_mlp* m, cudaStream_t s) {
+  const cudaError_t e = launch_pdl(pprows::clear_kernel,
+                                   dim3((unsigned)((m->n_params + 255) / 256)), dim3(256), 0, s,
+                                   m->G, m->n_params, m->loss_acc, m->loss);
+  if (e != cudaSuccess) return cuda_fail(e, "clear gradients");
+  m->g_dirty = false;
   return PP_OK;
 }
 
@@ -1470,12 +1617,34 @@ PP_API int pp_mlp_create(pp_mlp** out, int32_t device, int32_t n_in, int32_t hid
     wbytes += (long long)m->rows[l] * m->cols[l] * 2;  // rows, cols multiples of 16: 512-byte steps
   }
   A((void**)&m->wpack, (size_t)wbytes);
+  rows_setup(m);
+  if (m->rows_path) {
+    // each pack holds every weight once; blocks start at multiples of 16 bytes
+    uint32_t wf = 0, wb = 0;
+    for (int l = 0; l <= n_layers; ++l) {
+      m->wf_off.push_back(wf);
+      m->wb_off.push_back(wb);
+      wf += (uint32_t)(m->rows[l] * m->cols[l] * 2);
+      if (l > 0) wb += (uint32_t)(m->rows[l] * m->cols[l] * 2);
+    }
+    A((void**)&m->wf, wf);
+    A((void**)&m->wb, std::max(wb, 16u));
+    A((void**)&m->tiles, rows_tiles(m).total);
+    A((void**)&m->loss_acc, sizeof(float));
+    A((void**)&m->ctl, sizeof(pprows::TrainCtl));
+    A((void**)&m->d_sched, sizeof(float) * 4);
+    if (e == cudaSuccess) e = cudaMemset(m->loss_acc, 0, sizeof(float));
+    if (e == cudaSuccess) e = cudaMemset(m->G, 0, pb);
+    if (e == cudaSuccess)
+      e = cudaDeviceGetAttribute(&m->num_sms, cudaDevAttrMultiProcessorCount, device);
+    if (e == cudaSuccess) e = rows_attributes(m);
+  }
   if (e == cudaSuccess) e = cudaMemcpy(m->P, h.data(), pb, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(m->Mo, 0, pb);
   if (e == cudaSuccess) e = cudaMemset(m->Vo, 0, pb);
   if (e == cudaSuccess) e = cudaMemset(m->err, 0, sizeof(unsigned));
   if (e == cudaSuccess) {
-    to_bf16_kernel<<<(unsigned)((off + 255) / 256), 256>>>(m->P, off, m->P16);
+    refresh_bf16(m);
     e = cudaDeviceSynchronize();
   }
   if (e != cudaSuccess) {
@@ -1526,7 +1695,7 @@ PP_API int pp_mlp_set_params(pp_mlp* m, const float* host, int64_t n) {
   cudaSetDevice(m->device);
   cudaError_t e = cudaMemcpy(m->P, host, sizeof(float) * n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) {
-    to_bf16_kernel<<<(unsigned)((n + 255) / 256), 256>>>(m->P, n, m->P16);
+    refresh_bf16(m);
     e = cudaDeviceSynchronize();
   }
   m->pack_dirty = true;
@@ -1555,12 +1724,20 @@ PP_API int pp_mlp_loss_grad(pp_mlp* m, const float* d_x, const float* d_count,
     return fail(PP_ERR_INVALID, "bad arguments");
   cudaSetDevice(m->device);
   cudaStream_t s = (cudaStream_t)stream;
-  int rc = mlp_forward(m, d_x, B, s);
-  if (rc == PP_OK) rc = mlp_backward(m, d_count, d_hist, B, s);
+  int rc = PP_OK;
+  if (m->rows_path) {
+    if (m->g_dirty) rc = rows_clear(m, s);
+    m->g_dirty = true;
+    if (rc == PP_OK) rc = rows_gradients(m, d_x, d_count, d_hist, 0, B, false, s);
+  } else {
+    rc = mlp_forward(m, d_x, B, s);
+    if (rc == PP_OK) rc = mlp_backward(m, d_count, d_hist, B, s);
+  }
   if (rc != PP_OK) return rc;
   cudaError_t e = cudaSuccess;
   if (host_grad) e = cudaMemcpyAsync(host_grad, m->G, sizeof(float) * m->n_params,
                                      cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess && m->rows_path && (rc = rows_clear(m, s)) != PP_OK) return rc;
   if (e == cudaSuccess && host_loss)
     e = cudaMemcpyAsync(host_loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost, s);
   if (e != cudaSuccess) return cuda_fail(e, "copy gradients");
@@ -1575,8 +1752,15 @@ PP_API int pp_mlp_train_step(pp_mlp* m, const float* d_x, const float* d_count,
     return fail(PP_ERR_INVALID, "bad arguments");
   cudaSetDevice(m->device);
   cudaStream_t s = (cudaStream_t)stream;
-  int rc = mlp_forward(m, d_x, B, s);
-  if (rc == PP_OK) rc = mlp_backward(m, d_count, d_hist, B, s);
+  int rc = PP_OK;
+  if (m->rows_path) {
+    if (m->g_dirty) rc = rows_clear(m, s);
+    m->g_dirty = true;
+    if (rc == PP_OK) rc = rows_gradients(m, d_x, d_count, d_hist, 0, B, false, s);
+  } else {
+    rc = mlp_forward(m, d_x, B, s);
+    if (rc == PP_OK) rc = mlp_backward(m, d_count, d_hist, B, s);
+  }
   if (rc != PP_OK) return rc;
   m->step += 1;
   // bias corrections in double, rounded once: the captured step's
@@ -1585,6 +1769,14 @@ PP_API int pp_mlp_train_step(pp_mlp* m, const float* d_x, const float* d_count,
   // differ by an ulp, ~2e-5 of bc2 at small t)
   const float bc1 = (float)(1.0 - std::pow((double)m->b1, (double)m->step));
   const float bc2 = (float)(1.0 - std::pow((double)m->b2, (double)m->step));
+  if (m->rows_path) {
+    pprows::AdamParams p = rows_adam(m);
+    p.lr = lr; p.bc1 = bc1; p.bc2 = bc2;
+    if ((rc = rows_step(m, p, s)) != PP_OK) return rc;
+    m->g_dirty = false;
+    m->pack_dirty = true;
+    return PP_OK;
+  }
   cudaError_t ea = launch_pdl(adam_kernel, dim3((unsigned)((m->n_params + 255) / 256)), dim3(256),
                               0, s, m->P, (const float*)m->G, m->Mo, m->Vo, m->n_params, lr,
                               m->b1, m->b2, m->eps, bc1, bc2, m->P16);
@@ -1615,11 +1807,11 @@ int capture_train_step(pp_mlp* m, const pp_mlp::GraphKey& k) {
   cudaStream_t cs = m->cap_stream;
   e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return cuda_fail(e, "begin capture");
+  int rc = PP_OK;
   // (the first kernel of a step is launched plainly: it follows the previous
   // graph launch)
   schedule_kernel<<<1, 1, 0, cs>>>(m->d_step, k.step0, k.total, k.lr0, k.lr1, m->b1, m->b2,
                                    m->d_sched);
-  int rc = PP_OK;
   e = launch_pdl(gather_kernel, dim3((unsigned)((k.B + 7) / 8)), dim3(256), 0, cs, k.x, k.c, k.h,
                  (long long)k.n_rows, m->n_in, m->n_bins, k.B, (const long long*)m->d_step,
                  (uint32_t)k.seed, (uint32_t)(k.seed >> 32), m->bx, m->bc, m->bh);
@@ -1660,18 +1852,43 @@ PP_API int pp_mlp_train_steps(pp_mlp* m, const float* d_x, const float* d_count,
     return fail(PP_ERR_INVALID, "pp_mlp_train_steps: bad arguments");
   if (n_steps == 0) return PP_OK;
   cudaSetDevice(m->device);
-  const pp_mlp::GraphKey k{d_x, d_count, d_hist, (long long)n_rows, (long long)step0,
-                           (long long)total, (int)B, lr0, lr1, (unsigned long long)seed};
-  if (!m->step_graph || !(m->graph_key == k)) {
-    const int rc = capture_train_step(m, k);
-    if (rc != PP_OK) return rc;
-  }
   cudaStream_t s = (cudaStream_t)stream;
-  // the device counter continues from the host's count
-  set_step_kernel<<<1, 1, 0, s>>>(m->d_step, m->step);
-  cudaError_t e = cudaGetLastError();
-  for (int i = 0; e == cudaSuccess && i < n_steps; ++i) e = cudaGraphLaunch(m->step_graph, s);
-  if (e != cudaSuccess) return cuda_fail(e, "pp_mlp_train_steps");
+  if (m->rows_path) {
+    // Three launches a step, each overlapping the tail of the one before; the
+    // schedule, the step count and the batch stream's key are device data.  (A
+    // capture would replay this call's step count.)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(s, &capture);
+    if (e == cudaSuccess && capture != cudaStreamCaptureStatusNone)
+      e = cudaErrorStreamCaptureUnsupported;
+    if (e != cudaSuccess) return cuda_fail(e, "pp_mlp_train_steps");
+    int rc = m->g_dirty ? rows_clear(m, s) : PP_OK;
+    m->g_dirty = true;
+    const pprows::TrainCtl c{m->step, (long long)step0, (long long)total, lr0, lr1,
+                             (uint32_t)seed, (uint32_t)(seed >> 32)};
+    pprows::set_ctl_kernel<<<1, 1, 0, s>>>(m->ctl, c);
+    pprows::AdamParams p = rows_adam(m);
+    p.sched = m->d_sched;
+    p.ctl = m->ctl;
+    for (int i = 0; rc == PP_OK && i < n_steps; ++i) {
+      rc = rows_gradients(m, d_x, d_count, d_hist, n_rows, B, true, s);
+      if (rc == PP_OK) rc = rows_step(m, p, s);
+    }
+    if (rc != PP_OK) return rc;
+    m->g_dirty = false;
+  } else {
+    const pp_mlp::GraphKey k{d_x, d_count, d_hist, (long long)n_rows, (long long)step0,
+                             (long long)total, (int)B, lr0, lr1, (unsigned long long)seed};
+    if (!m->step_graph || !(m->graph_key == k)) {
+      const int rc = capture_train_step(m, k);
+      if (rc != PP_OK) return rc;
+    }
+    // the device counter continues from the host's count
+    set_step_kernel<<<1, 1, 0, s>>>(m->d_step, m->step);
+    cudaError_t e = cudaGetLastError();
+    for (int i = 0; e == cudaSuccess && i < n_steps; ++i) e = cudaGraphLaunch(m->step_graph, s);
+    if (e != cudaSuccess) return cuda_fail(e, "pp_mlp_train_steps");
+  }
   m->step += n_steps;
   m->pack_dirty = true;
   return PP_OK;

@@ -127,6 +127,20 @@ __device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
   return done != 0;
 }
 
+// Whether phase `parity` has completed, at once (a try may suspend the thread for
+// microseconds when it has not).
+__device__ __forceinline__ bool mbar_test(uint32_t a, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(a), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+
 // Wait for phase `parity` of the mbarrier for at most limit_ns.  A phase that
 // has already completed costs one try_wait: the clock is read only when the
 // first try fails (a single-thread MMA issuer has about 128 cycles per
