@@ -588,6 +588,7 @@ __global__ void repack_kernel(const float* __restrict__ w, int rows, int cols, f
 }
 
 constexpr int kMaxLayers = 17;
+constexpr int kMaxChunks = 256 / kChunkK;       // of a layer's input
 constexpr size_t kMaxInferSmem = 232448 - 256;  // 227 KB opt-in less the static barriers
 constexpr int kEpiWarps = 16;                        // epilogue warps (4 per TMEM lane quarter)
 constexpr int kEpiThreads = kEpiWarps * 32;
@@ -623,21 +624,31 @@ struct InferParams {
 // tiles past the last row are evaluated on zero rows and not stored.
 struct JobIter {
   int step = -1, slot = 0, layer = 0, round = 0;
+  int layer_of[2] = {0, 0}, round_of[2] = {0, 0};  // the slots' next jobs
   __device__ int tile() const { return (round * (int)gridDim.x + (int)blockIdx.x) * 2 + slot; }
   // advance to the next job; false when the CTA's work is done
   __device__ bool next(const InferParams& p) {
-    const int per_tile = p.n_layers + 1;
-    const int lag = per_tile / 2;
+    const int lag = (p.n_layers + 1) / 2;
     while (true) {
       ++step;
       slot = step & 1;
-      const int q = (step >> 1) - (slot ? lag : 0);
-      if (q < 0) continue;
-      round = q / per_tile;
-      layer = q - round * per_tile;
-      if (round < p.n_rounds) return true;
-      if (slot == 1) return false;  // slot 1 finishes last
+      if (slot == 0) {
+        if (!take(p, layer_of[0], round_of[0])) continue;
+        return true;
+      }
+      if ((step >> 1) < lag) continue;
+      return take(p, layer_of[1], round_of[1]);  // slot 1 finishes last
     }
+  }
+  __device__ bool take(const InferParams& p, int& l, int& r) {
+    layer = l;
+    round = r;
+    if (r >= p.n_rounds) return false;
+    if (++l > p.n_layers) {
+      l = 0;
+      ++r;
+    }
+    return true;
   }
 };
 
@@ -667,61 +678,50 @@ __device__ __forceinline__ void pack_input(const InferParams& p, unsigned char* 
   }
 }
 
-// b/2 of columns cb + 2 (lane % 16) and + 1 in FP32 (0 past the layer's
-// width; halving is exact): the bias operand of silu_slice, loaded before the
-// accumulator wait so that its latency is hidden.
-__device__ __forceinline__ float2 bias_pair(const float* __restrict__ b, int cb, int hidden,
-                                            int lane) {
-  const int c = cb + 2 * (lane & 15);
-  return c < hidden ? make_float2(0.5f * __ldg(b + c), 0.5f * __ldg(b + c + 1))
-                    : make_float2(0.0f, 0.0f);
+// 16 columns of a warp's 32 TMEM lanes, two 16x256b loads of 16 lanes: v[8 m + 4 q +
+// 2 k] and + 1 are columns 8 q + 2 (lane % 4) and + 1 of row 16 m + 8 k + lane / 4.
+__device__ __forceinline__ void tmem_ld_16(uint32_t taddr, uint32_t* v) {
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    uint32_t* r = v + 8 * m;
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+                   "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr + ((uint32_t)(16 * m) << 16))
+                 : "memory");
+  }
 }
 
-// Bias + SiLU of one 32-column slice (columns cb .. cb + 31 of this thread's
-// row) into the BF16 activations: h = acc + b/2 (the accumulator holds
+// Bias + SiLU of a tmem_ld_16 of a hidden layer's accumulators into the BF16
+// activations: h = acc + b/2 (the accumulator holds
 // z/2 - b/2), silu = h + h tanh(h) in FP32, one rounding to BF16 per
 // activation (the rounding point of the training forward pass).  The packed
 // BF16 tanh would save no SFU time (it costs two SFU operations per pair) and
 // runs about one BF16 unit low below |h| = 8, which the cancellation in
-// h (1 + tanh h) turns into a bias on SiLU's negative branch.  bp is this
-// lane's bias_pair of the slice; pair k is broadcast from lane k.
-// kFull: all 32 columns exist (no bound checks, fully interleavable).
-template <bool kFull>
-__device__ __forceinline__ void silu_slice(const uint32_t* v, float2 bp, int cb, int hidden,
-                                           unsigned char* act, int r) {
+// h (1 + tanh h) turns into a bias on SiLU's negative branch.
+// A thread has pairs of columns of four rows, so that a bias serves four values
+// and add and multiply are packed.  b, to: of this thread's first pair.
+__device__ __forceinline__ void silu_slice(const uint32_t* v, const float* __restrict__ b,
+                                           int hidden, unsigned char* to) {
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    if (!kFull && cb + q * 8 >= hidden) break;
-    uint32_t o[4];
+  for (int q = 0; q < 2; ++q) {
+    const float2 bq = __ldg(reinterpret_cast<const float2*>(b + 8 * q));
+    const float2 bp = make_float2(0.5f * bq.x, 0.5f * bq.y);  // (halving is exact)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int i = q * 8 + 2 * j;
-      const float h0 = __uint_as_float(v[i]) + __shfl_sync(0xffffffffu, bp.x, q * 4 + j);
-      const float h1 = __uint_as_float(v[i + 1]) + __shfl_sync(0xffffffffu, bp.y, q * 4 + j);
-      o[j] = pptc::bf16x2_from(pptc::silu_half(h0), pptc::silu_half(h1));
+    for (int k = 0; k < 4; ++k) {
+      const int i = (k >> 1) * 8 + 4 * q + 2 * (k & 1);
+      const float2 h =
+          ppdev::add2(make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), bp);
+      const float2 o =
+          ppdev::fma2(h, make_float2(pptc::tanh_approx(h.x), pptc::tanh_approx(h.y)), h);
+      *reinterpret_cast<uint32_t*>(to + q * 128 + k * (hidden * 16)) =
+          pptc::bf16x2_from(o.x, o.y);
     }
-    *reinterpret_cast<uint4*>(act + pptc::core_offset(r, (cb >> 3) + q, hidden)) =
-        make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 
 __device__ __forceinline__ void epi_sync() {
   asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-}
-
-// Barrier over the epilogue warps that also ANDs a flag across them, so that
-// all of them take the same branch after a bounded wait.
-__device__ __forceinline__ bool epi_all(bool v) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %1, 0;\n\t"
-      "bar.red.and.pred q, 1, %2, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(r)
-      : "r"((uint32_t)v), "n"(kEpiThreads)
-      : "memory");
-  return r != 0;
 }
 
 // Persistent, warp-specialised network evaluation, 256 rows (two tiles of
@@ -734,6 +734,12 @@ __device__ __forceinline__ bool epi_all(bool v) {
 //               (in place: the MMAs that read them have completed), or the
 //               head (expected count exp(min(o, 30)) and softmax PDF), then
 //               the slot's next input tile.
+// The next layer's MMAs follow the epilogue chunk by chunk.  Bound: the MMA
+// warp's own instructions (about 700 cycles per chunk between 16 busy warps
+// where the tensor core needs 512), then tanh (2048 cycles per tile and layer).
+// 1e6 rows of the 4 x 256 network with 64 bins: 684 us when MMAs waited for the
+// whole layer, every job began with a barrier and biases came by shuffle; 589
+// us with chunks; 574 us with the chunk-by-chunk issue loop.
 // Warp w reads TMEM lanes 32 (w % 4) .. + 31.  Every wait is bounded; a
 // timeout sets the error flag and the roles wind down (copies and MMAs in
 // flight are waited for, again bounded, before TMEM is released).
@@ -741,7 +747,8 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     infer_kernel(const __grid_constant__ InferParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t w_full[kRingSlots], w_empty[kRingSlots];
-  __shared__ __align__(8) uint64_t acc_full[2], act_ready[2], mma_done;
+  // ready[T][k]: chunk k of slot T's activations
+  __shared__ __align__(8) uint64_t acc_full[2], ready[2][kMaxChunks], mma_done;
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int abort_flag;
   unsigned char* ring = smem + p.ring_off;
@@ -754,7 +761,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     }
     for (int i = 0; i < 2; ++i) {
       pptc::mbar_init(&acc_full[i], 1);
-      pptc::mbar_init(&act_ready[i], kEpiThreads);
+      for (int k = 0; k < kMaxChunks; ++k) pptc::mbar_init(&ready[i][k], kEpiWarps);
     }
     pptc::mbar_init(&mma_done, 1);
     abort_flag = 0;
@@ -809,66 +816,75 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer
-    if (lane == 0) {
-      // The issue loop is kept short: the tensor core runs a 128x256x16 MMA
-      // in ~128 cycles, and this one thread's bookkeeping between MMAs (waits,
-      // descriptors, loop control) must fit in that time or the pipe idles.
-      JobIter it;
-      bool more = it.next(p);
-      uint32_t slot = 0, phase = 0;     // ring slot of the next chunk, its fill parity
-      uint32_t jobs[2] = {0u, 0u};      // jobs issued per slot
-      // descriptor of ring slot 0 holding a full-width chunk; descriptors
-      // advance by adding the byte offset / 16 to the start address field
-      // (shared addresses < 256 KB: the field never carries)
-      const uint64_t b_full = pptc::smem_desc(pptc::smem_u32(ring), 128, (uint32_t)(kChunkK / 8) * 128u);
-      const uint32_t idesc_hidden = pptc::idesc_bf16(128, p.hidden);
-      const uint32_t idesc_head = pptc::idesc_bf16(128, p.out_pad);
-      while (more && ok) {
-        const int T = it.slot, l = it.layer;
-        const int K = l == 0 ? p.in_pad : p.hidden;
-        if (abort_flag || !pptc::mbar_wait(&act_ready[T], jobs[T] & 1, p.wait_ns)) {
-          ok = false;
-          break;
-        }
-        pptc::fence_after_sync();
-        const uint32_t d = tmem + (uint32_t)T * p.slot_cols;
-        const uint64_t a_desc = pptc::smem_desc(pptc::smem_u32(smem + (size_t)T * p.act_bytes), 128,
-                                                (uint32_t)(K / 8) * 128u);
-        const uint32_t idesc = l == p.n_layers ? idesc_head : idesc_hidden;
-        for (int j = 0; j * kChunkK < K; ++j) {
-          if (!pptc::mbar_wait(&w_full[slot], phase, p.wait_ns) || abort_flag) {
-            ok = false;
-            break;
-          }
-          pptc::fence_after_sync();
-          const uint64_t a_j = a_desc + (uint64_t)(j * (kChunkK / 16) * 16);  // + j * 64 cols * 2 B / 16
-          const int w = chunk_width(K, j);
-          if (w == kChunkK) {
-            const uint64_t b = b_full + (uint64_t)(slot * (kSlotBytes / 16));
-#pragma unroll
-            for (int s = 0; s < kChunkK / 16; ++s)
-              pptc::mma_f16(d, a_j + (uint64_t)(s * 16), b + (uint64_t)(s * 16), idesc,
-                            j > 0 || s > 0);
-          } else {
-            const uint64_t b = pptc::smem_desc(pptc::smem_u32(ring + slot * kSlotBytes), 128,
-                                               (uint32_t)(w / 8) * 128u);
-            for (int s = 0; s < w / 16; ++s)
-              pptc::mma_f16(d, a_j + (uint64_t)(s * 16), b + (uint64_t)(s * 16), idesc,
-                            j > 0 || s > 0);
-          }
-          // the slot is free once these MMAs complete
-          pptc::mma_commit(&w_empty[slot]);
-          if (++slot == kRingSlots) {
-            slot = 0;
-            phase ^= 1u;
-          }
-        }
+    // The tensor core runs a chunk's four 128x256x16 MMAs in 512 cycles, and all of
+    // this warp's work for the next chunk must fit in that time or the pipe
+    // idles.  So the jobs are walked through chunk by chunk: the next chunk's
+    // operands are worked out, and its two barriers tested together, while the
+    // MMAs of this one run; the warp stays converged, as descriptors in uniform
+    // registers need no move each.
+    JobIter it;
+    bool more = it.next(p);
+    uint32_t slot = 0, phase = 0;  // ring slot of the chunk, its fill parity
+    uint32_t turns = 0;            // parities of ready[T][j], bit T * kMaxChunks + j
+    // descriptor of ring slot 0 holding a full-width chunk; descriptors
+    // advance by adding the byte offset / 16 to the start address field
+    // (shared addresses < 256 KB: the field never carries)
+    const uint64_t b_full = pptc::smem_desc(pptc::smem_u32(ring), 128, (uint32_t)(kChunkK / 8) * 128u);
+    const uint32_t idesc_hidden = pptc::idesc_bf16(128, p.hidden);
+    const uint32_t idesc_head = pptc::idesc_bf16(128, p.out_pad);
+    const uint64_t a_in = pptc::smem_desc(pptc::smem_u32(smem), 128, (uint32_t)(p.in_pad / 8) * 128u);
+    const uint64_t a_hid = pptc::smem_desc(pptc::smem_u32(smem), 128, (uint32_t)(p.hidden / 8) * 128u);
+    const bool leader = lane == 0;
+    int j = 0;  // the chunk of the job
+    while (more) {
+      const int T = it.slot, l = it.layer;
+      const int K = l == 0 ? p.in_pad : p.hidden;
+      const uint32_t d = tmem + (uint32_t)T * p.slot_cols;
+      const uint64_t a =
+          (l == 0 ? a_in : a_hid) + (uint64_t)(((uint32_t)T * p.act_bytes >> 4) + j * kChunkK);
+      const uint64_t b = b_full + (uint64_t)(slot * (kSlotBytes / 16));
+      const uint32_t idesc = l == p.n_layers ? idesc_head : idesc_hidden;
+      const int w = chunk_width(K, j);
+      uint64_t* const act = &ready[T][j];
+      const uint32_t bit = (uint32_t)(T * kMaxChunks + j), turn = (turns >> bit) & 1;
+      const bool t0 = pptc::mbar_test(pptc::smem_u32(&w_full[slot]), phase);
+      const bool t1 = pptc::mbar_test(pptc::smem_u32(act), turn);
+      if (!__all_sync(0xffffffffu, t0 && t1)) {
+        ok = __all_sync(0xffffffffu, !abort_flag &&
+                                         pptc::mbar_wait(&w_full[slot], phase, p.wait_ns) &&
+                                         pptc::mbar_wait(act, turn, p.wait_ns));
         if (!ok) break;
-        pptc::mma_commit(&acc_full[T]);
-        jobs[T]++;
+      }
+      pptc::fence_after_sync();
+      if (w == kChunkK) {
+#pragma unroll
+        for (int s = 0; s < kChunkK / 16; ++s)
+          pptc::mma_f16_by(leader, d, a + (uint64_t)(s * 16), b + (uint64_t)(s * 16), idesc,
+                           j > 0 || s > 0);
+      } else {
+        const uint64_t bn = pptc::smem_desc(pptc::smem_u32(ring + slot * kSlotBytes), 128,
+                                            (uint32_t)(w / 8) * 128u);
+        for (int s = 0; s < w / 16; ++s)
+          pptc::mma_f16_by(leader, d, a + (uint64_t)(s * 16), bn + (uint64_t)(s * 16), idesc,
+                           j > 0 || s > 0);
+      }
+      // the slot is free, and the job done, once these MMAs complete
+      const bool last = (j + 1) * kChunkK >= K;
+      pptc::mma_commit_by(leader && last, &acc_full[T]);
+      pptc::mma_commit_by(leader, &w_empty[slot]);
+      turns ^= 1u << bit;
+      if (++slot == kRingSlots) {
+        slot = 0;
+        phase ^= 1u;
+      }
+      ++j;
+      if (last) {
+        j = 0;
         more = it.next(p);
       }
-      // everything issued has completed before TMEM and shared memory go away
+    }
+    // everything issued has completed before TMEM and shared memory go away
+    if (lane == 0) {
       pptc::mma_commit(&mma_done);
       if (!pptc::mbar_wait(&mma_done, 0, p.wait_ns)) ok = false;
       if (!ok) abort_flag = 1;
@@ -881,16 +897,23 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     const int quad = warp & 3;  // TMEM lane quarter this warp may access
     const int cgrp = ew >> 2;   // column group 0..3
     const int r = quad * 32 + lane;
-    // the head's biases for the one-pass head (visible to every epilogue
-    // thread after the first epi_all barrier, long before the first head)
+    // the head's biases for the one-pass head
     float* head_bias = reinterpret_cast<float*>(smem + p.head_bias_off);
     if (p.head_bias_off)
       for (int c = t; c < p.out_pad; c += kEpiThreads) head_bias[c] = p.P[p.off_b[p.n_layers] + c];
+    epi_sync();
+    // chunks k0 .. of K columns of slot T's activations are written
+    auto arrive = [&](int T, int k0, int K) {
+      pptc::fence_async_smem();
+      pptc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0)
+        for (int k = k0; k * kChunkK < K; ++k) pptc::mbar_arrive(&ready[T][k]);
+    };
     // first tiles of both slots
     for (int T = 0; T < 2; ++T) {
       pack_input(p, smem + (size_t)T * p.act_bytes, (int)blockIdx.x * 2 + T, t);
-      pptc::fence_async_smem();
-      pptc::mbar_arrive(&act_ready[T]);
+      arrive(T, 0, p.in_pad);
     }
     JobIter it;
     bool more = it.next(p);
@@ -898,44 +921,48 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     while (more) {
       const int T = it.slot, l = it.layer;
       unsigned char* act = smem + (size_t)T * p.act_bytes;
-      // this lane's bias values of the job's two column slices, loaded
-      // before the wait (the inner loops broadcast them by shuffle): b for
-      // the head, pairs of b/2 for a hidden layer
+      // the head's biases of this lane's columns (broadcast by shuffle)
       const bool head = l == p.n_layers;
       const float* __restrict__ bias = p.P + p.off_b[l];
       const int s0 = cgrp * 32, s1 = (cgrp + 4) * 32;
       const float bl0 = head && s0 + lane < p.out_pad ? __ldg(bias + s0 + lane) : 0.0f;
       const float bl1 = head && s1 + lane < p.out_pad ? __ldg(bias + s1 + lane) : 0.0f;
-      const float2 bp0 = head ? make_float2(0.0f, 0.0f) : bias_pair(bias, s0, p.hidden, lane);
-      const float2 bp1 =
-          head ? make_float2(0.0f, 0.0f) : bias_pair(bias, s0 + 128, p.hidden, lane);
-      if (!epi_all(pptc::mbar_wait(&acc_full[T], jobs[T] & 1, p.wait_ns))) {
-        ok = false;
-        break;
-      }
-      jobs[T]++;
+      // No barrier here, so that warps that are done go on to the next job.  After
+      // a wait that ran out they go on as well, on whatever is there, as the
+      // barriers of the head count all of them.
+      const uint32_t turn = (T ? jobs[1]++ : jobs[0]++) & 1;
+      if (!pptc::mbar_try(pptc::smem_u32(&acc_full[T]), turn) && !abort_flag &&
+          !pptc::mbar_wait(&acc_full[T], turn, p.wait_ns))
+        abort_flag = 1;
+      __syncwarp();
       pptc::fence_after_sync();
       const uint32_t trow = tmem + (uint32_t)T * p.slot_cols + ((uint32_t)(quad * 32) << 16);
       if (l < p.n_layers) {
-        // two 32-column slices per load-wait (columns c0 and c0 + 128)
-        for (int c0 = cgrp * 32; c0 < p.hidden; c0 += 256) {
-          uint32_t v[2][32];
-          const bool two = c0 + 128 < p.hidden;
-          pptc::tmem_ld32_nowait(trow + (uint32_t)c0, v[0]);
-          if (two) pptc::tmem_ld32_nowait(trow + (uint32_t)(c0 + 128), v[1]);
-          pptc::tmem_wait();
-          // (hidden <= 256: one pass with the preloaded pairs; wider layers
-          // load theirs here)
-          const float2 b0 = c0 == s0 ? bp0 : bias_pair(bias, c0, p.hidden, lane);
-          const float2 b1 = c0 == s0 ? bp1 : bias_pair(bias, c0 + 128, p.hidden, lane);
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            if (h == 1 && !two) break;
-            const int cb = c0 + h * 128;
-            const float2 bp = h ? b1 : b0;
-            if (cb + 32 <= p.hidden) silu_slice<true>(v[h], bp, cb, p.hidden, act, r);
-            else silu_slice<false>(v[h], bp, cb, p.hidden, act, r);
-          }
+        // 16 columns of every chunk, two chunks in registers at a time.  All
+        // accumulators are read before the first two chunks are announced, as the
+        // MMAs of the next layer, which follow chunk by chunk, overwrite them.
+        uint32_t v[2][16];
+        const uint32_t col = trow + (uint32_t)(cgrp * 16);
+        const int mine = p.hidden - cgrp * 16;  // chunk k has columns of this warp if below
+        unsigned char* to = act + pptc::core_offset(quad * 32 + (lane >> 2), cgrp * 2, p.hidden) +
+                            4 * (lane & 3);
+        const float* bl = bias + cgrp * 16 + 2 * (lane & 3);
+        if (0 < mine) tmem_ld_16(col, v[0]);
+        if (kChunkK < mine) tmem_ld_16(col + kChunkK, v[1]);
+        pptc::tmem_wait();
+        if (0 < mine) silu_slice(v[0], bl, p.hidden, to);
+        if (2 * kChunkK < mine) tmem_ld_16(col + 2 * kChunkK, v[0]);
+        if (kChunkK < mine) silu_slice(v[1], bl + kChunkK, p.hidden, to + 1024);
+        if (3 * kChunkK < mine) tmem_ld_16(col + 3 * kChunkK, v[1]);
+        pptc::tmem_wait();
+        arrive(T, 0, min(p.hidden, 2 * kChunkK));
+        if (2 * kChunkK < p.hidden) {
+          if (2 * kChunkK < mine) silu_slice(v[0], bl + 2 * kChunkK, p.hidden, to + 2048);
+          arrive(T, 2, min(p.hidden, 3 * kChunkK));
+        }
+        if (3 * kChunkK < p.hidden) {
+          if (3 * kChunkK < mine) silu_slice(v[1], bl + 3 * kChunkK, p.hidden, to + 3072);
+          arrive(T, 3, p.hidden);
         }
       } else {
         // head: every epilogue warp takes the 32-column slices cgrp and
@@ -958,6 +985,11 @@ __global__ void __launch_bounds__(kInferThreads, 1)
         float xin[8];
         const bool more_rounds = it.round + 1 < p.n_rounds;
         if (prefetch && t < units && more_rounds) load_unit(p, next, t, xin);
+        if (!prefetch && more_rounds) {  // no registers for it: into L2 at least
+          const long long at = (long long)next * 128 * p.n_in + 32 * t;
+          if (t < 4 * p.n_in && at < p.n * p.n_in)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.x + at));
+        }
         if (one_pass) {
           // one pass: this warp's 32-column slice (if any) is read once; each
           // 16-column half's exponentials go to the staging rows relative to
@@ -1121,10 +1153,8 @@ __global__ void __launch_bounds__(kInferThreads, 1)
             pack_input(p, act, next, t);
           }
         }
+        arrive(T, 0, p.in_pad);
       }
-      pptc::fence_async_smem();  // activation writes -> the next MMAs of this slot
-      pptc::fence_before_sync();
-      pptc::mbar_arrive(&act_ready[T]);
       more = it.next(p);
     }
     if (!ok) abort_flag = 1;
