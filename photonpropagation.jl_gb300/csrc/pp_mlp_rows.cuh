@@ -280,57 +280,66 @@ __global__ void __launch_bounds__(kRowsThreads, 1)
   } else if (warp == kEpiThreads / 32) {
     // ---------------- MMA issuer
     // The four MMAs of a chunk (64 x 256 x 16: 128 cycles each) run while this warp
-    // gets the next chunk under way, if that takes less than their 512 cycles: its
-    // barriers are tested before the MMAs of the chunk before it are issued, and
-    // the warp stays converged so that descriptors live in uniform registers.
-    uint32_t parity[kParts];
-#pragma unroll
-    for (int k = 0; k < kParts; ++k) parity[k] = 0;
+    // works out the next chunk and tests its two barriers, if that takes less than
+    // their 512 cycles; the warp stays converged, as descriptors in uniform
+    // registers need no move each.
+    const bool leader = lane == 0;
+    uint32_t turns = 0;  // parity of chunk k's barriers, bit k
+    const uint32_t act0 = pptc::smem_u32(smem);
     const uint64_t b0 = pptc::smem_desc(pptc::smem_u32(ring), 128, (kChunk / 8) * 128u);
-    bool there = false;  // the next chunk's barrier has been seen complete
-    for (int n = 0; n < n_jobs && ok; ++n) {
-      const Job j = job_of<kHidden>(p, n);
-      const uint32_t act = pptc::smem_u32(smem + (size_t)(n & 1) * p.act_bytes);
-      const uint64_t a0 = pptc::smem_desc(act, 128, (uint32_t)(j.K / 8) * 128u);
+    int n = 0, k = 0;
+    Job j = job_of<kHidden>(p, 0);
+    while (true) {
+      const uint32_t act = act0 + (uint32_t)(n & 1) * p.act_bytes;
+      const uint64_t a = pptc::smem_desc(act, 128, (uint32_t)(j.K / 8) * 128u) +
+                         (uint64_t)(k * (kChunk / 16) * 16);
+      const uint64_t b = b0 + (uint64_t)(k * (kSlotBytes / 16));
       const uint32_t idesc =
           pptc::idesc_bf16(kRows, j.N) | (n > L ? 1u << 16 : 0u);  // B transposed backward
       const uint32_t d = tmem + (uint32_t)(n & 1) * kAccCols;
-#pragma unroll
-      for (int k = 0; k < kParts; ++k) {
-        if (k * kChunk >= j.K) break;
-        ok = __all_sync(0xffffffffu, there || (pptc::mbar_wait(&w_full[k], parity[k], p.wait_ns) &&
-                                               pptc::mbar_wait(&go[k], parity[k], p.wait_ns)));
+      const int kw = min(kChunk, j.K - k * kChunk);
+      const bool last = (k + 1) * kChunk >= j.K;
+      const uint32_t turn = (turns >> k) & 1;
+      const bool t0 = pptc::mbar_test(pptc::smem_u32(&w_full[k]), turn);
+      const bool t1 = pptc::mbar_test(pptc::smem_u32(&go[k]), turn);
+      if (!__all_sync(0xffffffffu, t0 && t1)) {
+        ok = __all_sync(0xffffffffu, !abort_flag &&
+                                         pptc::mbar_wait(&w_full[k], turn, p.wait_ns) &&
+                                         pptc::mbar_wait(&go[k], turn, p.wait_ns));
         if (!ok) break;
-        parity[k] ^= 1u;
-        pptc::fence_after_sync();
-        const int kw = min(kChunk, j.K - k * kChunk);
-        const bool last = (k + 1) * kChunk >= j.K;
-        const int next = (k + 1) % kParts;
-        there = !last && pptc::mbar_test(pptc::smem_u32(&w_full[next]), parity[next]) &&
-                pptc::mbar_test(pptc::smem_u32(&go[next]), parity[next]);
-        const uint64_t a = a0 + (uint64_t)(k * (kChunk / 16) * 16);
-        if (lane == 0) {
-          if (last) bulk_stores_read();
-          if (kw == kChunk) {
-            const uint64_t b = b0 + (uint64_t)(k * (kSlotBytes / 16));
-            pptc::mma_f16(d, a, b, idesc, k > 0);
-            pptc::mma_f16(d, a + 16, b + 16, idesc, true);
-            pptc::mma_f16(d, a + 32, b + 32, idesc, true);
-            pptc::mma_f16(d, a + 48, b + 48, idesc, true);
-          } else {
-            const uint64_t b = pptc::smem_desc(pptc::smem_u32(ring + k * kSlotBytes), 128,
-                                               (uint32_t)(kw / 8) * 128u);
-            for (int s = 0; s < kw / 16; ++s)
-              pptc::mma_f16(d, a + (uint64_t)(s * 16), b + (uint64_t)(s * 16), idesc,
-                            k > 0 || s > 0);
-          }
-          // The epilogue of this job overwrites the previous job's operand, which
-          // has been read; this job's own goes to memory meanwhile.
-          if (last) pptc::mma_commit(&acc_full);
+      }
+      pptc::fence_after_sync();
+      if (kw == kChunk) {
+#pragma unroll
+        for (int s = 0; s < kChunk / 16; ++s)
+          pptc::mma_f16_by(leader, d, a + (uint64_t)(s * 16), b + (uint64_t)(s * 16), idesc,
+                           k > 0 || s > 0);
+      } else {
+        const uint64_t bn = pptc::smem_desc(pptc::smem_u32(ring + k * kSlotBytes), 128,
+                                            (uint32_t)(kw / 8) * 128u);
+        for (int s = 0; s < kw / 16; ++s)
+          pptc::mma_f16_by(leader, d, a + (uint64_t)(s * 16), bn + (uint64_t)(s * 16), idesc,
+                           k > 0 || s > 0);
+      }
+      if (last) {
+        // The epilogue of this job overwrites the previous job's operand, which
+        // has been read; this job's own goes to memory meanwhile.
+        if (leader) {
+          bulk_stores_read();
+          pptc::mma_commit(&acc_full);
           pptc::mma_commit(&w_empty[k]);
-          if (last) bulk_store(operand_home(p, n, j.K), act, (uint32_t)(kRows * j.K * 2));
+          bulk_store(operand_home(p, n, j.K), act, (uint32_t)(kRows * j.K * 2));
         }
         __syncwarp();
+      } else {
+        pptc::mma_commit_by(leader, &w_empty[k]);
+      }
+      turns ^= 1u << k;
+      ++k;
+      if (last) {
+        if (++n == n_jobs) break;
+        k = 0;
+        j = job_of<kHidden>(p, n);
       }
     }
     if (ok) ok = __all_sync(0xffffffffu, pptc::mbar_wait(&epi_done, 0, p.wait_ns));
@@ -654,8 +663,8 @@ __global__ void __launch_bounds__(kDwThreads, 1) dw_kernel(const __grid_constant
   const uint32_t tmem = tmem_slot;
   bool ok = true;
   if (warp > 8) {
-    // eight 8-row groups of each operand; a stage is announced when the third one
-    // after it has been requested
+    // eight 8-row groups of each operand; a stage is announced when the one after
+    // it has been requested
     const int t = (int)threadIdx.x - 256 - 32;
     auto announce = [&](int k) {
       __syncwarp();
@@ -676,14 +685,14 @@ __global__ void __launch_bounds__(kDwThreads, 1) dw_kernel(const __grid_constant
         if (t < w.cols) fetch16(dst + kTileBytes + i * w.cols * 16, b + (size_t)i * 16 * w.b_cols);
       }
       fetch_commit();
-      if (c >= 3) {
-        fetch_wait<3>();
-        announce(k - 3);
+      if (c >= 1) {
+        fetch_wait<1>();
+        announce(k - 1);
       }
     }
     fetch_wait<0>();
     if (ok)
-      for (int q = max(k0, k - 3); q < k; ++q) announce(q);
+      for (int q = max(k0, k - 1); q < k; ++q) announce(q);
   } else if (warp == 8) {
     // (the result tile's rows past w.rows take whatever follows in the stage)
     const uint32_t idesc = pptc::idesc_bf16(128, w.cols) | (1u << 15) | (1u << 16);
@@ -702,16 +711,13 @@ __global__ void __launch_bounds__(kDwThreads, 1) dw_kernel(const __grid_constant
         phase ^= 1u;
       }
       there = k + 1 < k1 && pptc::mbar_test(pptc::smem_u32(&full[slot]), phase);
-      if (lane == 0) {
-        const uint64_t a = a0 + (uint64_t)(at * (kDwStageBytes / 16));
-        const uint64_t b = b0 + (uint64_t)(at * (kDwStageBytes / 16));
+      const uint64_t a = a0 + (uint64_t)(at * (kDwStageBytes / 16));
+      const uint64_t b = b0 + (uint64_t)(at * (kDwStageBytes / 16));
 #pragma unroll
-        for (int s = 0; s < 4; ++s)
-          pptc::mma_f16(tmem, a + (uint64_t)(s * 2 * w.rows), b + (uint64_t)(s * 2 * w.cols), idesc,
-                        k > k0 || s > 0);
-        pptc::mma_commit(&empty[at]);
-      }
-      __syncwarp();
+      for (int s = 0; s < 4; ++s)
+        pptc::mma_f16_by(lane == 0, tmem, a + (uint64_t)(s * 2 * w.rows),
+                         b + (uint64_t)(s * 2 * w.cols), idesc, k > k0 || s > 0);
+      pptc::mma_commit_by(lane == 0, &empty[at]);
     }
     if (lane == 0) {
       pptc::mma_commit(&done);
