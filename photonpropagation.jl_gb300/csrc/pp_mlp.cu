@@ -739,7 +739,9 @@ __device__ __forceinline__ void epi_sync() {
 // where the tensor core needs 512), then tanh (2048 cycles per tile and layer).
 // 1e6 rows of the 4 x 256 network with 64 bins: 684 us when MMAs waited for the
 // whole layer, every job began with a barrier and biases came by shuffle; 589
-// us with chunks; 574 us with the chunk-by-chunk issue loop.
+// us with chunks; 574 us with the next chunk worked out during this one's MMAs;
+// 560 us with both barriers in one test, rows copied out eight at a
+// time and the next input loaded under that.
 // Warp w reads TMEM lanes 32 (w % 4) .. + 31.  Every wait is bounded; a
 // timeout sets the error flag and the roles wind down (copies and MMAs in
 // flight are waited for, again bounded, before TMEM is released).
@@ -818,10 +820,11 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     // ---------------- MMA issuer
     // The tensor core runs a chunk's four 128x256x16 MMAs in 512 cycles, and all of
     // this warp's work for the next chunk must fit in that time or the pipe
-    // idles.  So the jobs are walked through chunk by chunk: the next chunk's
-    // operands are worked out, and its two barriers tested together, while the
-    // MMAs of this one run; the warp stays converged, as descriptors in uniform
-    // registers need no move each.
+    // idles.  The next chunk's operands are worked out, and its two barriers
+    // tested together, while the MMAs of this one run; the warp stays converged,
+    // as descriptors in uniform registers need no move each.  (Alone on the SM,
+    // tests, vote, fence, an MMA and commits take 402 cycles a chunk; beside warps
+    // that always have an instruction ready the scheduler gives it a ninth.)
     JobIter it;
     bool more = it.next(p);
     uint32_t slot = 0, phase = 0;  // ring slot of the chunk, its fill parity
@@ -835,53 +838,55 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     const uint64_t a_in = pptc::smem_desc(pptc::smem_u32(smem), 128, (uint32_t)(p.in_pad / 8) * 128u);
     const uint64_t a_hid = pptc::smem_desc(pptc::smem_u32(smem), 128, (uint32_t)(p.hidden / 8) * 128u);
     const bool leader = lane == 0;
-    int j = 0;  // the chunk of the job
+    const int chunks_in = (p.in_pad + kChunkK - 1) / kChunkK;
+    const int chunks_hid = (p.hidden + kChunkK - 1) / kChunkK;
+    const int tail_in = chunk_width(p.in_pad, chunks_in - 1);
+    const int tail_hid = chunk_width(p.hidden, chunks_hid - 1);
+    const uint32_t full0 = pptc::smem_u32(&w_full[0]), ready0 = pptc::smem_u32(&ready[0][0]);
     while (more) {
       const int T = it.slot, l = it.layer;
-      const int K = l == 0 ? p.in_pad : p.hidden;
+      const int last = (l == 0 ? chunks_in : chunks_hid) - 1;
+      const int tail = l == 0 ? tail_in : tail_hid;  // width of the last chunk
       const uint32_t d = tmem + (uint32_t)T * p.slot_cols;
-      const uint64_t a =
-          (l == 0 ? a_in : a_hid) + (uint64_t)(((uint32_t)T * p.act_bytes >> 4) + j * kChunkK);
-      const uint64_t b = b_full + (uint64_t)(slot * (kSlotBytes / 16));
       const uint32_t idesc = l == p.n_layers ? idesc_head : idesc_hidden;
-      const int w = chunk_width(K, j);
-      uint64_t* const act = &ready[T][j];
-      const uint32_t bit = (uint32_t)(T * kMaxChunks + j), turn = (turns >> bit) & 1;
-      const bool t0 = pptc::mbar_test(pptc::smem_u32(&w_full[slot]), phase);
-      const bool t1 = pptc::mbar_test(pptc::smem_u32(act), turn);
-      if (!__all_sync(0xffffffffu, t0 && t1)) {
-        ok = __all_sync(0xffffffffu, !abort_flag &&
-                                         pptc::mbar_wait(&w_full[slot], phase, p.wait_ns) &&
-                                         pptc::mbar_wait(act, turn, p.wait_ns));
-        if (!ok) break;
-      }
-      pptc::fence_after_sync();
-      if (w == kChunkK) {
+      const uint32_t act = ready0 + (uint32_t)(T * kMaxChunks * 8);
+      uint64_t a = (l == 0 ? a_in : a_hid) + (uint64_t)((uint32_t)T * p.act_bytes >> 4);
+      uint32_t turn = turns >> (T * kMaxChunks);
+      turns ^= ((2u << last) - 1) << (T * kMaxChunks);
+      for (int j = 0; j <= last; ++j) {
+        const bool there = pptc::mbar_test2(full0 + slot * 8, phase, act + j * 8, turn & 1);
+        if (!__all_sync(0xffffffffu, there)) {
+          ok = __all_sync(0xffffffffu, !abort_flag &&
+                                           pptc::mbar_wait(&w_full[slot], phase, p.wait_ns) &&
+                                           pptc::mbar_wait(&ready[T][j], turn & 1, p.wait_ns));
+          if (!ok) break;
+        }
+        pptc::fence_after_sync();
+        if (j < last || tail == kChunkK) {
+          const uint64_t b = b_full + (uint64_t)(slot * (kSlotBytes / 16));
 #pragma unroll
-        for (int s = 0; s < kChunkK / 16; ++s)
-          pptc::mma_f16_by(leader, d, a + (uint64_t)(s * 16), b + (uint64_t)(s * 16), idesc,
-                           j > 0 || s > 0);
-      } else {
-        const uint64_t bn = pptc::smem_desc(pptc::smem_u32(ring + slot * kSlotBytes), 128,
-                                            (uint32_t)(w / 8) * 128u);
-        for (int s = 0; s < w / 16; ++s)
-          pptc::mma_f16_by(leader, d, a + (uint64_t)(s * 16), bn + (uint64_t)(s * 16), idesc,
-                           j > 0 || s > 0);
+          for (int s = 0; s < kChunkK / 16; ++s)
+            pptc::mma_f16_by(leader, d, a + (uint64_t)(s * 16), b + (uint64_t)(s * 16), idesc,
+                             j > 0 || s > 0);
+        } else {
+          const uint64_t b = pptc::smem_desc(pptc::smem_u32(ring + slot * kSlotBytes), 128,
+                                             (uint32_t)(tail / 8) * 128u);
+          for (int s = 0; s < tail / 16; ++s)
+            pptc::mma_f16_by(leader, d, a + (uint64_t)(s * 16), b + (uint64_t)(s * 16), idesc,
+                             j > 0 || s > 0);
+        }
+        // the job is done, and the slot free, once these MMAs complete
+        if (j == last) pptc::mma_commit_by(leader, &acc_full[T]);
+        pptc::mma_commit_by(leader, &w_empty[slot]);
+        a += kChunkK;
+        turn >>= 1;
+        if (++slot == kRingSlots) {
+          slot = 0;
+          phase ^= 1u;
+        }
       }
-      // the slot is free, and the job done, once these MMAs complete
-      const bool last = (j + 1) * kChunkK >= K;
-      pptc::mma_commit_by(leader && last, &acc_full[T]);
-      pptc::mma_commit_by(leader, &w_empty[slot]);
-      turns ^= 1u << bit;
-      if (++slot == kRingSlots) {
-        slot = 0;
-        phase ^= 1u;
-      }
-      ++j;
-      if (last) {
-        j = 0;
-        more = it.next(p);
-      }
+      if (!ok) break;
+      more = it.next(p);
     }
     // everything issued has completed before TMEM and shared memory go away
     if (lane == 0) {
@@ -981,11 +986,11 @@ __global__ void __launch_bounds__(kInferThreads, 1)
         const int units = 16 * p.in_pad;  // 128 rows x in_pad / 8 chunks of 8
         // one-pass head (PDF output requested and the layout allows it)
         const bool one_pass = p.head_bias_off != 0 && p.pdf != nullptr;
-        const bool prefetch = units <= kEpiThreads && !one_pass;
+        const bool prefetch = units <= kEpiThreads;
         float xin[8];
         const bool more_rounds = it.round + 1 < p.n_rounds;
-        if (prefetch && t < units && more_rounds) load_unit(p, next, t, xin);
-        if (!prefetch && more_rounds) {  // no registers for it: into L2 at least
+        if (prefetch && !one_pass && t < units && more_rounds) load_unit(p, next, t, xin);
+        if ((!prefetch || one_pass) && more_rounds) {  // no registers yet: into L2 at least
           const long long at = (long long)next * 128 * p.n_in + 32 * t;
           if (t < 4 * p.n_in && at < p.n * p.n_in)
             asm volatile("prefetch.global.L2 [%0];" ::"l"(p.x + at));
@@ -1068,9 +1073,16 @@ __global__ void __launch_bounds__(kInferThreads, 1)
           const long long left = p.n - row0;
           const int nrows = left < 128 ? (int)left : 128;
           float* dst = p.pdf + row0 * p.n_bins;
-          for (int rr = ew; rr < nrows; rr += kEpiWarps)
-            for (int c = lane; c < p.n_bins; c += 32)
-              dst[rr * p.n_bins + c] = stage[rr * ld + c] * h_scale[rr * 8 + ((c + 1) >> 4)];
+          if (prefetch && t < units && more_rounds) load_unit(p, next, t, xin);
+          for (int c = lane; c < p.n_bins; c += 32) {
+            const float* from = stage + c;
+            const float* scale = h_scale + ((c + 1) >> 4);
+#pragma unroll
+            for (int i = 0; i < 128 / kEpiWarps; ++i) {
+              const int rr = ew + i * kEpiWarps;
+              if (rr < nrows) dst[rr * p.n_bins + c] = from[rr * ld] * scale[rr * 8];
+            }
+          }
         } else {
         // pass 1: the log count and this warp's part of the row maximum
         float o0 = 0.0f, mx = -INFINITY;

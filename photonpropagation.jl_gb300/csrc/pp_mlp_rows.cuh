@@ -9,7 +9,7 @@
 // over the rows (dw_kernel), and a third is Adam.
 //
 // Layouts.  Every operand is written once in the core-matrix order in which the
-// tensor core reads it (pp_tc.cuh), so that each is fetched by whole bulk copies:
+// tensor core reads it (pp_tc.cuh), so that each is fetched as it stands:
 //   * weights, twice (pack_offset): wf, K-major over the layer's input, for the
 //     forward pass, and wb, the transposed product's operand, for the backward
 //     pass; each as blocks of all of N x 64 of K;
@@ -198,7 +198,9 @@ __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v 
 // dw_kernel needs, 16 warps do the epilogues; two accumulators and two activation buffers alternate, and each
 // 64-column chunk of a layer's input starts its MMAs when its epilogue is done, so
 // that all but a layer's last chunk run under the epilogue before them.  Bound: the
-// serial chain of 2 L + 1 products, epilogue and MMA latency.
+// serial chain of 2 L + 1 products, epilogue and MMA latency: 25 us for 4 x 256, at
+// batch 1024 (16 CTAs) as at 8192 (128).  With 128 rows per CTA, halves of a layer
+// and one thread's waits between the MMAs it took 40 us, on 64 SMs.
 template <int kHidden>
 __global__ void __launch_bounds__(kRowsThreads, 1)
     rows_kernel(const __grid_constant__ RowsParams p) {
@@ -286,60 +288,55 @@ __global__ void __launch_bounds__(kRowsThreads, 1)
     const bool leader = lane == 0;
     uint32_t turns = 0;  // parity of chunk k's barriers, bit k
     const uint32_t act0 = pptc::smem_u32(smem);
+    const uint32_t full0 = pptc::smem_u32(&w_full[0]), go0 = pptc::smem_u32(&go[0]);
     const uint64_t b0 = pptc::smem_desc(pptc::smem_u32(ring), 128, (kChunk / 8) * 128u);
-    int n = 0, k = 0;
-    Job j = job_of<kHidden>(p, 0);
-    while (true) {
+    for (int n = 0; n < n_jobs && ok; ++n) {
+      const Job j = job_of<kHidden>(p, n);
       const uint32_t act = act0 + (uint32_t)(n & 1) * p.act_bytes;
-      const uint64_t a = pptc::smem_desc(act, 128, (uint32_t)(j.K / 8) * 128u) +
-                         (uint64_t)(k * (kChunk / 16) * 16);
-      const uint64_t b = b0 + (uint64_t)(k * (kSlotBytes / 16));
       const uint32_t idesc =
           pptc::idesc_bf16(kRows, j.N) | (n > L ? 1u << 16 : 0u);  // B transposed backward
       const uint32_t d = tmem + (uint32_t)(n & 1) * kAccCols;
-      const int kw = min(kChunk, j.K - k * kChunk);
-      const bool last = (k + 1) * kChunk >= j.K;
-      const uint32_t turn = (turns >> k) & 1;
-      const bool t0 = pptc::mbar_test(pptc::smem_u32(&w_full[k]), turn);
-      const bool t1 = pptc::mbar_test(pptc::smem_u32(&go[k]), turn);
-      if (!__all_sync(0xffffffffu, t0 && t1)) {
-        ok = __all_sync(0xffffffffu, !abort_flag &&
-                                         pptc::mbar_wait(&w_full[k], turn, p.wait_ns) &&
-                                         pptc::mbar_wait(&go[k], turn, p.wait_ns));
-        if (!ok) break;
-      }
-      pptc::fence_after_sync();
-      if (kw == kChunk) {
-#pragma unroll
-        for (int s = 0; s < kChunk / 16; ++s)
-          pptc::mma_f16_by(leader, d, a + (uint64_t)(s * 16), b + (uint64_t)(s * 16), idesc,
-                           k > 0 || s > 0);
-      } else {
-        const uint64_t bn = pptc::smem_desc(pptc::smem_u32(ring + k * kSlotBytes), 128,
-                                            (uint32_t)(kw / 8) * 128u);
-        for (int s = 0; s < kw / 16; ++s)
-          pptc::mma_f16_by(leader, d, a + (uint64_t)(s * 16), bn + (uint64_t)(s * 16), idesc,
-                           k > 0 || s > 0);
-      }
-      if (last) {
-        // The epilogue of this job overwrites the previous job's operand, which
-        // has been read; this job's own goes to memory meanwhile.
-        if (leader) {
-          bulk_stores_read();
-          pptc::mma_commit(&acc_full);
-          pptc::mma_commit(&w_empty[k]);
-          bulk_store(operand_home(p, n, j.K), act, (uint32_t)(kRows * j.K * 2));
+      const int last = (j.K + kChunk - 1) / kChunk - 1, tail = j.K - last * kChunk;
+      uint64_t a = pptc::smem_desc(act, 128, (uint32_t)(j.K / 8) * 128u), b = b0;
+      uint32_t turn = turns;
+      turns ^= (2u << last) - 1;
+      for (int k = 0; k <= last; ++k) {
+        const bool there = pptc::mbar_test2(full0 + k * 8, turn & 1, go0 + k * 8, turn & 1);
+        if (!__all_sync(0xffffffffu, there)) {
+          ok = __all_sync(0xffffffffu, !abort_flag &&
+                                           pptc::mbar_wait(&w_full[k], turn & 1, p.wait_ns) &&
+                                           pptc::mbar_wait(&go[k], turn & 1, p.wait_ns));
+          if (!ok) break;
         }
-        __syncwarp();
-      } else {
-        pptc::mma_commit_by(leader, &w_empty[k]);
-      }
-      turns ^= 1u << k;
-      ++k;
-      if (last) {
-        if (++n == n_jobs) break;
-        k = 0;
-        j = job_of<kHidden>(p, n);
+        pptc::fence_after_sync();
+        if (k < last || tail == kChunk) {
+#pragma unroll
+          for (int s = 0; s < kChunk / 16; ++s)
+            pptc::mma_f16_by(leader, d, a + (uint64_t)(s * 16), b + (uint64_t)(s * 16), idesc,
+                             k > 0 || s > 0);
+        } else {
+          const uint64_t bn = pptc::smem_desc(pptc::smem_u32(ring + k * kSlotBytes), 128,
+                                              (uint32_t)(tail / 8) * 128u);
+          for (int s = 0; s < tail / 16; ++s)
+            pptc::mma_f16_by(leader, d, a + (uint64_t)(s * 16), bn + (uint64_t)(s * 16), idesc,
+                             k > 0 || s > 0);
+        }
+        if (k == last) {
+          // The epilogue of this job overwrites the previous job's operand, which
+          // has been read; this job's own goes to memory meanwhile.
+          if (leader) {
+            bulk_stores_read();
+            pptc::mma_commit(&acc_full);
+            pptc::mma_commit(&w_empty[k]);
+            bulk_store(operand_home(p, n, j.K), act, (uint32_t)(kRows * j.K * 2));
+          }
+          __syncwarp();
+        } else {
+          pptc::mma_commit_by(leader, &w_empty[k]);
+        }
+        a += kChunk;
+        b += kSlotBytes / 16;
+        turn >>= 1;
       }
     }
     if (ok) ok = __all_sync(0xffffffffu, pptc::mbar_wait(&epi_done, 0, p.wait_ns));
@@ -598,6 +595,9 @@ __global__ void __launch_bounds__(kRowsThreads, 1)
 }
 
 // ---- weight and bias gradients -----------------------------------------------------
+// 13 us at batch 8192 (69 MB of operands out of L2, 9.4 MB of atomics; 17 us with
+// bulk copies of an 8-row group each), 7 us at 1024.  Two CTAs per SM double the
+// atomics: 13.7 and 10 us.
 // Every 128 x 128 tile of every layer's dW = dZ^T X, its rows (K) split over
 // blocks_per_split 64-row tiles per CTA so that all CTAs run at once, summed by
 // float4 atomics; the first column tile's CTAs also sum dZ's columns (the bias

@@ -164,6 +164,22 @@ __device__ __forceinline__ bool mbar_test(uint32_t a, uint32_t parity) {
   return done != 0;
 }
 
+// Both of two phases, tested side by side: one after the other takes 136 cycles.
+__device__ __forceinline__ bool mbar_test2(uint32_t a, uint32_t parity_a, uint32_t b,
+                                           uint32_t parity_b) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+      "and.pred p, p, q;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(a), "r"(parity_a), "r"(b), "r"(parity_b)
+      : "memory");
+  return done != 0;
+}
+
 // Wait for phase `parity` of the mbarrier for at most limit_ns.  A phase that
 // has already completed costs one try_wait: the clock is read only when the
 // first try fails (a single-thread MMA issuer has about 128 cycles per
