@@ -450,7 +450,7 @@ def bench_surrogate(pp, torch, local, args):
     e1.record()
     torch.cuda.synchronize()
     step_ms = e0.elapsed_time(e1) / 20
-    # the same step as captured replays (batch drawn on the device included)
+    # the library's own loop (batch drawn on the device included)
     xp = [t.data_ptr() for t in (x, c, h)]
     mlp.train_steps(*xp, n3, 8192, 3, 0, 10**9, 1e-6, 1e-6, 5, stream=cur)
     e0.record()

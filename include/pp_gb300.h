@@ -404,9 +404,9 @@ PP_API int pp_mlp_train_step(pp_mlp* mlp, const float* d_x, const float* d_count
  * batch of Adam step t is Philox4x32-10(i, t, tag; key = seed) scaled to
  * n_rows), and takes a step of size lr1 + (lr0 - lr1) (1 + cos(pi s / (total - 1))) / 2,
  * s = t - step0 the step's index in a cosine schedule that began at Adam step
- * step0.  One step is captured once as a CUDA graph (for these arguments) and
- * replayed, so n_steps calls cost n_steps graph launches; batches and step
- * sizes depend only on the global step index, so K1 then K2 steps equal
+ * step0.  A step is three launches, or for shapes that train layer by layer
+ * (other widths than 128 and 256, more than 64 inputs or 127 bins) the launch
+ * of a graph captured once for these arguments; batches and step sizes depend only on the global step index, so K1 then K2 steps equal
  * K1 + K2 steps in one call.  Asynchronous on `stream`. */
 PP_API int pp_mlp_train_steps(pp_mlp* mlp, const float* d_x, const float* d_count,
                               const float* d_hist, int64_t n_rows, int32_t B, int32_t n_steps,

@@ -303,7 +303,7 @@ class MLP:
         """`n_steps` Adam steps inside the library (pp_mlp_train_steps): batches
         of `B` rows drawn on the device from the `n_rows` training rows, cosine
         step size from `lr0` to `lr1` over `total` steps begun at Adam step
-        `step0`, one captured step replayed per step."""
+        `step0`."""
         check(self._lib.pp_mlp_train_steps(self.ptr, c_void_p(x_dev), c_void_p(count_dev),
                                            c_void_p(hist_dev), int(n_rows), int(B), int(n_steps),
                                            int(step0), int(total), float(lr0), float(lr1),
@@ -355,8 +355,7 @@ def train(mlp: MLP, x, counts, hists, steps: int, batch: int = 8192, lr: float =
     `lr` and follows a cosine down to `lr_final` (default lr / 100) at the last
     step, so that the final parameters are not those of one noisy step at full
     rate.  Batches are drawn on the device (Philox, keyed on `seed` and the Adam
-    step), and the steps between two log points run as replays of one captured
-    step, without a return to Python."""
+    step), and the steps between two log points run without a return to Python."""
     lr_final = lr * 0.01 if lr_final is None else lr_final
     x, counts, hists = (t.contiguous().float() for t in (x, counts, hists))
     n = x.shape[0]
