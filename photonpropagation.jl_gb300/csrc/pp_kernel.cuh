@@ -475,51 +475,101 @@ __device__ __forceinline__ void advance(const PhaseDev& ph, Walk2& w, float2 ste
                                   make_uint2(r0.w, r1.w));
 }
 
-// Shaped targets: test one step segment against every target in index order and
-// keep the first hit as photon `own`'s; a list of detector lines is searched
-// line by line (src/photon_prop_cuda.jl:611-634): the 2-D test of the line, then
-// its modules; the first crossed line ends the search.
+// Shaped targets: test the step segments of a lane's two photons (those that are
+// open) against every target in index order and keep a photon's first hit, which
+// closes it; a list of detector lines is searched line by line
+// (src/photon_prop_cuda.jl:611-634): the 2-D test of the line, then its modules;
+// the first crossed line ends the search.  Both photons take one pass over the
+// list.  Packed operations first decide for both whether the exact test can
+// succeed: a circle's discriminant not below zero by more than the rounding of
+// either form (at most 1.5e-6 of the squared distance q), or a horizontal shape's
+// box, a little enlarged, crossed inside the segment.  1e7 photons, 400 spheres: 68
+// ms with one photon per lane, 97 with the exact test for one photon after the
+// other, 59 now; 5e6 photons, 20 lines of 20: 2.4, 3.0 and 1.9 ms.
 template <bool kPrecise>
-__device__ __forceinline__ bool search_shapes(const LaunchArgs& a, float3 pos, float3 dir,
-                                              float step, float dist0, uint32_t k, uint32_t* key,
-                                              WarpBest& best, int own) {
-  int hit = -1;  // 0-based module index to report
-  float d = 0.0f;
+__device__ __forceinline__ void search_shapes(const LaunchArgs& a, const Vec2& p, const Vec2& v,
+                                              float2 steps, float2 dist0, uint32_t k,
+                                              uint32_t* key, WarpBest& best, int lane,
+                                              bool (&open)[2]) {
+  const float3 pos[2] = {first(p), second(p)}, dir[2] = {first(v), second(v)};
+  const float step[2] = {steps.x, steps.y};
+  bool search[2] = {open[0], open[1]};
+  int hit[2] = {-1, -1};  // 0-based module index to report
+  float d[2] = {0.0f, 0.0f};
   int line_no = 0;
-  for (int j = 0; j < a.n_shapes; ++j) {
-    const float4 h = __ldg(a.shapes + 2 * j + 1);
-    if (__float_as_int(h.y) == PP_TARGET_LINE) {
-      const int nm = __float_as_int(h.x);
-      ++line_no;
-      float dl;
-      if (!sphere_hit<kPrecise>(__ldg(a.shapes + 2 * j), make_float3(pos.x, pos.y, 0.0f),
-                                make_float3(dir.x, dir.y, 0.0f), step, &dl)) {
-        j += nm;
-        continue;
+  // (the distance above a shape, times `along`, is the way to its height; the
+  // crossing point is off by less than `slack`)
+  const float2 along = make_float2(-1.0f / copysignf(fmaxf(fabsf(v.z.x), 1e-30f), v.z.x),
+                                   -1.0f / copysignf(fmaxf(fabsf(v.z.y), 1e-30f), v.z.y));
+  const float2 end = make_float2(step[0] * 1.00001f, step[1] * 1.00001f);
+  const float2 slack = make_float2(
+      1e-5f * (step[0] + fmaxf(fabsf(p.x.x), fabsf(p.y.x))),
+      1e-5f * (step[1] + fmaxf(fabsf(p.x.y), fabsf(p.y.y))));
+  for (int j = 0; j < a.n_shapes && (search[0] || search[1]); ++j) {
+    const float4 s = __ldg(a.shapes + 2 * j), h = __ldg(a.shapes + 2 * j + 1);
+    const int kind = __float_as_int(h.y);
+    const float2 dz = sub2(p.z, dup2(s.z));
+    bool near0, near1;
+    if (kind == PP_TARGET_SPHERE || kind == PP_TARGET_LINE) {
+      const float2 dx = sub2(p.x, dup2(s.x)), dy = sub2(p.y, dup2(s.y));
+      float2 c = fma2(v.x, dx, mul2(v.y, dy)), q = fma2(dx, dx, mul2(dy, dy));
+      if (kind == PP_TARGET_SPHERE) {
+        c = fma2(v.z, dz, c);
+        q = fma2(dz, dz, q);
       }
-      for (int m = 1; m <= nm; ++m) {
-        if (shape_hit<kPrecise>(a.shapes, j + m, pos, dir, step, &d)) {
-          hit = m + nm * line_no - 1;
-          break;
+      const float2 b = fma2(q, dup2(4e-6f), fma2(c, c, sub2(dup2(s.w), q)));
+      near0 = b.x >= 0.0f;
+      near1 = b.y >= 0.0f;
+    } else {  // a horizontal shape: where the segment crosses its height
+      const float2 t = mul2(dz, along);
+      const float2 x = sub2(fma2(v.x, t, p.x), dup2(s.x)), y = sub2(fma2(v.y, t, p.y), dup2(s.y));
+      const bool rect = kind == PP_TARGET_RECTANGLE;
+      const float wx = (rect ? s.w : sqrtf(s.w)) * 1.0001f, wy = rect ? h.x * 1.0001f : wx;
+      near0 = t.x >= 0.0f && t.x <= end.x && fabsf(x.x) <= wx + slack.x && fabsf(y.x) <= wy + slack.x;
+      near1 = t.y >= 0.0f && t.y <= end.y && fabsf(x.y) <= wx + slack.y && fabsf(y.y) <= wy + slack.y;
+    }
+    if (near0 || near1) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if (!(search[i] && (i ? near1 : near0))) continue;
+        if (kind == PP_TARGET_LINE) {
+          float dl;
+          if (!sphere_hit<kPrecise>(s, make_float3(pos[i].x, pos[i].y, 0.0f),
+                                    make_float3(dir[i].x, dir[i].y, 0.0f), step[i], &dl))
+            continue;
+          search[i] = false;
+          const int nm = __float_as_int(h.x);
+          for (int m = 1; m <= nm; ++m) {
+            if (shape_hit<kPrecise>(a.shapes, j + m, pos[i], dir[i], step[i], &d[i])) {
+              hit[i] = m + nm * (line_no + 1) - 1;
+              break;
+            }
+          }
+        } else if (shape_hit<kPrecise>(a.shapes, j, pos[i], dir[i], step[i], &d[i])) {
+          hit[i] = j;
+          search[i] = false;
         }
       }
-      break;
     }
-    if (shape_hit<kPrecise>(a.shapes, j, pos, dir, step, &d)) {
-      hit = j;
-      break;
+    if (kind == PP_TARGET_LINE) {
+      ++line_no;
+      j += __float_as_int(h.x);
     }
   }
-  if (hit < 0) return false;
-  key[own] = (k << 16) | (uint32_t)hit;
-  best.hx[own] = madd<kPrecise>(dir.x, d, pos.x);
-  best.hy[own] = madd<kPrecise>(dir.y, d, pos.y);
-  best.hz[own] = madd<kPrecise>(dir.z, d, pos.z);
-  best.ox[own] = dir.x;
-  best.oy[own] = dir.y;
-  best.oz[own] = dir.z;
-  best.dist[own] = dist0 + d;
-  return true;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    if (hit[i] < 0) continue;
+    open[i] = false;
+    const int own = lane + 32 * i;
+    key[own] = (k << 16) | (uint32_t)hit[i];
+    best.hx[own] = madd<kPrecise>(dir[i].x, d[i], pos[i].x);
+    best.hy[own] = madd<kPrecise>(dir[i].y, d[i], pos[i].y);
+    best.hz[own] = madd<kPrecise>(dir[i].z, d[i], pos[i].z);
+    best.ox[own] = dir[i].x;
+    best.oy[own] = dir[i].y;
+    best.oz[own] = dir[i].z;
+    best.dist[own] = (i ? dist0.y : dist0.x) + d[i];
+  }
 }
 
 // What a hit's record needs: the emission again, and the hit itself.
@@ -660,7 +710,7 @@ __global__ void __launch_bounds__(kMaxBlockThreads, PP_PROPAGATE_MIN_BLOCKS)
       __syncwarp();
       // heights of the raw and the clipped stack (warp-uniform)
       int n1 = 0, n2 = 0;
-      bool found0 = false, found1 = false;  // shaped targets: the photon has hit
+      bool open[2] = {active0, active1};  // shaped targets: the photon has not hit yet
       // The step loop holds neither the clip nor the walk: it stops when 32 raw
       // entries wait, they are clipped, 32 clipped ones are walked as soon as
       // they wait, and the loop resumes; after the last step the same code
@@ -673,13 +723,9 @@ __global__ void __launch_bounds__(kMaxBlockThreads, PP_PROPAGATE_MIN_BLOCKS)
           const uint4 r1 = philox_words(ph1, pt, a.round_keys);
           const float2 step = step_lengths<kPrecise>(r0.x, r1.x, sca_len);
           if constexpr (kShapes) {
-            if (active0 && !found0)
-              found0 = search_shapes<kPrecise>(a, first(w.pos), first(w.dir), step.x,
-                                               w.dist.x - w.comp.x, (uint32_t)k, q.key, best, lane);
-            if (active1 && !found1)
-              found1 = search_shapes<kPrecise>(a, second(w.pos), second(w.dir), step.y,
-                                               w.dist.y - w.comp.y, (uint32_t)k, q.key, best,
-                                               lane + 32);
+            search_shapes<kPrecise>(a, w.pos, w.dir, step,
+                                    make_float2(w.dist.x - w.comp.x, w.dist.y - w.comp.y),
+                                    (uint32_t)k, q.key, best, lane, open);
           } else {
             bool clear0, clear1;
             segments_clear<kSmemGrid>(a.sgrid, field, w.pos, w.dir, step, &clear0, &clear1);
