@@ -611,8 +611,8 @@ def bench_detection(pp, torch, local, n=100_000_000, reps=5):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                          "frac": achieved / hbm if hbm else None,
                          "note": "40 algorithmic bytes per hit; peak = measured copy bandwidth. "
-                                 "The kernel is instruction-issue bound, not HBM-bound: each hit "
-                                 "evaluates acos, sqrt and exp2 for 16 PMTs"},
+                                 "The kernel streams whole 80-byte records (88 bytes a hit with "
+                                 "its results), which is what bounds it"},
             "cpu_baseline": {"value": cpu_rate, "unit": "hits/s", "cores": 1, "kind": "port",
                              "sample": f"numpy oracle on the first {m} records"}}
 
