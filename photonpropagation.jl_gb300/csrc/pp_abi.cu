@@ -255,6 +255,15 @@ int build_queue(pp_ctx* ctx, bool wait = true) {
   return PP_OK;
 }
 
+// Grid and safety field go to shared memory when two CTAs of the configured
+// size still fit on an SM; otherwise both are read from global memory.
+bool fits_smem(const pp_ctx* ctx, uint32_t field_bytes) {
+  if (ctx->tuning.grid_in_global) return false;
+  return pp::propagate_smem_bytes(ctx->grid.blob_bytes, field_bytes, true,
+                                  ctx->tuning.block_threads, nullptr, nullptr) <=
+         pp::smem_budget(ctx->tuning.block_threads);
+}
+
 int rebuild_grid(pp_ctx* ctx, float cell_size) {
   cudaFree(ctx->d_blob);
   ctx->d_blob = nullptr;
@@ -272,7 +281,12 @@ int rebuild_grid(pp_ctx* ctx, float cell_size) {
   cudaFree(ctx->d_safety);
   ctx->d_safety = nullptr;
   float hs = ctx->tuning.safety_cell;
-  if (!(hs > 0.0f)) hs = (float)pp::SafetyDev::auto_cell(g.lo, g.hi, n);
+  if (!(hs > 0.0f)) {
+    hs = (float)pp::SafetyDev::auto_cell(g.lo, g.hi, n);
+    pp::SafetyDev shape{};
+    shape.set_shape(g.lo, g.hi, hs);
+    if (!fits_smem(ctx, shape.bytes)) hs = (float)pp::SafetyDev::auto_cell(g.lo, g.hi, n, false);
+  }
   pp::SafetyDev sg{};
   unsigned char* field = nullptr;
   if (pp::build_safety(ctx->d_targets, n, g, hs, ctx->stream, &sg, &field, &err) != 0)
@@ -298,14 +312,7 @@ int check_ready(const pp_ctx* ctx) {
   return PP_OK;
 }
 
-// Grid and safety field go to shared memory when two CTAs of the configured
-// size still fit on an SM; otherwise both are read from global memory.
-bool use_smem_grid(const pp_ctx* ctx) {
-  if (ctx->tuning.grid_in_global) return false;
-  return pp::propagate_smem_bytes(ctx->grid.blob_bytes, ctx->sgrid.bytes, true,
-                                  ctx->tuning.block_threads, nullptr, nullptr) <=
-         pp::smem_budget(ctx->tuning.block_threads);
-}
+bool use_smem_grid(const pp_ctx* ctx) { return fits_smem(ctx, ctx->sgrid.bytes); }
 
 LaunchArgs make_args(const pp_ctx* ctx, long long seed, int n_steps, pp_hit_record* hits,
                      long long capacity, pp_counters* ctr) {
