@@ -449,6 +449,43 @@ bool bound_applies(const pp_pom_model& m) {
 // without; 1e6: 72 and 83).
 constexpr long long kManyHits = 1 << 20;
 
+// A call's targets and models reach the device as kernel parameters, which a launch
+// takes when it is made: the caller's structures, and the image they are gathered
+// in, are free when the call returns, also under stream capture and where a copy
+// from pageable memory is asynchronous.
+constexpr int kSmallImage = 250, kLargeImage = 2040;  // 16-byte words a launch carries
+template <int kWords>
+struct ImagePart {
+  uint4 w[kWords];
+};
+template <int kWords>
+__global__ void __launch_bounds__(256)
+    write_kernel(uint4* __restrict__ dst, const __grid_constant__ ImagePart<kWords> part, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) dst[i] = part.w[i];
+}
+// Room for `bytes` and, after them, for what a launch reads past the last part.
+std::vector<unsigned char> host_image(size_t bytes) {
+  return std::vector<unsigned char>(bytes + sizeof(ImagePart<kLargeImage>));
+}
+// The first `bytes` (a multiple of 16) of a host_image to device memory.
+cudaError_t write_image(void* dst, std::vector<unsigned char>& image, size_t bytes,
+                        cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
+  size_t words = bytes / 16, at = 0;
+  while (e == cudaSuccess && at < words) {
+    const bool small = words - at <= (size_t)kSmallImage;
+    int n = (int)std::min<size_t>(words - at, small ? kSmallImage : kLargeImage);
+    uint4* to = static_cast<uint4*>(dst) + at;
+    void* params[] = {&to, image.data() + 16 * at, &n};
+    e = cudaLaunchKernel(small ? (const void*)write_kernel<kSmallImage>
+                               : (const void*)write_kernel<kLargeImage>,
+                         dim3((unsigned)((n + 255) / 256)), dim3(256), params, 0, s);
+    at += n;
+  }
+  return e;
+}
+
 __global__ void tres_kernel(const pp_hit_record* __restrict__ rec, long long n,
                             const double* __restrict__ tgeo, int n_targets, double t0,
                             double* __restrict__ tres) {
@@ -529,7 +566,7 @@ PP_API int pp_make_hits_from_photons_models(const pp_hit_record* d_records, int6
   const bool many = pom && n >= kManyHits && bound_applies(*pom);
   const size_t total = ob_place + (many ? sizeof(float4) * (size_t)n_targets : 0);
   const size_t alloc = total + (many ? sizeof(float2) * kMapSize * kMapSize : 0);
-  std::vector<unsigned char> image(total);  // one copy (pageable: taken before the call returns)
+  std::vector<unsigned char> image = host_image(total);
   if (n_targets > 0) memcpy(image.data(), targets, sizeof(pp_pmt_target) * n_targets);
   if (pom) memcpy(image.data() + ob_pom, pom, sizeof(pp_pom_model));
   if (dom) memcpy(image.data() + ob_dom, dom, sizeof(pp_dom_model));
@@ -543,8 +580,7 @@ PP_API int pp_make_hits_from_photons_models(const pp_hit_record* d_records, int6
   }
   unsigned char* buf = nullptr;
   cudaError_t e = cudaMallocAsync((void**)&buf, alloc, s);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(buf, image.data(), total, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = write_image(buf, image, total, s);
   if (e != cudaSuccess) {
     if (buf) cudaFreeAsync(buf, s);
     return pp::report_error(PP_ERR_CUDA, std::string(kWho) + cudaGetErrorString(e));
