@@ -191,8 +191,19 @@ constexpr size_t kHitsOffset = 128;  // of the hits in the result buffer
 constexpr long long kFirstRows = 256;
 constexpr size_t kPinnedQueue = 256 * 1024;
 
+// Waits for an upload that is still in flight: launches on other streams are not
+// ordered after it.
+void finish_upload(pp_ctx* ctx) {
+  if (ctx->queue_in_flight) cudaStreamSynchronize(ctx->stream);
+  ctx->queue_in_flight = false;
+}
+struct UploadScope {
+  pp_ctx* ctx;
+  ~UploadScope() { finish_upload(ctx); }
+};
+
 // The work queue of ctx->h_sources on the device.  Without `wait` the upload is
-// only ordered before later work on ctx->stream.
+// only ordered before later work on ctx->stream, and the caller holds an UploadScope.
 int build_queue(pp_ctx* ctx, bool wait = true) {
   const int n = (int)ctx->h_sources.size();
   auto up16 = [](size_t v) { return (v + 15) & ~(size_t)15; };
@@ -896,12 +907,10 @@ PP_API int pp_propagate(pp_ctx* ctx, const pp_source* sources, int32_t n_src, in
   ctx->last_hits = 0;
   ctx->h_rows = 0;
   DeviceScope ds(ctx->device);
+  UploadScope upload{ctx};  // the sources are set whatever follows
   int rc = set_sources(ctx, sources, n_src, photon_scaling, false);
   if (rc == PP_OK) rc = check_ready(ctx);
-  if (rc != PP_OK) {
-    cudaStreamSynchronize(ctx->stream);  // the sources are set all the same
-    return rc;
-  }
+  if (rc != PP_OK) return rc;
   // A photon hits at most once: the device buffer never needs more rows than
   // there are photons.
   const long long dev_cap = std::max<long long>(1, std::min<long long>(capacity, ctx->total_photons));
@@ -909,12 +918,8 @@ PP_API int pp_propagate(pp_ctx* ctx, const pp_source* sources, int32_t n_src, in
     cudaFree(ctx->d_result);
     ctx->d_result = nullptr;
     ctx->d_hits_cap = 0;
-    const cudaError_t e =
-        cudaMalloc(&ctx->d_result, kHitsOffset + sizeof(pp_hit_record) * dev_cap);
-    if (e != cudaSuccess) {
-      cudaStreamSynchronize(ctx->stream);
-      return cuda_error(e, "cudaMalloc(hit buffer)");
-    }
+    PP_CUDA(cudaMalloc(&ctx->d_result, kHitsOffset + sizeof(pp_hit_record) * dev_cap),
+            "cudaMalloc(hit buffer)");
     ctx->d_ctr = reinterpret_cast<pp_counters*>(ctx->d_result);
     ctx->d_hits = reinterpret_cast<pp_hit_record*>(ctx->d_result + kHitsOffset);
     ctx->d_hits_cap = dev_cap;
