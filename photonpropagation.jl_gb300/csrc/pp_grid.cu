@@ -213,6 +213,110 @@ __global__ void fp32_peak_kernel(float* __restrict__ sink, int iters) {
 
 }  // namespace
 
+namespace {
+
+// The grid of the box `bb` with cells of edge h (made coarser if there would be too
+// many).
+int build_grid_at(const pp_sphere* targets_dev, int n, const float* bb, const double* ext, double h,
+                  cudaStream_t stream, GridDev* grid_out, unsigned char** blob_out,
+                  long long* n_items_out, std::string* err) {
+  auto fail = [&](const std::string& m) {
+    if (err) *err = m;
+    return -1;
+  };
+  GridDev g{};
+  // Keep the cell count bounded.
+  const double kMaxCells = 4.0 * 1024 * 1024;
+  for (int guard = 0; guard < 64; ++guard) {
+    double cells = 1.0;
+    for (int a = 0; a < 3; ++a) cells *= std::max(1.0, std::ceil(ext[a] / h));
+    if (cells <= kMaxCells) break;
+    h *= 1.25;
+  }
+  for (int a = 0; a < 3; ++a) {
+    g.dims[a] = (int)std::max(1.0, std::ceil(ext[a] / h));
+    g.lo[a] = bb[a];
+    g.cell[a] = (float)h;
+    g.inv_cell[a] = (float)(1.0 / h);
+    g.hi[a] = (float)((double)bb[a] + g.dims[a] * h);
+  }
+  g.n_cells = g.dims[0] * g.dims[1] * g.dims[2];
+  g.n_targets = n;
+
+  unsigned *d_counts = nullptr, *d_start = nullptr, *d_cursor = nullptr, *d_tot = nullptr;
+  auto cleanup = [&]() {
+    cudaFree(d_counts);
+    cudaFree(d_start);
+    cudaFree(d_cursor);
+    cudaFree(d_tot);
+  };
+  const size_t cbytes = (size_t)g.n_cells * sizeof(unsigned);
+  if (cudaMalloc(&d_counts, cbytes) != cudaSuccess || cudaMalloc(&d_start, cbytes) != cudaSuccess ||
+      cudaMalloc(&d_cursor, cbytes) != cudaSuccess || cudaMalloc(&d_tot, 2 * sizeof(unsigned)) != cudaSuccess) {
+    cleanup();
+    return fail("cudaMalloc(grid scratch) failed");
+  }
+  cudaMemsetAsync(d_counts, 0, cbytes, stream);
+  cudaMemsetAsync(d_cursor, 0, cbytes, stream);
+  const int tb = 256;
+  count_kernel<<<(n + tb - 1) / tb, tb, 0, stream>>>(g, targets_dev, n, d_counts);
+  scan_kernel<<<1, 1024, 0, stream>>>(d_counts, g.n_cells, d_start, d_tot);
+  unsigned tot[2];
+  cudaError_t e = cudaMemcpyAsync(tot, d_tot, sizeof(tot), cudaMemcpyDeviceToHost, stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  if (e != cudaSuccess) {
+    cleanup();
+    return fail(std::string("grid count: ") + cudaGetErrorString(e));
+  }
+  const long long n_items = tot[0];
+  if (n_items > (long long)kCellStartMask || tot[1] > kCellMaxCount) {
+    cleanup();
+    char buf[200];
+    snprintf(buf, sizeof(buf),
+             "grid too dense (%lld items, %u in one cell): choose a smaller cell size", n_items,
+             tot[1]);
+    fail(buf);
+    return kGridTooDense;
+  }
+  auto pad16 = [](size_t b) { return (b + 15) & ~(size_t)15; };
+  const size_t cells_b = pad16(cbytes);
+  const size_t items_b = pad16((size_t)std::max<long long>(n_items, 1) * sizeof(uint16_t));
+  const size_t sph_b = (size_t)n * sizeof(float4);
+  g.off_items = (uint32_t)cells_b;
+  g.off_spheres = (uint32_t)(cells_b + items_b);
+  const size_t total = cells_b + items_b + sph_b;
+  if (total > 0xffffffffull) {
+    cleanup();
+    return fail("grid blob larger than 4 GiB");
+  }
+  g.blob_bytes = (uint32_t)total;
+  unsigned char* blob = nullptr;
+  if (cudaMalloc(&blob, total) != cudaSuccess) {
+    cleanup();
+    return fail("cudaMalloc(grid blob) failed");
+  }
+  cudaMemsetAsync(blob, 0, total, stream);
+  fill_kernel<<<(n + tb - 1) / tb, tb, 0, stream>>>(g, targets_dev, n, d_start, d_cursor,
+                                                   reinterpret_cast<uint16_t*>(blob + g.off_items));
+  const int m = std::max(g.n_cells, n);
+  pack_kernel<<<(m + tb - 1) / tb, tb, 0, stream>>>(
+      d_counts, d_start, g.n_cells, reinterpret_cast<uint32_t*>(blob), targets_dev, n,
+      reinterpret_cast<float4*>(blob + g.off_spheres));
+  e = cudaStreamSynchronize(stream);
+  cleanup();
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    cudaFree(blob);
+    return fail(std::string("grid build: ") + cudaGetErrorString(e));
+  }
+  *grid_out = g;
+  *blob_out = blob;
+  *n_items_out = n_items;
+  return 0;
+}
+
+}  // namespace
+
 int build_grid(const pp_sphere* targets_dev, int n, float cell_size, cudaStream_t stream,
                GridDev* grid_out, unsigned char** blob_out, long long* n_items_out,
                std::string* err) {
@@ -256,97 +360,16 @@ int build_grid(const pp_sphere* targets_dev, int n, float cell_size, cudaStream_
     ext[a] = std::max(1e-3, (double)bb[3 + a] - (double)bb[a]);
     vol *= ext[a];
   }
-  double h = cell_size;
-  // (400 modules: 8 cells per target 15.0 ms per 1e8 photons, 16 15.7, 4 15.2:
-  // fewer cells to cross against more spheres per cell)
-  if (!(h > 0.0)) h = std::cbrt(vol / (8.0 * n));  // about 8 cells per target
-  // Keep the cell count bounded.
-  const double kMaxCells = 4.0 * 1024 * 1024;
-  for (int guard = 0; guard < 64; ++guard) {
-    double cells = 1.0;
-    for (int a = 0; a < 3; ++a) cells *= std::max(1.0, std::ceil(ext[a] / h));
-    if (cells <= kMaxCells) break;
-    h *= 1.25;
+  // An automatic cell that gathers more spheres than its count can hold (a dense
+  // cluster in a wide list) is made smaller.
+  int rc = kGridTooDense;
+  for (int i = 0; i < kAutoCells && rc == kGridTooDense; ++i) {
+    const bool given = cell_size > 0.0f;
+    const double h = given ? cell_size : std::cbrt(vol / (kAutoCellsPerTarget[i] * n));
+    rc = build_grid_at(targets_dev, n, bb, ext, h, stream, grid_out, blob_out, n_items_out, err);
+    if (given) break;
   }
-  for (int a = 0; a < 3; ++a) {
-    g.dims[a] = (int)std::max(1.0, std::ceil(ext[a] / h));
-    g.lo[a] = bb[a];
-    g.cell[a] = (float)h;
-    g.inv_cell[a] = (float)(1.0 / h);
-    g.hi[a] = (float)((double)bb[a] + g.dims[a] * h);
-  }
-  g.n_cells = g.dims[0] * g.dims[1] * g.dims[2];
-  g.n_targets = n;
-
-  unsigned *d_counts = nullptr, *d_start = nullptr, *d_cursor = nullptr, *d_tot = nullptr;
-  auto cleanup = [&]() {
-    cudaFree(d_counts);
-    cudaFree(d_start);
-    cudaFree(d_cursor);
-    cudaFree(d_tot);
-  };
-  const size_t cbytes = (size_t)g.n_cells * sizeof(unsigned);
-  if (cudaMalloc(&d_counts, cbytes) != cudaSuccess || cudaMalloc(&d_start, cbytes) != cudaSuccess ||
-      cudaMalloc(&d_cursor, cbytes) != cudaSuccess || cudaMalloc(&d_tot, 2 * sizeof(unsigned)) != cudaSuccess) {
-    cleanup();
-    return fail("cudaMalloc(grid scratch) failed");
-  }
-  cudaMemsetAsync(d_counts, 0, cbytes, stream);
-  cudaMemsetAsync(d_cursor, 0, cbytes, stream);
-  const int tb = 256;
-  count_kernel<<<(n + tb - 1) / tb, tb, 0, stream>>>(g, targets_dev, n, d_counts);
-  scan_kernel<<<1, 1024, 0, stream>>>(d_counts, g.n_cells, d_start, d_tot);
-  unsigned tot[2];
-  e = cudaMemcpyAsync(tot, d_tot, sizeof(tot), cudaMemcpyDeviceToHost, stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-  if (e != cudaSuccess) {
-    cleanup();
-    return fail(std::string("grid count: ") + cudaGetErrorString(e));
-  }
-  const long long n_items = tot[0];
-  if (n_items > (long long)kCellStartMask || tot[1] > kCellMaxCount) {
-    cleanup();
-    char buf[200];
-    snprintf(buf, sizeof(buf),
-             "grid too dense (%lld items, %u in one cell): choose a smaller cell size", n_items,
-             tot[1]);
-    return fail(buf);
-  }
-  auto pad16 = [](size_t b) { return (b + 15) & ~(size_t)15; };
-  const size_t cells_b = pad16(cbytes);
-  const size_t items_b = pad16((size_t)std::max<long long>(n_items, 1) * sizeof(uint16_t));
-  const size_t sph_b = (size_t)n * sizeof(float4);
-  g.off_items = (uint32_t)cells_b;
-  g.off_spheres = (uint32_t)(cells_b + items_b);
-  const size_t total = cells_b + items_b + sph_b;
-  if (total > 0xffffffffull) {
-    cleanup();
-    return fail("grid blob larger than 4 GiB");
-  }
-  g.blob_bytes = (uint32_t)total;
-  unsigned char* blob = nullptr;
-  if (cudaMalloc(&blob, total) != cudaSuccess) {
-    cleanup();
-    return fail("cudaMalloc(grid blob) failed");
-  }
-  cudaMemsetAsync(blob, 0, total, stream);
-  fill_kernel<<<(n + tb - 1) / tb, tb, 0, stream>>>(g, targets_dev, n, d_start, d_cursor,
-                                                   reinterpret_cast<uint16_t*>(blob + g.off_items));
-  const int m = std::max(g.n_cells, n);
-  pack_kernel<<<(m + tb - 1) / tb, tb, 0, stream>>>(
-      d_counts, d_start, g.n_cells, reinterpret_cast<uint32_t*>(blob), targets_dev, n,
-      reinterpret_cast<float4*>(blob + g.off_spheres));
-  e = cudaStreamSynchronize(stream);
-  cleanup();
-  if (e == cudaSuccess) e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    cudaFree(blob);
-    return fail(std::string("grid build: ") + cudaGetErrorString(e));
-  }
-  *grid_out = g;
-  *blob_out = blob;
-  *n_items_out = n_items;
-  return 0;
+  return rc;
 }
 
 int build_safety(const pp_sphere* targets_dev, int n, const GridDev& grid, float cell,
@@ -397,8 +420,10 @@ int build_grid_into(const pp_sphere* targets_dev, int n, const GridDev& shape, u
   if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) return fail(std::string("grid count: ") + cudaGetErrorString(e));
   const long long n_items = tot[0];
-  if (n_items > (long long)kCellStartMask || tot[1] > kCellMaxCount)
-    return fail("grid too dense: choose a smaller cell size");
+  if (n_items > (long long)kCellStartMask || tot[1] > kCellMaxCount) {
+    fail("grid too dense: choose a smaller cell size");
+    return kGridTooDense;
+  }
   auto pad16 = [](size_t b) { return (b + 15) & ~(size_t)15; };
   const size_t cells_b = pad16(cbytes);
   const size_t items_b = pad16((size_t)std::max<long long>(n_items, 1) * sizeof(uint16_t));

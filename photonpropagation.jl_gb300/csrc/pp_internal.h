@@ -153,6 +153,12 @@ struct WarpBest {
 constexpr uint32_t kCellStartBits = 20;                    // first item index
 constexpr uint32_t kCellStartMask = (1u << kCellStartBits) - 1u;
 constexpr uint32_t kCellMaxCount = (1u << (32 - kCellStartBits)) - 1u;
+// Automatic cells: 8 per target, 16 for lists that are too dense for that.  (400
+// modules: 8 15.0 ms per 1e8 photons, 16 15.7, 4 15.2: fewer cells to cross against
+// more spheres per cell.)
+constexpr double kAutoCellsPerTarget[] = {8.0, 16.0};
+constexpr int kAutoCells = 2;
+constexpr int kGridTooDense = 1;                           // of build_grid, build_grid_into
 constexpr float kGridMargin = 0.01f;                       // m, AABB inflation
 
 // Phase-function constants derived once per medium.
@@ -331,7 +337,8 @@ int propagate_occupancy(int block_threads, bool precise, bool smem_tables, uint3
                         uint32_t safety_bytes);
 
 // Grid build on the device (pp_grid.cu).  targets_dev: n spheres in device
-// memory.  Returns 0 on success; *blob_out is allocated with cudaMalloc.
+// memory.  Returns 0 on success, kGridTooDense or -1; *blob_out is allocated with
+// cudaMalloc.
 int build_grid(const pp_sphere* targets_dev, int n, float cell_size, cudaStream_t stream,
                GridDev* grid_out, unsigned char** blob_out, long long* n_items_out,
                std::string* err);

@@ -94,7 +94,8 @@ long long scaled_photons(long long photons, float scaling) {
 
 // Grid shape from the host copy of the targets, with the
 // same box, automatic cell sizes and limits as pp_set_targets.
-void grid_shape(const pp_sphere* t, int n, float cell_size, pp::GridDev* g) {
+void grid_shape(const pp_sphere* t, int n, float cell_size, double cells_per_target,
+                pp::GridDev* g) {
   *g = pp::GridDev{};
   if (n <= 0) {
     for (int a = 0; a < 3; ++a) {
@@ -117,7 +118,7 @@ void grid_shape(const pp_sphere* t, int n, float cell_size, pp::GridDev* g) {
     vol *= ext[a];
   }
   double h = cell_size;
-  if (!(h > 0.0)) h = std::cbrt(vol / (8.0 * n));
+  if (!(h > 0.0)) h = std::cbrt(vol / (cells_per_target * n));
   for (int guard = 0; guard < 64; ++guard) {
     double cells = 1.0;
     for (int a = 0; a < 3; ++a) cells *= std::max(1.0, std::ceil(ext[a] / h));
@@ -211,10 +212,6 @@ extern "C" PP_API int pp_propagate_static(
   if (num_sms < 1) return fail(PP_ERR_CUDA, "device reports no multiprocessors");
 
   // ---- host-side shapes and the work queue ----
-  pp::GridDev gshape;
-  grid_shape(targets, n_targets, cell_size, &gshape);
-  pp::SafetyDev sshape;
-  sshape.set_shape(gshape.lo, gshape.hi, pp::SafetyDev::auto_cell(gshape.lo, gshape.hi, n_targets));
   const int ppt = 8, block = 1024;
   const long long chunk = 32LL * ppt;
   std::vector<unsigned long long> prefix(n_src + 1, 0);
@@ -249,19 +246,35 @@ extern "C" PP_API int pp_propagate_static(
   unsigned long long* d_prefix = ar.take<unsigned long long>(n_src + 1);
   long long* d_photons = ar.take<long long>(std::max(n_src, 1));
   pp_counters* d_ctr = ar.take<pp_counters>(1);
-  unsigned* d_counts = ar.take<unsigned>(gshape.n_cells);
-  unsigned* d_start = ar.take<unsigned>(gshape.n_cells);
-  unsigned* d_cursor = ar.take<unsigned>(gshape.n_cells);
-  unsigned* d_totals = ar.take<unsigned>(2);
-  const size_t blob_cap = (((size_t)gshape.n_cells * 4 + 15) & ~(size_t)15) +
-                          ((item_bound(targets, n_targets, gshape) * 2 + 15) & ~(size_t)15) + 16 +
-                          (size_t)n_targets * sizeof(float4);
-  unsigned char* d_blob = ar.take<unsigned char>(blob_cap);
-  unsigned char* d_field = ar.take<unsigned char>(sshape.bytes);
-  if (ar.overflow)
-    return fail(PP_ERR_INVALID, "inputs need more scratch than the " +
-                                    std::to_string(PP_STATIC_SCRATCH_BYTES >> 20) +
-                                    " MiB static array holds (fewer targets, sources or table knots)");
+  // the rest is the grid's and the safety field's
+  const Arena inputs = ar;
+  pp::GridDev gshape;
+  pp::SafetyDev sshape;
+  unsigned *d_counts, *d_start, *d_cursor, *d_totals;
+  unsigned char *d_blob, *d_field;
+  size_t blob_cap = 0;
+  auto carve_grid = [&](double cells_per_target) {
+    ar = inputs;
+    grid_shape(targets, n_targets, cell_size, cells_per_target, &gshape);
+    sshape = pp::SafetyDev{};
+    sshape.set_shape(gshape.lo, gshape.hi,
+                     pp::SafetyDev::auto_cell(gshape.lo, gshape.hi, n_targets));
+    d_counts = ar.take<unsigned>(gshape.n_cells);
+    d_start = ar.take<unsigned>(gshape.n_cells);
+    d_cursor = ar.take<unsigned>(gshape.n_cells);
+    d_totals = ar.take<unsigned>(2);
+    blob_cap = (((size_t)gshape.n_cells * 4 + 15) & ~(size_t)15) +
+               ((item_bound(targets, n_targets, gshape) * 2 + 15) & ~(size_t)15) + 16 +
+               (size_t)n_targets * sizeof(float4);
+    d_blob = ar.take<unsigned char>(blob_cap);
+    d_field = ar.take<unsigned char>(sshape.bytes);
+    return ar.overflow ? fail(PP_ERR_INVALID,
+                              "inputs need more scratch than the " +
+                                  std::to_string(PP_STATIC_SCRATCH_BYTES >> 20) +
+                                  " MiB static array holds (fewer targets, sources or table knots)")
+                       : PP_OK;
+  };
+  if ((rc = carve_grid(pp::kAutoCellsPerTarget[0])) != PP_OK) return rc;
 
   // ---- inputs into the scratch (copies only; nothing is allocated) ----
   auto h2d = [&](void* dst, const void* src, size_t bytes) {
@@ -283,9 +296,15 @@ extern "C" PP_API int pp_propagate_static(
   std::string err;
   pp::GridDev grid;
   long long n_items = 0;
-  if (pp::build_grid_into(d_targets, n_targets, gshape, d_counts, d_start, d_cursor, d_totals,
-                          d_blob, blob_cap, stream, &grid, &n_items, &err) != 0)
-    return fail(PP_ERR_INVALID, "grid: " + err);
+  for (int i = 0;;) {
+    const int built =
+        pp::build_grid_into(d_targets, n_targets, gshape, d_counts, d_start, d_cursor, d_totals,
+                            d_blob, blob_cap, stream, &grid, &n_items, &err);
+    if (built == 0) break;
+    if (built != pp::kGridTooDense || cell_size > 0.0f || ++i == pp::kAutoCells)
+      return fail(PP_ERR_INVALID, "grid: " + err);
+    if ((rc = carve_grid(pp::kAutoCellsPerTarget[i])) != PP_OK) return rc;
+  }
   if (pp::build_safety_into(d_targets, n_targets, sshape, d_field, stream, &err) != 0)
     return fail(PP_ERR_CUDA, err);
 
