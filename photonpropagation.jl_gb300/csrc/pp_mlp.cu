@@ -1286,13 +1286,15 @@ namespace {
 
 void mlp_free(pp_mlp* m) {
   cudaFree(m->P); cudaFree(m->G); cudaFree(m->Mo); cudaFree(m->Vo); cudaFree(m->P16);
-  cudaFree(m->X0); cudaFree(m->O); cudaFree(m->dO16);
+  cudaFree(m->dO16);
   cudaFree(m->dZ[0]); cudaFree(m->dZ[1]); cudaFree(m->loss); cudaFree(m->err);
   cudaFree(m->wpack);
   cudaFree(m->wf); cudaFree(m->wb); cudaFree(m->tiles); cudaFree(m->loss_acc); cudaFree(m->ctl);
   cudaFree(m->bx); cudaFree(m->bc); cudaFree(m->bh); cudaFree(m->d_step); cudaFree(m->d_sched);
   if (m->step_graph) cudaGraphExecDestroy(m->step_graph);
   if (m->cap_stream) cudaStreamDestroy(m->cap_stream);
+  if (m->rows_path) return;  // (the rest is part of m->tiles)
+  cudaFree(m->X0); cudaFree(m->O);
   for (auto* p : m->Z) cudaFree(p);
   for (auto* p : m->Y) cudaFree(p);
 }
@@ -1468,10 +1470,10 @@ cudaError_t rows_attributes(const pp_mlp* m) {
   return e;
 }
 
-// Blocks of one batch, carved from m->tiles: inputs, the layers' activations,
-// pre-activations and their gradients, the head's gradient.
+// Blocks of one batch, carved from m->tiles: inputs, the head's gradient, the layers'
+// activations, and their pre-activations, over which the gradients of these go.
 struct RowsTiles {
-  unsigned char *x0, *y, *z, *dz, *dout;
+  unsigned char *x0, *dout, *y, *z;
   size_t layer, total;
 };
 RowsTiles rows_tiles(const pp_mlp* m) {
@@ -1483,9 +1485,22 @@ RowsTiles rows_tiles(const pp_mlp* m) {
   t.dout = p; p += rows * m->out_pad * 2;
   t.y = p; p += t.layer * m->n_layers;
   t.z = p; p += t.layer * m->n_layers;
-  t.dz = p; p += t.layer * m->n_layers;
   t.total = (size_t)(p - m->tiles);
   return t;
+}
+// pp_mlp_forward's arrays in the same memory (no step needs another call's blocks),
+// its FP32 outputs after them.
+size_t tiles_bytes(const pp_mlp* m) {
+  return rows_tiles(m).total + sizeof(float) * (size_t)m->max_batch * m->out_pad;
+}
+void forward_tiles(pp_mlp* m) {
+  const RowsTiles t = rows_tiles(m);
+  m->X0 = reinterpret_cast<bf16*>(t.x0);
+  for (int l = 0; l < m->n_layers; ++l) {
+    m->Y[l] = reinterpret_cast<bf16*>(t.y + (size_t)l * t.layer);
+    m->Z[l] = reinterpret_cast<bf16*>(t.z + (size_t)l * t.layer);
+  }
+  m->O = reinterpret_cast<float*>(m->tiles + t.total);
 }
 
 // Forward, loss and all gradients of a batch into m->G and m->loss_acc (which
@@ -1506,7 +1521,7 @@ int rows_gradients(pp_mlp* m, const float* x, const float* count, const float* h
     p.wb_off[l] = m->wb_off[l];
     p.bias[l] = m->P + m->off_b[l];
   }
-  p.x0 = t.x0; p.y = t.y; p.z = t.z; p.dz = t.dz; p.dout = t.dout; p.layer_bytes = t.layer;
+  p.x0 = t.x0; p.y = t.y; p.z = t.z; p.dout = t.dout; p.layer_bytes = t.layer;
   p.gbias = m->G + m->off_b[L]; p.loss = m->loss_acc;
   p.act_bytes = m->rows_act; p.err = m->err; p.wait_ns = kWaitNs;
   const dim3 grid((unsigned)((B + pprows::kRows - 1) / pprows::kRows));
@@ -1522,7 +1537,7 @@ int rows_gradients(pp_mlp* m, const float* x, const float* count, const float* h
       for (int j = 0; j < nt; ++j) {
         // (128 columns of a block of 8-row groups are 128 * 16 bytes apart)
         pprows::DwTile& w = d.tile[d.n_tiles++];
-        w.a = l < L ? t.dz + (size_t)l * t.layer + (size_t)i * 2048 : t.dout;
+        w.a = l < L ? t.z + (size_t)l * t.layer + (size_t)i * 2048 : t.dout;
         w.a_cols = l < L ? m->hidden : m->out_pad;
         w.rows = l < L ? 128 : m->out_pad;
         w.b = l == 0 ? t.x0 : t.y + (size_t)(l - 1) * t.layer + (size_t)j * 2048;
@@ -1640,17 +1655,20 @@ PP_API int pp_mlp_create(pp_mlp** out, int32_t device, int32_t n_in, int32_t hid
   };
   A((void**)&m->P, pb); A((void**)&m->G, pb); A((void**)&m->Mo, pb); A((void**)&m->Vo, pb);
   A((void**)&m->P16, sizeof(bf16) * off);
-  A((void**)&m->X0, sizeof(bf16) * Bn * m->in_pad);
   m->Z.assign(n_layers, nullptr);
   m->Y.assign(n_layers, nullptr);
-  for (int l = 0; l < n_layers; ++l) {
-    A((void**)&m->Z[l], sizeof(bf16) * Bn * hidden);
-    A((void**)&m->Y[l], sizeof(bf16) * Bn * hidden);
+  rows_setup(m);
+  if (!m->rows_path) {
+    A((void**)&m->X0, sizeof(bf16) * Bn * m->in_pad);
+    for (int l = 0; l < n_layers; ++l) {
+      A((void**)&m->Z[l], sizeof(bf16) * Bn * hidden);
+      A((void**)&m->Y[l], sizeof(bf16) * Bn * hidden);
+    }
+    A((void**)&m->O, sizeof(float) * Bn * m->out_pad);
+    A((void**)&m->dO16, sizeof(bf16) * Bn * m->out_pad);
+    A((void**)&m->dZ[0], sizeof(bf16) * Bn * hidden);
+    A((void**)&m->dZ[1], sizeof(bf16) * Bn * hidden);
   }
-  A((void**)&m->O, sizeof(float) * Bn * m->out_pad);
-  A((void**)&m->dO16, sizeof(bf16) * Bn * m->out_pad);
-  A((void**)&m->dZ[0], sizeof(bf16) * Bn * hidden);
-  A((void**)&m->dZ[1], sizeof(bf16) * Bn * hidden);
   A((void**)&m->loss, sizeof(float));
   A((void**)&m->err, sizeof(unsigned));
   long long wbytes = 0;
@@ -1659,7 +1677,6 @@ PP_API int pp_mlp_create(pp_mlp** out, int32_t device, int32_t n_in, int32_t hid
     wbytes += (long long)m->rows[l] * m->cols[l] * 2;  // rows, cols multiples of 16: 512-byte steps
   }
   A((void**)&m->wpack, (size_t)wbytes);
-  rows_setup(m);
   if (m->rows_path) {
     // each pack holds every weight once; blocks start at multiples of 16 bytes
     uint32_t wf = 0, wb = 0;
@@ -1671,7 +1688,8 @@ PP_API int pp_mlp_create(pp_mlp** out, int32_t device, int32_t n_in, int32_t hid
     }
     A((void**)&m->wf, wf);
     A((void**)&m->wb, std::max(wb, 16u));
-    A((void**)&m->tiles, rows_tiles(m).total);
+    A((void**)&m->tiles, tiles_bytes(m));
+    forward_tiles(m);
     A((void**)&m->loss_acc, sizeof(float));
     A((void**)&m->ctl, sizeof(pprows::TrainCtl));
     A((void**)&m->d_sched, sizeof(float) * 4);

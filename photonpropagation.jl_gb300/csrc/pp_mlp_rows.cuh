@@ -75,8 +75,9 @@ struct RowsParams {
   const unsigned char *wf, *wb;
   uint32_t wf_off[kMaxLayers], wb_off[kMaxLayers];
   const float* bias[kMaxLayers];
-  unsigned char *x0, *y, *z, *dz, *dout;  // 64-row blocks; layer l of y, z, dz at
-                                          // l * layer_bytes (z in rows_kernel's own order)
+  // 64-row blocks; layer l of y and z at l * layer_bytes.  z: pre-activations in
+  // rows_kernel's own order, and over them, once a CTA has read them, their gradients
+  unsigned char *x0, *y, *z, *dout;
   size_t layer_bytes;
   float *gbias, *loss;                    // the head's bias gradient, the batch loss
   uint32_t act_bytes;                     // one activation buffer
@@ -109,7 +110,7 @@ __device__ __forceinline__ unsigned char* operand_home(const RowsParams& p, int 
   unsigned char* base = n == 0       ? p.x0
                         : n <= L     ? p.y + (size_t)(n - 1) * p.layer_bytes
                         : n == L + 1 ? p.dout
-                                     : p.dz + (size_t)(2 * L + 1 - n) * p.layer_bytes;
+                                     : p.z + (size_t)(2 * L + 1 - n) * p.layer_bytes;
   return base + (size_t)blockIdx.x * (size_t)(kRows * K * 2);
 }
 __device__ __forceinline__ void bulk_store(void* dst, uint32_t src, uint32_t bytes) {
@@ -436,6 +437,8 @@ __global__ void __launch_bounds__(kRowsThreads, 1)
                 out + pptc::core_offset(ra + 8 * (e & 1), k * 8 + cgrp * 2 + (e >> 1), kHidden) +
                 2 * cl) = bf16x2(x.x, x.y);
           }
+          // (the pre-activations are written and read: their place is the bulk store's)
+          if (!fwd && k + 1 == kParts) asm volatile("fence.proxy.async.global;" ::: "memory");
           if (n + 1 < n_jobs) arrive(&go[k]);
           if (fwd) zt[k * kEpiThreads] = make_uint4(z[0], z[1], z[2], z[3]);
         }
