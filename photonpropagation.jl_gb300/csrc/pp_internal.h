@@ -307,7 +307,8 @@ struct LaunchArgs {
 
 // Dynamic shared memory of one CTA: [grid blob | safety field] when staged,
 // then the per-warp state (the queues, whose room the shaped targets' hits use).
-static_assert(sizeof(WarpBest) <= offsetof(WarpQueue, key), "shares the stacks' room");
+static_assert(sizeof(WarpBest) <= offsetof(WarpQueue, clip_t), "shares the stacks' room");
+static_assert(sizeof(int) * kGroup <= sizeof(float2) * kClippedCap, "the list of a group's hits");
 inline size_t propagate_smem_bytes(uint32_t blob_bytes, uint32_t safety_bytes, bool smem_tables,
                                    int block_threads, uint32_t* safety_offset,
                                    uint32_t* state_offset) {

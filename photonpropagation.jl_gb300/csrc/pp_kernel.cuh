@@ -254,9 +254,9 @@ __device__ __forceinline__ int clip_entries(WarpQueue& q, int base, int c, int n
 // mean one 3): an entry of length l is cut into
 // 1 + floor(l / (total / (32 - c))) equal pieces, overlapping by the clip slack,
 // one lane each.  The earliest (step, target) per photon wins via a shared
-// atomicMin on the key (step << 16 | target).
+// atomicMin on the key (step << 16 | target).  Returns whether there was a hit.
 template <bool P>
-__device__ __forceinline__ void test_queue(WarpQueue& q, int base, int c,
+__device__ __forceinline__ bool test_queue(WarpQueue& q, int base, int c,
                                            const GridDev& g, const uint32_t* cells,
                                            const uint16_t* items, const float4* sph, int lane) {
   // pieces of this lane's entry, in units of 1/64 m so that the sums are exact
@@ -280,6 +280,7 @@ __device__ __forceinline__ void test_queue(WarpQueue& q, int base, int c,
   const int m = __shfl_sync(0xffffffffu, n, el);
   const int piece = lane - (31 - __clz(starts));
   const int e = base + el;
+  int j = -1;
   if (piece < m) {
     const float4 ea = q.clip_a[e], eb = q.clip_b[e];
     const float2 t = q.clip_t[e];
@@ -287,14 +288,15 @@ __device__ __forceinline__ void test_queue(WarpQueue& q, int base, int c,
     const float ta = piece == 0 ? t.x : fmaxf(fmaf((float)piece, w, t.x) - kClipSlack, t.x);
     const float tb =
         piece == m - 1 ? t.y : fminf(fmaf((float)(piece + 1), w, t.x) + kClipSlack, t.y);
-    const int j = first_hit<P>(g, cells, items, sph, make_float3(ea.x, ea.y, ea.z),
-                               make_float3(eb.x, eb.y, eb.z), ea.w, ta, tb);
+    j = first_hit<P>(g, cells, items, sph, make_float3(ea.x, ea.y, ea.z),
+                     make_float3(eb.x, eb.y, eb.z), ea.w, ta, tb);
     if (j >= 0) {
       const uint32_t meta = __float_as_uint(eb.w);
       atomicMin(&q.key[meta & (kGroup - 1u)], ((meta >> 8) << 16) | (uint32_t)j);
     }
   }
   __syncwarp();
+  return __any_sync(0xffffffffu, j >= 0);
 }
 
 // Append one hit: one atomic per warp for all lanes that record in this pass;
@@ -429,6 +431,10 @@ __device__ __forceinline__ PhotonInit init_photon(const LaunchArgs& a, int s, ui
 #ifndef PP_PROPAGATE_MIN_BLOCKS
 #define PP_PROPAGATE_MIN_BLOCKS 1
 #endif
+
+// Where photons that have hit go on (m): outside every safety field by more than any
+// step is long, and with a square that FP32 holds in units of any node spacing.
+constexpr float kFarAway = 1e12f;
 
 // The step lengths of the two photons from their first random words.
 template <bool kPrecise>
@@ -761,22 +767,45 @@ __global__ void __launch_bounds__(kMaxBlockThreads, PP_PROPAGATE_MIN_BLOCKS)
         if (n2 >= 32 || (last && n2 > 0)) {
           const int take = min(n2, 32);
           n2 -= take;
-          test_queue<kPrecise>(q, n2, take, a.grid, cells, items, sph, lane);
+          const bool hits = test_queue<kPrecise>(q, n2, take, a.grid, cells, items, sph, lane);
+          if (hits && !last) {
+            // No later step of a photon with a hit: it goes on far from every target
+            // (its hit is replayed), and the steps end when that is all of them.
+            // Earlier steps may still wait.
+            const bool hit0 = q.key[lane] != 0xffffffffu, hit1 = q.key[lane + 32] != 0xffffffffu;
+            w.pos.x.x = hit0 ? kFarAway : w.pos.x.x;
+            w.pos.x.y = hit1 ? kFarAway : w.pos.x.y;
+            if (__all_sync(0xffffffffu, (hit0 || !active0) && (hit1 || !active1)))
+              k = a.n_steps + 1;
+          }
         }
         if (last && n2 == 0) break;
       }
       __syncwarp();
 
-#pragma unroll 1
-      for (int j = 0; j < 2; ++j) {
-        const int own = lane + 32 * j;
-        const bool active = own < count;
-        const uint32_t key = q.key[own];
-        bool overflowed = false;
-        int steps_taken = a.n_steps;
-        if (active && key != 0xffffffffu) {
-          steps_taken = (int)(key >> 16);
-          const uint32_t plo = j ? plo1 : plo0;
+      constexpr uint32_t kNone = 0xffffffffu;
+      const uint32_t key0 = active0 ? q.key[lane] : kNone;
+      const uint32_t key1 = active1 ? q.key[lane + 32] : kNone;
+      const bool hit0 = key0 != kNone, hit1 = key1 != kNone;
+      if (active0) steps_acc += hit0 ? key0 >> 16 : (uint32_t)a.n_steps;
+      if (active1) steps_acc += hit1 ? key1 >> 16 : (uint32_t)a.n_steps;
+      sim_acc += (unsigned)active0 + (unsigned)active1;
+      // The group's hits, gathered so that one lane takes each: a pass of replays lasts
+      // as long as its latest hit, and 32 hits are one pass whichever photons have them.
+      // (With this and the steps above: 5e6 photons beside a sphere that half of them
+      // hit 1.09 -> 0.97 ms, 1e6 among 300 spheres of 3 m 0.52 -> 0.48, 1e8 in the
+      // 400-module detector 13.15 -> 13.09.)
+      const unsigned m0 = __ballot_sync(0xffffffffu, hit0), m1 = __ballot_sync(0xffffffffu, hit1);
+      const int n_hit = __popc(m0) + __popc(m1);
+      if (n_hit > 0) {
+        int* list = reinterpret_cast<int*>(q.clip_t);  // (free, and past a WarpBest)
+        if (hit0) list[__popc(m0 & lanemask_lt)] = lane;
+        if (hit1) list[__popc(m0) + __popc(m1 & lanemask_lt)] = lane + 32;
+        __syncwarp();
+        for (int h = lane; h < n_hit; h += 32) {
+          const int own = list[h];
+          const uint32_t key = q.key[own], plo = (uint32_t)pb + (uint32_t)own;
+          const int steps_taken = (int)(key >> 16);
           Hit hit;
           if constexpr (kShapes) {
             hit.in = init_photon<kPrecise>(a, s, plo, phi);
@@ -800,14 +829,12 @@ __global__ void __launch_bounds__(kMaxBlockThreads, PP_PROPAGATE_MIN_BLOCKS)
             atomicAdd(row + 1 + bin, abs_w);
             atomicAdd(u64(&a.counters->n_hits), 1ull);
           } else {
+            bool overflowed = false;
             record_hit(a, hit.pos, hit.in.wl, hit.dir, hit.dist, hit.in.dir, abs_w, time,
                        (long long)(((unsigned long long)phi << 32) | plo),
                        (int)(key & 0xffffu) + 1, steps_taken, s, &overflowed);
+            if (overflowed) sim_acc -= 1;
           }
-        }
-        if (active) {
-          steps_acc += (unsigned long long)steps_taken;
-          if (!overflowed) sim_acc += 1;
         }
       }
       __syncwarp();  // the hits are read before the next group clears them
