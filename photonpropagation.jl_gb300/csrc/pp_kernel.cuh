@@ -486,12 +486,13 @@ __device__ __forceinline__ void advance(const PhaseDev& ph, Walk2& w, float2 ste
 // closes it; a list of detector lines is searched line by line
 // (src/photon_prop_cuda.jl:611-634): the 2-D test of the line, then its modules;
 // the first crossed line ends the search.  Both photons take one pass over the
-// list.  Packed operations first decide for both whether the exact test can
-// succeed: a circle's discriminant not below zero by more than the rounding of
-// either form (at most 1.5e-6 of the squared distance q), or a horizontal shape's
-// box, a little enlarged, crossed inside the segment.  1e7 photons, 400 spheres: 68
-// ms with one photon per lane, 97 with the exact test for one photon after the
-// other, 59 now; 5e6 photons, 20 lines of 20: 2.4, 3.0 and 1.9 ms.
+// list.  Horizontal shapes: shape_hit in packed operations, each half rounding as it
+// does (1e6 photons, 20 discs of 50 m: 284 us with one photon per lane, 397 with a
+// wider packed test before shape_hit, 283 now; 50 discs of 2 m: 1,270, 1,342 and
+// 828).  Spheres and lines: packed operations decide first whether sphere_hit can
+// succeed, the discriminant being below zero by no more than the rounding of either
+// form (at most 1.5e-6 of the squared distance q).  1e7 photons, 400 spheres: 68 ms
+// with one photon per lane, 97 with sphere_hit for one photon after the other, 54 now.
 template <bool kPrecise>
 __device__ __forceinline__ void search_shapes(const LaunchArgs& a, const Vec2& p, const Vec2& v,
                                               float2 steps, float2 dist0, uint32_t k,
@@ -503,14 +504,14 @@ __device__ __forceinline__ void search_shapes(const LaunchArgs& a, const Vec2& p
   int hit[2] = {-1, -1};  // 0-based module index to report
   float d[2] = {0.0f, 0.0f};
   int line_no = 0;
-  // (the distance above a shape, times `along`, is the way to its height; the
-  // crossing point is off by less than `slack`)
-  const float2 along = make_float2(-1.0f / copysignf(fmaxf(fabsf(v.z.x), 1e-30f), v.z.x),
-                                   -1.0f / copysignf(fmaxf(fabsf(v.z.y), 1e-30f), v.z.y));
-  const float2 end = make_float2(step[0] * 1.00001f, step[1] * 1.00001f);
-  const float2 slack = make_float2(
-      1e-5f * (step[0] + fmaxf(fabsf(p.x.x), fabsf(p.y.x))),
-      1e-5f * (step[1] + fmaxf(fabsf(p.x.y), fabsf(p.y.y))));
+  // 1 / v.z as shape_hit's division takes it; in the replay variant, which divides, a
+  // value that makes the way to a shape's height no longer than it is
+  float2 rz;
+  if constexpr (kPrecise)
+    rz = make_float2(1.0f / copysignf(fmaxf(fabsf(v.z.x), 1e-30f), v.z.x),
+                     1.0f / copysignf(fmaxf(fabsf(v.z.y), 1e-30f), v.z.y));
+  else
+    rz = make_float2(f_rcp<false>(v.z.x), f_rcp<false>(v.z.y));
   for (int j = 0; j < a.n_shapes && (search[0] || search[1]); ++j) {
     const float4 s = __ldg(a.shapes + 2 * j), h = __ldg(a.shapes + 2 * j + 1);
     const int kind = __float_as_int(h.y);
@@ -526,13 +527,25 @@ __device__ __forceinline__ void search_shapes(const LaunchArgs& a, const Vec2& p
       const float2 b = fma2(q, dup2(4e-6f), fma2(c, c, sub2(dup2(s.w), q)));
       near0 = b.x >= 0.0f;
       near1 = b.y >= 0.0f;
-    } else {  // a horizontal shape: where the segment crosses its height
-      const float2 t = mul2(dz, along);
-      const float2 x = sub2(fma2(v.x, t, p.x), dup2(s.x)), y = sub2(fma2(v.y, t, p.y), dup2(s.y));
-      const bool rect = kind == PP_TARGET_RECTANGLE;
-      const float wx = (rect ? s.w : sqrtf(s.w)) * 1.0001f, wy = rect ? h.x * 1.0001f : wx;
-      near0 = t.x >= 0.0f && t.x <= end.x && fabsf(x.x) <= wx + slack.x && fabsf(y.x) <= wy + slack.x;
-      near1 = t.y >= 0.0f && t.y <= end.y && fabsf(x.y) <= wx + slack.y && fabsf(y.y) <= wy + slack.y;
+    } else {  // a horizontal shape: the way to its height is in the segment
+      const float2 t = mul2(sub2(dup2(s.z), p.z), rz);
+      if constexpr (kPrecise) {
+        near0 = !(t.x < 0.0f || t.x > step[0] * 1.00001f);
+        near1 = !(t.y < 0.0f || t.y > step[1] * 1.00001f);
+      } else {  // and, rounding as in shape_hit, ends in the shape
+        const float2 x = sub2(fma2(v.x, t, p.x), dup2(s.x));
+        const float2 y = sub2(fma2(v.y, t, p.y), dup2(s.y));
+        if (kind == PP_TARGET_RECTANGLE) {
+          near0 = fabsf(x.x) < s.w && fabsf(y.x) < h.x;
+          near1 = fabsf(x.y) < s.w && fabsf(y.y) < h.x;
+        } else {
+          const float2 r2 = add2(mul2(x, x), mul2(y, y));
+          near0 = r2.x < s.w;
+          near1 = r2.y < s.w;
+        }
+        near0 = near0 && !(t.x < 0.0f || t.x > step[0]);
+        near1 = near1 && !(t.y < 0.0f || t.y > step[1]);
+      }
     }
     if (near0 || near1) {
 #pragma unroll
@@ -621,7 +634,8 @@ __device__ __noinline__ void replay_hit(const LaunchArgs& a, int s, uint32_t plo
 // kShapes: shaped targets (a.shapes), every target tested at every step in
 // index order (no grid, no deferred queue).
 template <bool kPrecise, bool kSmemGrid, bool kShapes = false>
-__global__ void __launch_bounds__(kMaxBlockThreads, PP_PROPAGATE_MIN_BLOCKS)
+__global__ void __launch_bounds__(kShapes ? kShapesThreads : kMaxBlockThreads,
+                                  kShapes ? kShapesBlocks : PP_PROPAGATE_MIN_BLOCKS)
     propagate_kernel(const __grid_constant__ LaunchArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) unsigned long long bar;
@@ -732,6 +746,7 @@ __global__ void __launch_bounds__(kMaxBlockThreads, PP_PROPAGATE_MIN_BLOCKS)
             search_shapes<kPrecise>(a, w.pos, w.dir, step,
                                     make_float2(w.dist.x - w.comp.x, w.dist.y - w.comp.y),
                                     (uint32_t)k, q.key, best, lane, open);
+            if (!__any_sync(0xffffffffu, open[0] || open[1])) break;
           } else {
             bool clear0, clear1;
             segments_clear<kSmemGrid>(a.sgrid, field, w.pos, w.dir, step, &clear0, &clear1);

@@ -42,6 +42,10 @@ cudaError_t launch_propagate(const LaunchArgs& args, int block_threads, int ctas
   const void* k = select_kernel(precise, smem_grid, shapes);
   if (block_threads > 1024 || block_threads % 32)
     return cudaErrorInvalidValue;
+  if (shapes && block_threads > kShapesBlock) {  // (as many warps an SM as were asked for)
+    ctas_per_sm *= propagate_warps(block_threads) / propagate_warps(kShapesBlock);
+    block_threads = kShapesBlock;
+  }
   const int threads = propagate_warps(block_threads) * 32;
   LaunchArgs a = args;
   const size_t smem = propagate_smem_bytes(args.grid.blob_bytes, args.sgrid.bytes, smem_grid,
