@@ -27,7 +27,7 @@ def test_same_hits_at_every_launch_shape(pp, gpu_ctx, lines):
         for ctas in (0, 1, 3):
             ctx.set_tuning(block_threads=block, ctas_per_sm=ctas)
             rc, hits, sim = ctx.propagate(setup.source_records(), 1, setup.seed, 15, 1.0, 30_000)
-            assert rc == 0 and hits > 1000 and sim == 30_000
+            assert rc == 0 and hits > 0 and sim == 30_000  # (something to compare)
             cols = ctx.fetch_hits(hits)
             order = np.argsort(cols["photon_index"])
             got = {k: v[order] for k, v in cols.items()}
