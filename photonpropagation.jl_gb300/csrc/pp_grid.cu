@@ -132,41 +132,90 @@ __global__ void pack_kernel(const unsigned* __restrict__ counts, const unsigned*
   }
 }
 
-// One thread per safety node: min over spheres of |c - s| - r - margin,
-// floored to the quantum.  Targets are staged through shared memory.
-__global__ void safety_kernel(const SafetyDev sg, const pp_sphere* __restrict__ t, int n,
-                              unsigned char* __restrict__ out) {
-  __shared__ float4 sh[256];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  float cx = 0.0f, cy = 0.0f, cz = 0.0f;
-  if (i < sg.n_cells) {
-    const int x = i % sg.dims[0];
-    const int y = (i / sg.dims[0]) % sg.dims[1];
-    const int z = i / (sg.dims[0] * sg.dims[1]);
-    cx = sg.lo[0] + x * sg.cell;
-    cy = sg.lo[1] + y * sg.cell;
-    cz = sg.lo[2] + z * sg.cell;
-  }
+// The safety field, a brick of 8 x 8 x 4 nodes per CTA and a node per thread: the
+// least |c - s| - r - margin over the spheres, floored to the quantum.  All spheres are
+// passed over twice for a brick and not once for each of its nodes: for the nearest to
+// its centre, then for those that may be nearest to one of its nodes, which are kept
+// in shared memory.  Where these are too many (a cluster seen from afar, a wide
+// spacing), a node goes through all spheres, or, in a field of more than kExactPairs
+// nodes times spheres, takes what the distance from the centre proves.
+// pp_set_targets, ms, with 32k nodes that each went through all spheres, with up to
+// 2e10 such distances, and now: 9,000 spheres 0.82, 2.95, 0.42 (540k nodes); 20,000
+// 2.0, 11.4, 1.1; 65,000 5.3, 12.9, 5.1 (3.9e6).
+constexpr int kBrickX = 8, kBrickY = 8, kBrickZ = 4, kBrick = kBrickX * kBrickY * kBrickZ;
+constexpr int kNearSpheres = 1024;
+constexpr double kExactPairs = 2e10;  // 8 ms
+__global__ void __launch_bounds__(kBrick)
+    safety_kernel(const SafetyDev sg, const pp_sphere* __restrict__ t, int n, bool exact,
+                  unsigned char* __restrict__ out) {
+  __shared__ float4 near[kNearSpheres];
+  __shared__ float warp_best[kBrick / 32];
+  __shared__ int n_near;
+  const int bx = (sg.dims[0] + kBrickX - 1) / kBrickX, by = (sg.dims[1] + kBrickY - 1) / kBrickY;
+  const int b = blockIdx.x;
+  const int first[3] = {b % bx * kBrickX, b / bx % by * kBrickY, b / (bx * by) * kBrickZ};
+  const float centre[3] = {sg.lo[0] + (first[0] + 0.5f * (kBrickX - 1)) * sg.cell,
+                           sg.lo[1] + (first[1] + 0.5f * (kBrickY - 1)) * sg.cell,
+                           sg.lo[2] + (first[2] + 0.5f * (kBrickZ - 1)) * sg.cell};
+  auto sphere = [&](int j) {
+    return make_float4(t[j].position[0], t[j].position[1], t[j].position[2],
+                       t[j].radius + kGridMargin);
+  };
+  auto distance = [](float cx, float cy, float cz, float4 s) {
+    const float dx = cx - s.x, dy = cy - s.y, dz = cz - s.z;
+    return sqrtf(dx * dx + dy * dy + dz * dz) - s.w;
+  };
+  if (threadIdx.x == 0) n_near = 0;
   float best = 1e30f;
-  for (int base = 0; base < n; base += 256) {
-    const int j = base + threadIdx.x;
-    __syncthreads();
-    if (j < n)
-      sh[threadIdx.x] = make_float4(t[j].position[0], t[j].position[1], t[j].position[2],
-                                    t[j].radius + kGridMargin);
-    __syncthreads();
-    const int m = min(256, n - base);
-    for (int k = 0; k < m; ++k) {
-      const float4 s = sh[k];
-      const float dx = cx - s.x, dy = cy - s.y, dz = cz - s.z;
-      best = fminf(best, sqrtf(dx * dx + dy * dy + dz * dz) - s.w);
+  for (int j = threadIdx.x; j < n; j += kBrick)
+    best = fminf(best, distance(centre[0], centre[1], centre[2], sphere(j)));
+  for (int o = 16; o > 0; o >>= 1) best = fminf(best, __shfl_xor_sync(0xffffffffu, best, o));
+  if ((threadIdx.x & 31) == 0) warp_best[threadIdx.x >> 5] = best;
+  __syncthreads();
+  float from_centre = warp_best[0];
+  for (int w = 1; w < kBrick / 32; ++w) from_centre = fminf(from_centre, warp_best[w]);
+  const float radius = 0.5f * sg.cell * sqrtf((kBrickX - 1) * (kBrickX - 1) +
+                                              (kBrickY - 1) * (kBrickY - 1) +
+                                              (kBrickZ - 1) * (kBrickZ - 1)) * 1.0001f;
+  float slack = 1e-3f + 1e-4f * fabsf(from_centre);  // the rounding of distances and places
+  for (int a = 0; a < 3; ++a) slack += 1e-6f * fmaxf(fabsf(sg.lo[a]), fabsf(sg.hi[a]));
+  const bool far = from_centre - radius - slack > 256.0f * kSafetyQuantum;
+  if (!far) {
+    const float reach = from_centre + 2.0f * radius + 2.0f * slack;
+    for (int j = threadIdx.x; j < n; j += kBrick) {
+      const float4 s = sphere(j);
+      if (distance(centre[0], centre[1], centre[2], s) > reach) continue;
+      const int at = atomicAdd(&n_near, 1);
+      if (at < kNearSpheres) near[at] = s;
     }
   }
-  if (i < sg.n_cells) {
-    // 1 mm of slack covers the rounding of the distance itself
-    const float q = floorf((best - 1e-3f) / kSafetyQuantum);
-    out[i] = (unsigned char)fminf(fmaxf(q, 0.0f), 255.0f);
+  __syncthreads();
+  const int x = first[0] + threadIdx.x % kBrickX, y = first[1] + threadIdx.x / kBrickX % kBrickY;
+  const int z = first[2] + threadIdx.x / (kBrickX * kBrickY);
+  if (x >= sg.dims[0] || y >= sg.dims[1] || z >= sg.dims[2]) return;
+  const float cx = sg.lo[0] + x * sg.cell, cy = sg.lo[1] + y * sg.cell,
+              cz = sg.lo[2] + z * sg.cell;
+  best = 1e30f;
+  if (far || (n_near > kNearSpheres && !exact)) {
+    best = from_centre - distance(cx, cy, cz, make_float4(centre[0], centre[1], centre[2], 0.0f)) -
+           slack;
+  } else if (n_near > kNearSpheres) {
+    for (int j = 0; j < n; ++j) best = fminf(best, distance(cx, cy, cz, sphere(j)));
+  } else {
+    for (int k = 0; k < n_near; ++k) best = fminf(best, distance(cx, cy, cz, near[k]));
   }
+  // 1 mm of slack covers the rounding of the distance itself
+  const float q = floorf((best - 1e-3f) / kSafetyQuantum);
+  out[((long long)z * sg.dims[1] + y) * sg.dims[0] + x] =
+      (unsigned char)fminf(fmaxf(q, 0.0f), 255.0f);
+}
+void launch_safety(const SafetyDev& sg, const pp_sphere* targets_dev, int n, unsigned char* field,
+                   cudaStream_t stream) {
+  const long long bricks = (long long)((sg.dims[0] + kBrickX - 1) / kBrickX) *
+                           ((sg.dims[1] + kBrickY - 1) / kBrickY) *
+                           ((sg.dims[2] + kBrickZ - 1) / kBrickZ);
+  safety_kernel<<<(unsigned)bricks, kBrick, 0, stream>>>(
+      sg, targets_dev, n, (double)sg.n_cells * n <= kExactPairs, field);
 }
 
 __global__ void hits_to_columns_kernel(const pp_hit_record* __restrict__ rec, long long n,
@@ -386,7 +435,7 @@ int build_safety(const pp_sphere* targets_dev, int n, const GridDev& grid, float
   if (n <= 0) {
     cudaMemsetAsync(f, 255, (size_t)sg.n_cells, stream);
   } else {
-    safety_kernel<<<(sg.n_cells + 255) / 256, 256, 0, stream>>>(sg, targets_dev, n, f);
+    launch_safety(sg, targets_dev, n, f, stream);
   }
   cudaError_t e = cudaStreamSynchronize(stream);
   if (e == cudaSuccess) e = cudaGetLastError();
@@ -454,7 +503,7 @@ int build_safety_into(const pp_sphere* targets_dev, int n, const SafetyDev& shap
   if (n <= 0) {
     cudaMemsetAsync(d_field, 255, (size_t)shape.n_cells, stream);
   } else {
-    safety_kernel<<<(shape.n_cells + 255) / 256, 256, 0, stream>>>(shape, targets_dev, n, d_field);
+    launch_safety(shape, targets_dev, n, d_field, stream);
   }
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {

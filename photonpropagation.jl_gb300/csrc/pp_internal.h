@@ -103,15 +103,14 @@ inline void SafetyDev::set_shape(const float* blo, const float* bhi, double h) {
 // KB of the SM to L1.  400 modules, ms per 1e8 photons (per 4e7 of 256 emitters):
 // 34k nodes 13.54 (4.48), 48k 13.13 (4.46), 60k 13.16 (4.56), 72k 13.02 (4.54).
 // Tables that stay in global memory (staged false: some 1,700 spheres and more) have
-// no L1 to share: 60 nodes per sphere, as long as building them takes at most 2e10
-// distances (8 ms of an upload of 70).  2e6 photons in a 600 m cube, ms with 48k
-// nodes and with these: 4,000 spheres 1.35 and 1.08, 6,000 1.81 and 1.30, 20,000 3.94
-// and 2.52.
+// no L1 to share: 60 nodes per sphere.  2e6 photons in a 600 m cube, ms with 48k nodes
+// and with these, 16 warps an SM: 4,000 spheres 1.35 and 1.04, 20,000 3.94 and 2.34,
+// 60,000 6.4 and 4.0 (120 nodes 3.8).
 inline double SafetyDev::auto_cell(const float* blo, const float* bhi, int n, bool staged) {
   double vol = 1.0;
   for (int a = 0; a < 3; ++a) vol *= std::max(1e-6, (double)bhi[a] - (double)blo[a]);
   double nodes = std::min(std::max(120.0 * n, 2048.0), 48000.0);
-  if (!staged) nodes = std::max(nodes, std::min(60.0 * n, 2e10 / n));
+  if (!staged) nodes = std::max(nodes, 60.0 * n);
   double h = std::max(1e-3, std::cbrt(vol / nodes));
   for (int guard = 0; guard < 512 && safety_nodes(blo, bhi, h) > nodes; ++guard) h *= 1.02;
   return h;
