@@ -127,13 +127,28 @@ constexpr int kMaxBlockThreads = 32 * kSmWarps;
 inline int propagate_warps(int block_threads) {
   return (block_threads * kSmWarps + 1023) / 1024;
 }
-// Shaped targets stage no tables and take fewer registers: small CTAs fill an SM with
-// 20 warps (of 96) where one large CTA has 16 (1e6 photons, 50 discs of 2 m: 1,059 us
-// with 16 warps, 828 with 20; 400 spheres in the unculled loop, 2e6 photons: 13.8 and
-// 10.9 ms).
-constexpr int kShapesBlock = 256;  // block_threads at most
-constexpr int kShapesThreads = 32 * (kShapesBlock * kSmWarps / 1024);
-constexpr int kShapesBlocks = 5;   // an SM
+// Where a kernel's tables are.  The last two run small CTAs, so that registers and not
+// a CTA's size set the warps of an SM.
+enum class Tables {
+  kStaged,      // in shared memory
+  kGlobal,      // kept in global memory, or too large and a workload of one round of warps
+  kGlobalMany,  // too large for shared memory, more chunks than kManyChunks an SM
+  kShapes       // no tables: a list of shapes
+};
+// Tables that are too large: 32 warps of 64 registers, whose spills cost less than the
+// latency of L2 with 16 warps to hide it, as soon as 16 do not take the whole
+// workload at once.  60,000 spheres in a cube of 600 m, 2e6 photons: 4.02 ms with 16
+// warps, 3.29 with 24, 2.64 with 32 (200,000 photons 0.55 and 0.39, 155,000 0.338 and
+// 0.385); of 120 m: 5.12, 4.22, 3.28; 4,000 of 600 m: 1.05, 0.93, 0.83.  Shapes: 20 of
+// 96 (1e6 photons, 50 discs of 2 m: 1,059 us with 16 warps, 828 with 20; 400 spheres in
+// the unculled loop, 2e6 photons: 13.8 and 10.9 ms).
+constexpr int kManyChunks = 16;
+constexpr bool small_ctas(Tables t) { return t == Tables::kGlobalMany || t == Tables::kShapes; }
+constexpr int min_ctas(Tables t) {  // of an SM
+  return t == Tables::kGlobalMany ? 8 : t == Tables::kShapes ? 5 : 1;
+}
+constexpr int kSmallBlock = 256;  // in units of block_threads
+constexpr int kSmallThreads = 32 * (kSmallBlock * kSmWarps / 1024);
 
 // Per-warp shared-memory state of the propagation kernel: the step segments
 // whose hit test is deferred (two stacks: those not yet clipped by the safety
@@ -339,10 +354,6 @@ inline size_t smem_budget(int block_threads) {
 cudaError_t launch_propagate(const LaunchArgs& args, int block_threads, int ctas_per_sm,
                              bool precise, bool smem_grid, int num_sms, cudaStream_t stream,
                              int* grid_out);
-// Resident CTAs per SM for a configuration (occupancy calculator).
-int propagate_occupancy(int block_threads, bool precise, bool smem_tables, uint32_t blob_bytes,
-                        uint32_t safety_bytes);
-
 // Grid build on the device (pp_grid.cu).  targets_dev: n spheres in device
 // memory.  Returns 0 on success, kGridTooDense or -1; *blob_out is allocated with
 // cudaMalloc.

@@ -427,11 +427,6 @@ __device__ __forceinline__ PhotonInit init_photon(const LaunchArgs& a, int s, ui
   return in;
 }
 
-// One CTA of kMaxBlockThreads per SM caps the kernel at 128 registers.
-#ifndef PP_PROPAGATE_MIN_BLOCKS
-#define PP_PROPAGATE_MIN_BLOCKS 1
-#endif
-
 // Where photons that have hit go on (m): outside every safety field by more than any
 // step is long, and with a square that FP32 holds in units of any node spacing.
 constexpr float kFarAway = 1e12f;
@@ -633,10 +628,11 @@ __device__ __noinline__ void replay_hit(const LaunchArgs& a, int s, uint32_t plo
 
 // kShapes: shaped targets (a.shapes), every target tested at every step in
 // index order (no grid, no deferred queue).
-template <bool kPrecise, bool kSmemGrid, bool kShapes = false>
-__global__ void __launch_bounds__(kShapes ? kShapesThreads : kMaxBlockThreads,
-                                  kShapes ? kShapesBlocks : PP_PROPAGATE_MIN_BLOCKS)
+template <bool kPrecise, Tables kTables>
+__global__ void __launch_bounds__(small_ctas(kTables) ? kSmallThreads : kMaxBlockThreads,
+                                  min_ctas(kTables))
     propagate_kernel(const __grid_constant__ LaunchArgs a) {
+  constexpr bool kSmemGrid = kTables == Tables::kStaged, kShapes = kTables == Tables::kShapes;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) unsigned long long bar;
 
@@ -882,9 +878,18 @@ __global__ void __launch_bounds__(kShapes ? kShapesThreads : kMaxBlockThreads,
   }
 }
 
-template <bool P, bool S, bool Sh = false>
-const void* kernel_ptr() {
-  return reinterpret_cast<const void*>(&propagate_kernel<P, S, Sh>);
+template <bool P>
+const void* kernel_ptr(Tables t) {
+  switch (t) {
+    case Tables::kStaged:
+      return reinterpret_cast<const void*>(&propagate_kernel<P, Tables::kStaged>);
+    case Tables::kGlobal:
+      return reinterpret_cast<const void*>(&propagate_kernel<P, Tables::kGlobal>);
+    case Tables::kGlobalMany:
+      return reinterpret_cast<const void*>(&propagate_kernel<P, Tables::kGlobalMany>);
+    default:
+      return reinterpret_cast<const void*>(&propagate_kernel<P, Tables::kShapes>);
+  }
 }
 
 }  // namespace

@@ -3,48 +3,39 @@
 // the staged target grid).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "pp_kernel.cuh"
 
 namespace pp {
 
 // Replay variant, instantiated in pp_propagate_precise.cu.
-const void* precise_kernel_ptr(bool smem_grid, bool shapes);
+const void* precise_kernel_ptr(Tables t);
 
 namespace {
 
-const void* select_kernel(bool precise, bool smem_grid, bool shapes = false) {
-  if (precise) return precise_kernel_ptr(smem_grid, shapes);
-  if (shapes) return kernel_ptr<false, false, true>();
-  return smem_grid ? kernel_ptr<false, true>() : kernel_ptr<false, false>();
+const void* select_kernel(bool precise, Tables t) {
+  return precise ? precise_kernel_ptr(t) : kernel_ptr<false>(t);
 }
 
 }  // namespace
 
-int propagate_occupancy(int block_threads, bool precise, bool smem_tables, uint32_t blob_bytes,
-                        uint32_t safety_bytes) {
-  const void* k = select_kernel(precise, smem_tables);
-  const size_t smem_bytes = propagate_smem_bytes(blob_bytes, safety_bytes, smem_tables,
-                                                 block_threads, nullptr, nullptr);
-  if (smem_bytes > 48 * 1024)
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-  int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, propagate_warps(block_threads) * 32,
-                                                    smem_bytes) != cudaSuccess)
-    return 0;
-  return n;
-}
-
 cudaError_t launch_propagate(const LaunchArgs& args, int block_threads, int ctas_per_sm,
                              bool precise, bool smem_grid, int num_sms, cudaStream_t stream,
                              int* grid_out) {
-  const bool shapes = args.shapes != nullptr;
-  if (shapes) smem_grid = false;
-  const void* k = select_kernel(precise, smem_grid, shapes);
-  if (block_threads > 1024 || block_threads % 32)
-    return cudaErrorInvalidValue;
-  if (shapes && block_threads > kShapesBlock) {  // (as many warps an SM as were asked for)
-    ctas_per_sm *= propagate_warps(block_threads) / propagate_warps(kShapesBlock);
-    block_threads = kShapesBlock;
+  if (block_threads > 1024 || block_threads % 32) return cudaErrorInvalidValue;
+  if (args.shapes) smem_grid = false;
+  const bool fit = propagate_smem_bytes(args.grid.blob_bytes, args.sgrid.bytes, true, block_threads,
+                                        nullptr, nullptr) <= smem_budget(block_threads);
+  const Tables t =
+      args.shapes ? Tables::kShapes
+      : smem_grid ? Tables::kStaged
+      : !fit && args.total_chunks > (unsigned long long)(kManyChunks * num_sms) ? Tables::kGlobalMany
+                                                                                : Tables::kGlobal;
+  const void* k = select_kernel(precise, t);
+  if (small_ctas(t)) {  // the same share of an SM
+    ctas_per_sm = (std::min(ctas_per_sm, 32) * block_threads * min_ctas(t) + 1023) / 1024;
+    block_threads = kSmallBlock;
   }
   const int threads = propagate_warps(block_threads) * 32;
   LaunchArgs a = args;

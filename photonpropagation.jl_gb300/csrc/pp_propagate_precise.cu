@@ -10,9 +10,6 @@
 
 namespace pp {
 
-const void* precise_kernel_ptr(bool smem_grid, bool shapes) {
-  if (shapes) return kernel_ptr<true, false, true>();
-  return smem_grid ? kernel_ptr<true, true>() : kernel_ptr<true, false>();
-}
+const void* precise_kernel_ptr(Tables t) { return kernel_ptr<true>(t); }
 
 }  // namespace pp
