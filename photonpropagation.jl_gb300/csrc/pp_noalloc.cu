@@ -84,7 +84,13 @@ struct Arena {
     used = off + bytes;
     return reinterpret_cast<T*>(base + off);
   }
+  size_t left() const {
+    const size_t off = (used + 255) & ~(size_t)255;
+    return off < PP_STATIC_SCRATCH_BYTES ? PP_STATIC_SCRATCH_BYTES - off : 0;
+  }
 };
+
+constexpr size_t kLeastField = 4096;  // bytes of the safety field that are always there
 
 long long scaled_photons(long long photons, float scaling) {
   const float x = (float)photons * scaling;
@@ -214,6 +220,10 @@ extern "C" PP_API int pp_propagate_static(
   // ---- host-side shapes and the work queue ----
   const int ppt = 8, block = 1024;
   const long long chunk = 32LL * ppt;
+  auto fits = [&](const pp::GridDev& g, const pp::SafetyDev& f) {  // in shared memory
+    return pp::propagate_smem_bytes(g.blob_bytes, f.bytes, true, block, nullptr, nullptr) <=
+           pp::smem_budget(block);
+  };
   std::vector<unsigned long long> prefix(n_src + 1, 0);
   std::vector<long long> nph(std::max(n_src, 1), 0);
   for (int i = 0; i < n_src; ++i) {
@@ -249,16 +259,12 @@ extern "C" PP_API int pp_propagate_static(
   // the rest is the grid's and the safety field's
   const Arena inputs = ar;
   pp::GridDev gshape;
-  pp::SafetyDev sshape;
   unsigned *d_counts, *d_start, *d_cursor, *d_totals;
-  unsigned char *d_blob, *d_field;
+  unsigned char* d_blob;
   size_t blob_cap = 0;
   auto carve_grid = [&](double cells_per_target) {
     ar = inputs;
     grid_shape(targets, n_targets, cell_size, cells_per_target, &gshape);
-    sshape = pp::SafetyDev{};
-    sshape.set_shape(gshape.lo, gshape.hi,
-                     pp::SafetyDev::auto_cell(gshape.lo, gshape.hi, n_targets));
     d_counts = ar.take<unsigned>(gshape.n_cells);
     d_start = ar.take<unsigned>(gshape.n_cells);
     d_cursor = ar.take<unsigned>(gshape.n_cells);
@@ -267,12 +273,12 @@ extern "C" PP_API int pp_propagate_static(
                ((item_bound(targets, n_targets, gshape) * 2 + 15) & ~(size_t)15) + 16 +
                (size_t)n_targets * sizeof(float4);
     d_blob = ar.take<unsigned char>(blob_cap);
-    d_field = ar.take<unsigned char>(sshape.bytes);
-    return ar.overflow ? fail(PP_ERR_INVALID,
-                              "inputs need more scratch than the " +
-                                  std::to_string(PP_STATIC_SCRATCH_BYTES >> 20) +
-                                  " MiB static array holds (fewer targets, sources or table knots)")
-                       : PP_OK;
+    Arena least = ar;
+    least.take<unsigned char>(kLeastField);
+    if (!least.overflow) return (int)PP_OK;
+    return fail(PP_ERR_INVALID, "inputs need more scratch than the " +
+                                    std::to_string(PP_STATIC_SCRATCH_BYTES >> 20) +
+                                    " MiB static array holds (fewer targets, sources or table knots)");
   };
   if ((rc = carve_grid(pp::kAutoCellsPerTarget[0])) != PP_OK) return rc;
 
@@ -305,6 +311,18 @@ extern "C" PP_API int pp_propagate_static(
       return fail(PP_ERR_INVALID, "grid: " + err);
     if ((rc = carve_grid(pp::kAutoCellsPerTarget[i])) != PP_OK) return rc;
   }
+  // the field that pp_set_targets makes, or as fine as what is left of the scratch allows
+  pp::SafetyDev sshape{};
+  double spacing = pp::SafetyDev::auto_cell(grid.lo, grid.hi, n_targets);
+  sshape.set_shape(grid.lo, grid.hi, spacing);
+  if (!fits(grid, sshape)) {
+    spacing = pp::SafetyDev::auto_cell(grid.lo, grid.hi, n_targets, false);
+    sshape.set_shape(grid.lo, grid.hi, spacing);
+  }
+  while (sshape.bytes > ar.left() && sshape.bytes > kLeastField)
+    sshape.set_shape(grid.lo, grid.hi, spacing *= 1.02);
+  unsigned char* d_field = ar.take<unsigned char>(sshape.bytes);
+  if (ar.overflow) return fail(PP_ERR_INVALID, "no scratch left for the safety field");
   if (pp::build_safety_into(d_targets, n_targets, sshape, d_field, stream, &err) != 0)
     return fail(PP_ERR_CUDA, err);
 
@@ -338,9 +356,7 @@ extern "C" PP_API int pp_propagate_static(
   a.counters = d_ctr;
   a.wait_limit_ns = 2000000000ull;
   if (a.total_chunks > 0) {
-    const bool smem = pp::propagate_smem_bytes(grid.blob_bytes, sshape.bytes, true, block, nullptr,
-                                               nullptr) <= pp::smem_budget(block);
-    e = pp::launch_propagate(a, block, 0, false, smem, num_sms, stream, nullptr);
+    e = pp::launch_propagate(a, block, 0, false, fits(grid, sshape), num_sms, stream, nullptr);
     if (e != cudaSuccess) return cuda_fail(e, "launch propagate kernel");
   }
   pp_counters c{};
