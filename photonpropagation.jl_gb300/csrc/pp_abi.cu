@@ -147,6 +147,7 @@ struct pp_ctx {
   // sources and work queue
   std::vector<pp_source> h_sources;
   float scaling = 1.0f;
+  bool field_staged = true;  // stages_auto_field when the field was built
   // one device buffer {sources, prefix, photons} and its host image (pinned when
   // small), uploaded in one copy
   unsigned char* d_queue = nullptr;
@@ -266,13 +267,44 @@ int build_queue(pp_ctx* ctx, bool wait = true) {
   return PP_OK;
 }
 
-// Grid and safety field go to shared memory when two CTAs of the configured
-// size still fit on an SM; otherwise both are read from global memory.
+// Grid and safety field go to shared memory when as many CTAs of the configured size
+// as make up an SM's warps still fit on it (one of 1024); otherwise both are read from
+// global memory.
 bool fits_smem(const pp_ctx* ctx, uint32_t field_bytes) {
   if (ctx->tuning.grid_in_global) return false;
   return pp::propagate_smem_bytes(ctx->grid.blob_bytes, field_bytes, true,
                                   ctx->tuning.block_threads, nullptr, nullptr) <=
          pp::smem_budget(ctx->tuning.block_threads);
+}
+
+// Whether the automatic field of tables in shared memory fits there: what its spacing
+// is chosen by.
+bool stages_auto_field(const pp_ctx* ctx) {
+  const GridDev& g = ctx->grid;
+  pp::SafetyDev shape{};
+  shape.set_shape(g.lo, g.hi,
+                  (float)pp::SafetyDev::auto_cell(g.lo, g.hi, (int)ctx->h_targets.size()));
+  return fits_smem(ctx, shape.bytes);
+}
+
+// The safety field over the grid's box.
+int rebuild_field(pp_ctx* ctx) {
+  cudaFree(ctx->d_safety);
+  ctx->d_safety = nullptr;
+  const GridDev& g = ctx->grid;
+  const int n = (int)ctx->h_targets.size();
+  float hs = ctx->tuning.safety_cell;
+  ctx->field_staged = stages_auto_field(ctx);
+  if (!(hs > 0.0f)) hs = (float)pp::SafetyDev::auto_cell(g.lo, g.hi, n, ctx->field_staged);
+  std::string err;
+  pp::SafetyDev sg{};
+  unsigned char* field = nullptr;
+  if (pp::build_safety(ctx->d_targets, n, g, hs, ctx->stream, &sg, &field, &err) != 0)
+    return set_error(PP_ERR_CUDA, "pp_set_targets: %s", err.c_str());
+  ctx->sgrid = sg;
+  ctx->d_safety = field;
+  ctx->version++;
+  return PP_OK;
 }
 
 int rebuild_grid(pp_ctx* ctx, float cell_size) {
@@ -288,24 +320,7 @@ int rebuild_grid(pp_ctx* ctx, float cell_size) {
   ctx->grid = g;
   ctx->d_blob = blob;
   ctx->n_items = n_items;
-  // Safety field over the same box.
-  cudaFree(ctx->d_safety);
-  ctx->d_safety = nullptr;
-  float hs = ctx->tuning.safety_cell;
-  if (!(hs > 0.0f)) {
-    hs = (float)pp::SafetyDev::auto_cell(g.lo, g.hi, n);
-    pp::SafetyDev shape{};
-    shape.set_shape(g.lo, g.hi, hs);
-    if (!fits_smem(ctx, shape.bytes)) hs = (float)pp::SafetyDev::auto_cell(g.lo, g.hi, n, false);
-  }
-  pp::SafetyDev sg{};
-  unsigned char* field = nullptr;
-  if (pp::build_safety(ctx->d_targets, n, g, hs, ctx->stream, &sg, &field, &err) != 0)
-    return set_error(PP_ERR_CUDA, "pp_set_targets: %s", err.c_str());
-  ctx->sgrid = sg;
-  ctx->d_safety = field;
-  ctx->version++;
-  return PP_OK;
+  return rebuild_field(ctx);
 }
 
 int check_ready(const pp_ctx* ctx) {
@@ -758,6 +773,12 @@ PP_API int pp_set_tuning(pp_ctx* ctx, const pp_tuning* t) {
   }
   if (cell_changed && ctx->has_targets) {
     int rc = rebuild_grid(ctx, t->cell_size);
+    if (rc != PP_OK) return rc;
+  }
+  // an automatic field is sized by where the tables go
+  if (ctx->has_targets && !(t->safety_cell > 0.0f) &&
+      stages_auto_field(ctx) != ctx->field_staged) {
+    int rc = rebuild_field(ctx);
     if (rc != PP_OK) return rc;
   }
   return PP_OK;
