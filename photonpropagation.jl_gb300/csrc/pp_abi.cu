@@ -328,6 +328,8 @@ int check_ready(const pp_ctx* ctx) {
   if (!ctx->has_spectrum)
     return set_error(PP_ERR_NOT_READY, "spectrum not set (pp_set_spectrum / pp_set_monochromatic)");
   if (!ctx->has_targets) return set_error(PP_ERR_NOT_READY, "targets not set (pp_set_targets)");
+  if (!ctx->d_blob || !ctx->d_safety)  // their rebuild failed, as for a refused cell size
+    return set_error(PP_ERR_NOT_READY, "the targets' tables are not built (pp_set_tuning)");
   if (!ctx->has_sources) return set_error(PP_ERR_NOT_READY, "sources not set (pp_set_sources)");
   if (ctx->needs_track && ctx->n_track < 2)
     return set_error(PP_ERR_NOT_READY,

@@ -46,3 +46,28 @@ def test_accepted_with_the_hits_of_the_unculled_loop(pp, gpu_ctx):
     for k in runs[0]:
         for r, o in zip(runs[1:], order[1:]):
             np.testing.assert_array_equal(runs[0][k][order[0]], r[k][o], err_msg=k)
+
+
+@pytest.mark.gpu
+def test_refused_cell_size_leaves_no_targets(pp, gpu_ctx):
+    """A cell size that is refused leaves no tables: launches are refused too, until
+    another one is set."""
+    targets, middle = _targets(pp)
+    medium = pp.workloads.c1_setup(photons=1, seed=1).medium
+    src = pp.PointlikeIsotropicEmitter([middle, middle, middle - 15.0], 0.0, 20_000)
+    setup = pp.PhotonPropSetup([src], targets, medium, pp.make_monochromatic_spectrum(450.0), 5)
+    ctx = pp.Context(0)
+    setup.upload(ctx)
+
+    def run():
+        return ctx.propagate(setup.source_records(), 1, setup.seed, 15, 1.0, 20_000)
+
+    want = run()
+    assert want[1] > 0
+    with pytest.raises(pp._lib.PPError, match="too dense"):
+        ctx.set_tuning(cell_size=500.0)
+    with pytest.raises(pp._lib.PPError, match="tables are not built"):
+        run()
+    ctx.set_tuning(cell_size=0.0)
+    assert run() == want
+    ctx.close()
