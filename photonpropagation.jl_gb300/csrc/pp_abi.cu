@@ -160,6 +160,7 @@ struct pp_ctx {
   long long* d_src_photons = nullptr;
   int n_src = 0;
   unsigned long long total_chunks = 0;
+  bool mixed = false;  // groups of several sources' photons
   long long total_photons = 0;
   bool has_sources = false;
   bool needs_track = false;
@@ -222,7 +223,7 @@ int build_queue(pp_ctx* ctx, bool wait = true) {
     PP_CUDA(cudaMalloc(&ctx->d_queue, bytes), "cudaMalloc(sources)");
     ctx->queue_cap = bytes;
   }
-  // (pinning pays for small copies; a pageable one is taken before the call returns)
+  // (pinning pays for small copies; an image is not touched while queue_in_flight)
   const bool pinned = bytes <= kPinnedQueue;
   if (pinned && !ctx->h_queue)
     PP_CUDA(cudaMallocHost(&ctx->h_queue, kPinnedQueue), "cudaMallocHost(sources)");
@@ -231,7 +232,6 @@ int build_queue(pp_ctx* ctx, bool wait = true) {
   if (n > 0) memcpy(image, ctx->h_sources.data(), sizeof(pp_source) * n);
   unsigned long long* prefix = reinterpret_cast<unsigned long long*>(image + off_prefix);
   long long* nph = reinterpret_cast<long long*>(image + off_photons);
-  prefix[0] = 0;
   long long total = 0;
   for (int i = 0; i < n; ++i) {
     nph[i] = source_photons(ctx->h_sources[i].photons, ctx->scaling);
@@ -246,8 +246,7 @@ int build_queue(pp_ctx* ctx, bool wait = true) {
   const long long resident_warps = (long long)pp::kSmWarps * std::max(ctx->num_sms, 1);
   while (ppt > 2 && total / (32LL * ppt) < 2 * resident_warps) ppt /= 2;
   const long long chunk = std::max<long long>(32LL * ppt, pp::kGroup);
-  for (int i = 0; i < n; ++i)
-    prefix[i + 1] = prefix[i] + (unsigned long long)((nph[i] + chunk - 1) / chunk);
+  ctx->total_chunks = pp::make_queue(nph, n, chunk, ctx->num_sms, prefix, &ctx->mixed);
   ctx->chunk_photons = (int)chunk;
   ctx->d_sources = reinterpret_cast<pp_source*>(ctx->d_queue);
   ctx->d_prefix = reinterpret_cast<unsigned long long*>(ctx->d_queue + off_prefix);
@@ -261,7 +260,6 @@ int build_queue(pp_ctx* ctx, bool wait = true) {
     }
   }
   ctx->n_src = n;
-  ctx->total_chunks = prefix[n];
   ctx->total_photons = total;
   ctx->version++;
   return PP_OK;
@@ -349,6 +347,7 @@ LaunchArgs make_args(const pp_ctx* ctx, long long seed, int n_steps, pp_hit_reco
   a.chunk_prefix = ctx->d_prefix;
   a.src_photons = ctx->d_src_photons;
   a.total_chunks = ctx->total_chunks;
+  a.mixed = ctx->mixed;
   a.n_src = ctx->n_src;
   a.chunk_photons = ctx->chunk_photons;
   a.blob = ctx->d_blob;

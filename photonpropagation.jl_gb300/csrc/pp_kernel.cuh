@@ -626,9 +626,36 @@ __device__ __noinline__ void replay_hit(const LaunchArgs& a, int s, uint32_t plo
   out->dist = (w.dist.x - w.comp.x) + d;
 }
 
+// Photon i of source s: its number and the source.
+struct PhotonId {
+  int s;
+  uint32_t lo, hi;
+};
+// Last s in [0, n) with prefix[s] <= i.
+__device__ __forceinline__ int owner_of(const unsigned long long* __restrict__ prefix, int n,
+                                        unsigned long long i) {
+  int lo = 0, hi = n;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (__ldg(prefix + mid) <= i) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+// Photon i of all sources' photons in order (mixed groups).
+__device__ __forceinline__ PhotonId photon_of_all(const LaunchArgs& a, unsigned long long i) {
+  const int s = owner_of(a.chunk_prefix, a.n_src, i);
+  const unsigned long long p =
+      (unsigned long long)__ldg(&a.sources[s].first_photon) + (i - __ldg(a.chunk_prefix + s));
+  return {s, (uint32_t)p, (uint32_t)(p >> 32)};
+}
+
 // kShapes: shaped targets (a.shapes), every target tested at every step in
 // index order (no grid, no deferred queue).
-template <bool kPrecise, Tables kTables>
+// kMixed: the photons of all sources are numbered one after the other
+// (chunk_prefix holds photons), and a group takes 64 of them, of as many sources as they
+// come from: for workloads of many sources of few photons, which would leave most of
+// a group of one source's photons empty.
+template <bool kPrecise, Tables kTables, bool kMixed>
 __global__ void __launch_bounds__(small_ctas(kTables) ? kSmallThreads : kMaxBlockThreads,
                                   min_ctas(kTables))
     propagate_kernel(const __grid_constant__ LaunchArgs a) {
@@ -677,34 +704,35 @@ __global__ void __launch_bounds__(small_ctas(kTables) ? kSmallThreads : kMaxBloc
       stop = *reinterpret_cast<volatile unsigned*>(&a.counters->err_flags) & PP_FLAG_OVERFLOW;
     }
 
-    // Source owning chunk c: last s with chunk_prefix[s] <= c.
-    int lo = 0, hi = a.n_src;
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (__ldg(a.chunk_prefix + mid) <= c) lo = mid; else hi = mid;
-    }
-    const int s = lo;
-    const long long p0 = (long long)(c - __ldg(a.chunk_prefix + s)) * a.chunk_photons;
-    const long long pend = min(p0 + (long long)a.chunk_photons, __ldg(a.src_photons + s));
-    const long long first_photon = __ldg(&a.sources[s].first_photon);
+    // The chunk's photons, of the source that owns it or of all.
+    const int s = kMixed ? 0 : owner_of(a.chunk_prefix, a.n_src, c);
+    const long long p0 =
+        (long long)(kMixed ? c : c - __ldg(a.chunk_prefix + s)) * a.chunk_photons;
+    const long long pend =
+        min(p0 + (long long)a.chunk_photons,
+            kMixed ? (long long)__ldg(a.chunk_prefix + a.n_src) : __ldg(a.src_photons + s));
+    const long long first_photon = kMixed ? 0ll : __ldg(&a.sources[s].first_photon);
 
     int count;
     for (long long base = p0; base < pend; base += count) {
-      // A group: up to 64 photons, lane l carrying the l-th and the (32 + l)-th,
-      // all with the same high counter word.
+      // A group: up to 64 photons, lane l carrying the l-th and the (32 + l)-th; of one
+      // source, all with the same high counter word.
       const long long pb = first_photon + base;
-      count = (int)min(min(pend - base, (long long)kGroup),
-                       0x100000000ll - (long long)(uint32_t)pb);
-      const uint32_t phi = (uint32_t)((unsigned long long)pb >> 32);
+      count = (int)min(pend - base, (long long)kGroup);
+      if (!kMixed) count = (int)min((long long)count, 0x100000000ll - (long long)(uint32_t)pb);
+      auto photon = [&](int i) -> PhotonId {
+        if (kMixed) return photon_of_all(a, (unsigned long long)(pb + i));
+        return {s, (uint32_t)pb + (uint32_t)i, (uint32_t)((unsigned long long)pb >> 32)};
+      };
       const bool active0 = lane < count, active1 = lane + 32 < count;
       // Lanes past the end replay the group's first photon (never recorded).
-      const uint32_t plo0 = (uint32_t)pb + (active0 ? (uint32_t)lane : 0u);
-      const uint32_t plo1 = (uint32_t)pb + (active1 ? (uint32_t)lane + 32u : 0u);
+      const PhotonId id0 = photon(active0 ? lane : 0), id1 = photon(active1 ? lane + 32 : 0);
       Walk2 w;
       float2 sca_len;
 #pragma unroll 1
       for (int j = 0; j < 2; ++j) {
-        const PhotonInit in = init_photon<kPrecise>(a, s, j ? plo1 : plo0, phi);
+        const PhotonInit in = init_photon<kPrecise>(a, kMixed && j ? id1.s : id0.s,
+                                                    j ? id1.lo : id0.lo, kMixed && j ? id1.hi : id0.hi);
         if (j == 0) {
           w.pos.x.x = in.pos.x; w.pos.y.x = in.pos.y; w.pos.z.x = in.pos.z;
           const float3 d = on_axis(in.dir);
@@ -717,8 +745,9 @@ __global__ void __launch_bounds__(small_ctas(kTables) ? kSmallThreads : kMaxBloc
           sca_len.y = in.med.x;
         }
       }
-      const PhiloxPhoton ph0 = philox_photon(plo0, (uint32_t)s, a.round_keys);
-      const PhiloxPhoton ph1 = philox_photon(plo1, (uint32_t)s, a.round_keys);
+      const PhiloxPhoton ph0 = philox_photon(id0.lo, (uint32_t)id0.s, a.round_keys);
+      const PhiloxPhoton ph1 =
+          philox_photon(id1.lo, (uint32_t)(kMixed ? id1.s : id0.s), a.round_keys);
       w.dist = dup2(0.0f);
       w.comp = dup2(0.0f);
       q.key[lane] = 0xffffffffu;
@@ -734,9 +763,10 @@ __global__ void __launch_bounds__(small_ctas(kTables) ? kSmallThreads : kMaxBloc
       int k = 1;
       while (true) {
         for (; k <= a.n_steps && n1 < 32; ++k) {
-          const PhiloxStep pt = philox_step((uint32_t)k, phi, a.round_keys);
-          const uint4 r0 = philox_words(ph0, pt, a.round_keys);
-          const uint4 r1 = philox_words(ph1, pt, a.round_keys);
+          const PhiloxStep pt0 = philox_step((uint32_t)k, id0.hi, a.round_keys);
+          const PhiloxStep pt1 = kMixed ? philox_step((uint32_t)k, id1.hi, a.round_keys) : pt0;
+          const uint4 r0 = philox_words(ph0, pt0, a.round_keys);
+          const uint4 r1 = philox_words(ph1, pt1, a.round_keys);
           const float2 step = step_lengths<kPrecise>(r0.x, r1.x, sca_len);
           if constexpr (kShapes) {
             search_shapes<kPrecise>(a, w.pos, w.dir, step,
@@ -815,35 +845,36 @@ __global__ void __launch_bounds__(small_ctas(kTables) ? kSmallThreads : kMaxBloc
         __syncwarp();
         for (int h = lane; h < n_hit; h += 32) {
           const int own = list[h];
-          const uint32_t key = q.key[own], plo = (uint32_t)pb + (uint32_t)own;
+          const uint32_t key = q.key[own];
+          const PhotonId id = photon(own);
           const int steps_taken = (int)(key >> 16);
           Hit hit;
           if constexpr (kShapes) {
-            hit.in = init_photon<kPrecise>(a, s, plo, phi);
+            hit.in = init_photon<kPrecise>(a, id.s, id.lo, id.hi);
             hit.pos = make_float3(best.hx[own], best.hy[own], best.hz[own]);
             hit.dir = make_float3(best.ox[own], best.oy[own], best.oz[own]);
             hit.dist = best.dist[own];
           } else {
-            replay_hit<kPrecise>(a, s, plo, phi, steps_taken, sph[key & 0xffffu], &hit);
+            replay_hit<kPrecise>(a, id.s, id.lo, id.hi, steps_taken, sph[key & 0xffffu], &hit);
           }
           const float4 med = hit.in.med;
           const double time = (double)hit.in.t0 + (double)hit.dist / (double)med.y;
           const float abs_w = f_exp<kPrecise>(-f_div<kPrecise>(hit.dist, med.z));
           if (a.hist) {
             // arrival-time histogram of this source, weighted by absorption
-            const float tres = (float)(time - (double)__ldg(a.hist_tgeo + s));
+            const float tres = (float)(time - (double)__ldg(a.hist_tgeo + id.s));
             const float u = log10f(fmaxf(tres + a.hist_t_offset, 1e-30f));
             const int bin = min(max((int)floorf((u - a.hist_log_lo) * a.hist_inv_log_width), 0),
                                 a.hist_bins - 1);
-            float* row = a.hist + (size_t)s * (size_t)(a.hist_bins + 1);
+            float* row = a.hist + (size_t)id.s * (size_t)(a.hist_bins + 1);
             atomicAdd(row, abs_w);
             atomicAdd(row + 1 + bin, abs_w);
             atomicAdd(u64(&a.counters->n_hits), 1ull);
           } else {
             bool overflowed = false;
             record_hit(a, hit.pos, hit.in.wl, hit.dir, hit.dist, hit.in.dir, abs_w, time,
-                       (long long)(((unsigned long long)phi << 32) | plo),
-                       (int)(key & 0xffffu) + 1, steps_taken, s, &overflowed);
+                       (long long)(((unsigned long long)id.hi << 32) | id.lo),
+                       (int)(key & 0xffffu) + 1, steps_taken, id.s, &overflowed);
             if (overflowed) sim_acc -= 1;
           }
         }
@@ -878,18 +909,22 @@ __global__ void __launch_bounds__(small_ctas(kTables) ? kSmallThreads : kMaxBloc
   }
 }
 
-template <bool P>
-const void* kernel_ptr(Tables t) {
+template <bool P, bool kMixed>
+const void* kernel_for(Tables t) {
   switch (t) {
     case Tables::kStaged:
-      return reinterpret_cast<const void*>(&propagate_kernel<P, Tables::kStaged>);
+      return reinterpret_cast<const void*>(&propagate_kernel<P, Tables::kStaged, kMixed>);
     case Tables::kGlobal:
-      return reinterpret_cast<const void*>(&propagate_kernel<P, Tables::kGlobal>);
+      return reinterpret_cast<const void*>(&propagate_kernel<P, Tables::kGlobal, kMixed>);
     case Tables::kGlobalMany:
-      return reinterpret_cast<const void*>(&propagate_kernel<P, Tables::kGlobalMany>);
+      return reinterpret_cast<const void*>(&propagate_kernel<P, Tables::kGlobalMany, kMixed>);
     default:
-      return reinterpret_cast<const void*>(&propagate_kernel<P, Tables::kShapes>);
+      return reinterpret_cast<const void*>(&propagate_kernel<P, Tables::kShapes, kMixed>);
   }
+}
+template <bool P>
+const void* kernel_ptr(Tables t, bool mixed) {
+  return mixed ? kernel_for<P, true>(t) : kernel_for<P, false>(t);
 }
 
 }  // namespace

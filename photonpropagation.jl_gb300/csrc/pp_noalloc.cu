@@ -226,10 +226,10 @@ extern "C" PP_API int pp_propagate_static(
   };
   std::vector<unsigned long long> prefix(n_src + 1, 0);
   std::vector<long long> nph(std::max(n_src, 1), 0);
-  for (int i = 0; i < n_src; ++i) {
-    nph[i] = scaled_photons(sources[i].photons, photon_scaling);
-    prefix[i + 1] = prefix[i] + (unsigned long long)((nph[i] + chunk - 1) / chunk);
-  }
+  for (int i = 0; i < n_src; ++i) nph[i] = scaled_photons(sources[i].photons, photon_scaling);
+  bool mixed = false;
+  const unsigned long long total_chunks =
+      pp::make_queue(nph.data(), n_src, chunk, num_sms, prefix.data(), &mixed);
   std::vector<float4> table(medium->n_knots);
   for (int i = 0; i < medium->n_knots; ++i) {
     table[i] = make_float4(medium->scattering_length[i], medium->group_velocity[i],
@@ -331,7 +331,8 @@ extern "C" PP_API int pp_propagate_static(
   a.sources = d_sources;
   a.chunk_prefix = d_prefix;
   a.src_photons = d_photons;
-  a.total_chunks = prefix[n_src];
+  a.total_chunks = total_chunks;
+  a.mixed = mixed;
   a.n_src = n_src;
   a.chunk_photons = (int)chunk;
   a.blob = d_blob;

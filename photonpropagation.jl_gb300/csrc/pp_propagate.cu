@@ -10,12 +10,12 @@
 namespace pp {
 
 // Replay variant, instantiated in pp_propagate_precise.cu.
-const void* precise_kernel_ptr(Tables t);
+const void* precise_kernel_ptr(Tables t, bool mixed);
 
 namespace {
 
-const void* select_kernel(bool precise, Tables t) {
-  return precise ? precise_kernel_ptr(t) : kernel_ptr<false>(t);
+const void* select_kernel(bool precise, Tables t, bool mixed) {
+  return precise ? precise_kernel_ptr(t, mixed) : kernel_ptr<false>(t, mixed);
 }
 
 }  // namespace
@@ -32,7 +32,7 @@ cudaError_t launch_propagate(const LaunchArgs& args, int block_threads, int ctas
       : smem_grid ? Tables::kStaged
       : !fit && args.total_chunks > (unsigned long long)(kManyChunks * num_sms) ? Tables::kGlobalMany
                                                                                 : Tables::kGlobal;
-  const void* k = select_kernel(precise, t);
+  const void* k = select_kernel(precise, t, args.mixed);
   if (small_ctas(t)) {  // the same share of an SM
     ctas_per_sm = (std::min(ctas_per_sm, 32) * block_threads * min_ctas(t) + 1023) / 1024;
     block_threads = kSmallBlock;

@@ -10,6 +10,6 @@
 
 namespace pp {
 
-const void* precise_kernel_ptr(Tables t) { return kernel_ptr<true>(t); }
+const void* precise_kernel_ptr(Tables t, bool mixed) { return kernel_ptr<true>(t, mixed); }
 
 }  // namespace pp
