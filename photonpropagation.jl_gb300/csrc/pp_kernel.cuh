@@ -699,11 +699,6 @@ __global__ void __launch_bounds__(small_ctas(kTables) ? kSmallThreads : kMaxBloc
   unsigned long long next = (unsigned long long)warp * gridDim.x + blockIdx.x;
   while (next < a.total_chunks) {
     const unsigned long long c = next;
-    unsigned stop = 0;
-    if (lane == 0) {
-      stop = *reinterpret_cast<volatile unsigned*>(&a.counters->err_flags) & PP_FLAG_OVERFLOW;
-    }
-
     // The chunk's photons, of the source that owns it or of all.
     const int s = kMixed ? 0 : owner_of(a.chunk_prefix, a.n_src, c);
     const long long p0 =
@@ -882,11 +877,14 @@ __global__ void __launch_bounds__(small_ctas(kTables) ? kSmallThreads : kMaxBloc
       __syncwarp();  // the hits are read before the next group clears them
     }
     if (lane == 0) {
+      // (no more chunks once the hit buffer has overflowed)
+      const unsigned stop =
+          *reinterpret_cast<volatile unsigned*>(&a.counters->err_flags) & PP_FLAG_OVERFLOW;
       next = n_warps < a.total_chunks ? n_warps + atomicAdd(u64(&a.counters->work_next), 1ull)
                                       : a.total_chunks;
+      if (stop) next = a.total_chunks;
     }
     next = __shfl_sync(0xffffffffu, next, 0);
-    if (__shfl_sync(0xffffffffu, stop, 0)) break;
   }
 
   // One atomic per CTA for each of the photon and step counters.
