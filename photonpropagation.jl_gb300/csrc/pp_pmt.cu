@@ -95,7 +95,13 @@ __device__ __forceinline__ Rayleigh rayleigh(const pp_pom_model& m) {
   return y;
 }
 
-// The PMT (0: none) and QE weight of hit record i.
+// x a[0] + y a[1] + z a[2] with its roundings written out.
+__device__ __forceinline__ float dot3(float x, float y, float z, const float* a) {
+  return fmaf(z, a[2], fmaf(x, a[0], __fmul_rn(y, a[1])));
+}
+
+// The PMT (0: none) and QE weight of hit record i.  Every sum of products is an explicit
+// FMA, so that the kernels that inline this, and any compiler, round alike.
 __device__ __forceinline__ void detect(const PmtArgs& a, const Models& s, const Rayleigh& y,
                                        long long i, int& id, float& qe) {
   const pp_pom_model& sm = s.pom;
@@ -131,11 +137,10 @@ __device__ __forceinline__ void detect(const PmtArgs& a, const Models& s, const 
       float total = 0.0f;
 #pragma unroll
       for (int k = 0; k < kPomPmts; ++k) {
-        const float c = fminf(fmaxf(rx * m.pmt_dir[k][0] + ry * m.pmt_dir[k][1] +
-                                        rz * m.pmt_dir[k][2], -1.0f), 1.0f);
+        const float c = fminf(fmaxf(dot3(rx, ry, rz, m.pmt_dir[k]), -1.0f), 1.0f);
         const float pt = acosf(c);
         const bool g1 = m.pmt_group[k] == 1;
-        const float s = sqrtf(fmaxf(1.0f - c * c, 0.0f));  // sin(acos(c)) for pt in [0, pi]
+        const float s = sqrtf(fmaxf(fmaf(-c, c, 1.0f), 0.0f));  // sin(acos(c)) for pt in [0, pi]
         const float pdf = pt * (g1 ? inv_s2_1 : inv_s2_2) * exp2f(pt * pt * (g1 ? e2_1 : e2_2));
         // w / 8 = pdf / (s / 2) / 8 = pdf / (4 s)
         prob[k] = s != 0.0f ? __fdividef(pdf, 4.0f * s) * (g1 ? acc1 : acc2) : 0.0f;
@@ -157,7 +162,7 @@ __device__ __forceinline__ void detect(const PmtArgs& a, const Models& s, const 
       qe = interp0(m.qe_wavelength, m.qe, m.n_qe, pw.w);
     } else if (t.kind == PP_PMT_DOM && a.dom) {
       const pp_dom_model& m = sdom;
-      const float cz = dw.x * m.zenith_axis[0] + dw.y * m.zenith_axis[1] + dw.z * m.zenith_axis[2];
+      const float cz = dot3(dw.x, dw.y, dw.z, m.zenith_axis);
       float poly = 0.0f;
       for (int k = m.n_poly - 1; k >= 0; --k) poly = fmaf(poly, cz, m.poly[k]);
       const bool ang = u1 * m.polymax < poly;
@@ -168,8 +173,7 @@ __device__ __forceinline__ void detect(const PmtArgs& a, const Models& s, const 
       const pp_multipmt_model& m = smp;
       float proj = 0.0f;
       for (int k = 0; k < m.n_pmt; ++k) {
-        const float c = dw.x * m.pmt_dir_module[k][0] + dw.y * m.pmt_dir_module[k][1] +
-                        dw.z * m.pmt_dir_module[k][2];
+        const float c = dot3(dw.x, dw.y, dw.z, m.pmt_dir_module[k]);
         if (c > 0.0f) proj += c;
       }
       const float prob = proj * m.pmt_area / (3.14159265358979f * t.radius * t.radius);
@@ -180,13 +184,13 @@ __device__ __forceinline__ void detect(const PmtArgs& a, const Models& s, const 
         const float rz = (pw.z - t.position[2]) * inv_r;
         float wsum = 0.0f;
         for (int k = 0; k < m.n_pmt; ++k)
-          wsum -= rx * m.pmt_dir[k][0] + ry * m.pmt_dir[k][1] + rz * m.pmt_dir[k][2];
+          wsum -= dot3(rx, ry, rz, m.pmt_dir[k]);
         const float target = u2 * wsum;
         int j = 0;
-        float cw = -(rx * m.pmt_dir[0][0] + ry * m.pmt_dir[0][1] + rz * m.pmt_dir[0][2]);
+        float cw = -dot3(rx, ry, rz, m.pmt_dir[0]);
         while (cw < target && j < m.n_pmt - 1) {
           ++j;
-          cw -= rx * m.pmt_dir[j][0] + ry * m.pmt_dir[j][1] + rz * m.pmt_dir[j][2];
+          cw -= dot3(rx, ry, rz, m.pmt_dir[j]);
         }
         id = j + 1;
       }
@@ -221,8 +225,8 @@ __global__ void __launch_bounds__(256) pmt_kernel(const PmtArgs a) {
 // S_2max is undetected, and only the rest -- collected by each warp into full
 // passes -- take the 16 PMTs' acos, sqrt and exp2.  The decisions are those of
 // `detect`, bit for bit.  Issue bound before (1,800 instructions per 32 hits, 2.76
-// ms for 5e7); now 0.94 ms, 70% of what the 80-byte records' stream takes at the
-// measured copy bandwidth (4.4 GB: 0.66 ms).
+// ms for 5e7); now 0.76 ms, in which the 80-byte records and the results (4.4 GB) pass
+// at 87% of the measured copy bandwidth.
 constexpr int kMapSize = 64;             // cells per side
 constexpr float kNormSlack = 1e-3f;      // |rel| within 1 +- this, else no bound is used
 constexpr int kBuckets = 256;            // of a wavelength table's search
@@ -303,7 +307,8 @@ __device__ __forceinline__ int knot_from(const float* x, int n, int k, float v) 
 }
 
 // One CTA of 1024 per SM, so that the map and the models are there once and the
-// rest is L1 (5e7 hits: 0.94 ms; 2 x 512 threads 1.02, 4 x 256 1.08).
+// rest is L1 (5e7 hits, some of them off the modules' surfaces: 0.94 ms; 2 x 512
+// threads 1.02, 4 x 256 1.08).
 constexpr int kManyThreads = 1024;
 __global__ void __launch_bounds__(kManyThreads, 1)
     pmt_many_kernel(const PmtArgs a, const float4* __restrict__ place,
@@ -446,7 +451,10 @@ bool bound_applies(const pp_pom_model& m) {
          std::isfinite(m.qe_wavelength[0]) && std::isfinite(m.qe_wavelength[m.n_qe - 1]);
 }
 // Hits from which on the map's extra launch pays (3e5 hits: 54 us with it, 39
-// without; 1e6: 72 and 83).
+// without; 1e6: 72 and 83), whatever share of them POMs have: 400 modules of which one is
+// a POM and the others DOMs 155 us (152 without) for 2^20 hits, 415 (445) for 2^24,
+// multi-PMT modules 166 (162) and 562 (679), homogeneous ones 141 (142) and 361 (403); 20 POMs
+// among DOMs 153 (187) and 445 (1,072).
 constexpr long long kManyHits = 1 << 20;
 
 // A call's targets and models reach the device as kernel parameters, which a launch
