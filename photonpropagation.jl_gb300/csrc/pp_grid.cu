@@ -276,7 +276,7 @@ int build_grid_at(const pp_sphere* targets_dev, int n, const float* bb, const do
   GridDev g{};
   // Keep the cell count bounded.
   const double kMaxCells = 4.0 * 1024 * 1024;
-  for (int guard = 0; guard < 64; ++guard) {
+  for (int guard = 0; guard < 512; ++guard) {
     double cells = 1.0;
     for (int a = 0; a < 3; ++a) cells *= std::max(1.0, std::ceil(ext[a] / h));
     if (cells <= kMaxCells) break;

@@ -85,7 +85,7 @@ inline double safety_nodes(const float* blo, const float* bhi, double h) {
 }
 
 inline void SafetyDev::set_shape(const float* blo, const float* bhi, double h) {
-  for (int guard = 0; guard < 64 && safety_nodes(blo, bhi, h) > 8.0e6; ++guard) h *= 1.25;
+  for (int guard = 0; guard < 512 && safety_nodes(blo, bhi, h) > 8.0e6; ++guard) h *= 1.25;
   n_cells = 1;
   for (int a = 0; a < 3; ++a) {
     dims[a] = (int)std::ceil(std::max(1e-6, (double)bhi[a] - (double)blo[a]) / h) + 1;

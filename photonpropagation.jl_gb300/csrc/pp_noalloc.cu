@@ -125,7 +125,7 @@ void grid_shape(const pp_sphere* t, int n, float cell_size, double cells_per_tar
   }
   double h = cell_size;
   if (!(h > 0.0)) h = std::cbrt(vol / (cells_per_target * n));
-  for (int guard = 0; guard < 64; ++guard) {
+  for (int guard = 0; guard < 512; ++guard) {
     double cells = 1.0;
     for (int a = 0; a < 3; ++a) cells *= std::max(1.0, std::ceil(ext[a] / h));
     if (cells <= 4.0 * 1024 * 1024) break;
