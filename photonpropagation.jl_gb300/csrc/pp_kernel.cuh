@@ -709,6 +709,13 @@ __global__ void __launch_bounds__(small_ctas(kTables) ? kSmallThreads : kMaxBloc
     const long long first_photon = kMixed ? 0ll : __ldg(&a.sources[s].first_photon);
 
     int count;
+    // A full hit buffer: a warp whose hits it did not take stops after this chunk, and so
+    // does one that finds the flag now.  (Asking at the chunk's end, or at each group,
+    // makes every warp wait for the counters' busy line: 13.08 -> 13.14 ms per 1e8.)
+    bool full = false;
+    unsigned stop = 0;
+    if (lane == 0)
+      stop = *reinterpret_cast<volatile unsigned*>(&a.counters->err_flags) & PP_FLAG_OVERFLOW;
     for (long long base = p0; base < pend; base += count) {
       // A group: up to 64 photons, lane l carrying the l-th and the (32 + l)-th; of one
       // source, all with the same high counter word.
@@ -870,21 +877,22 @@ __global__ void __launch_bounds__(small_ctas(kTables) ? kSmallThreads : kMaxBloc
             record_hit(a, hit.pos, hit.in.wl, hit.dir, hit.dist, hit.in.dir, abs_w, time,
                        (long long)(((unsigned long long)id.hi << 32) | id.lo),
                        (int)(key & 0xffffu) + 1, steps_taken, id.s, &overflowed);
-            if (overflowed) sim_acc -= 1;
+            if (overflowed) {
+              sim_acc -= 1;
+              full = true;
+            }
           }
         }
       }
       __syncwarp();  // the hits are read before the next group clears them
     }
     if (lane == 0) {
-      // (no more chunks once the hit buffer has overflowed)
-      const unsigned stop =
-          *reinterpret_cast<volatile unsigned*>(&a.counters->err_flags) & PP_FLAG_OVERFLOW;
       next = n_warps < a.total_chunks ? n_warps + atomicAdd(u64(&a.counters->work_next), 1ull)
                                       : a.total_chunks;
       if (stop) next = a.total_chunks;
     }
     next = __shfl_sync(0xffffffffu, next, 0);
+    if (__any_sync(0xffffffffu, full)) break;
   }
 
   // One atomic per CTA for each of the photon and step counters.
