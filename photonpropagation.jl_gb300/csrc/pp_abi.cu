@@ -148,10 +148,14 @@ struct pp_ctx {
   std::vector<pp_source> h_sources;
   float scaling = 1.0f;
   bool field_staged = true;  // stages_auto_field when the field was built
-  // one device buffer {sources, prefix, photons} and its host image (pinned when
-  // small), uploaded in one copy
+  // host memory of the images below: pageable, then pinned (need_image)
+  std::vector<unsigned char> h_pageable;
+  unsigned char* h_pinned = nullptr;
+  unsigned char* h_image = nullptr;
+  int image_uses = 0;
+  // one device buffer {sources, prefix, photons}, uploaded in one copy from its host
+  // image (a large one has its own)
   unsigned char* d_queue = nullptr;
-  unsigned char* h_queue = nullptr;
   std::vector<unsigned char> h_queue_big;
   size_t queue_cap = 0;
   bool queue_in_flight = false;  // the image may still be being read
@@ -167,14 +171,13 @@ struct pp_ctx {
 
   pp_tuning tuning{1024, 8, 0, 0, 0.0f, 0, 0.0f, 0};
 
-  // scratch of pp_propagate: one device buffer {counters, hits} and a pinned
-  // host image of its first rows
+  // scratch of pp_propagate: one device buffer {counters, hits} and a host image of
+  // its first rows
   unsigned char* d_result = nullptr;
   pp_hit_record* d_hits = nullptr;
   long long d_hits_cap = 0;
   pp_counters* d_ctr = nullptr;
-  unsigned char* h_result = nullptr;
-  long long h_rows = 0;  // hit rows of the last pp_propagate in h_result
+  long long h_rows = 0;  // hit rows of the last pp_propagate in its host image
   pp_hit_record* h_stage = nullptr;
   long long h_stage_cap = 0;
 
@@ -191,7 +194,29 @@ namespace {
 // call's hits all come with them, saving it a second round trip.
 constexpr size_t kHitsOffset = 128;  // of the hits in the result buffer
 constexpr long long kFirstRows = 256;
-constexpr size_t kPinnedQueue = 256 * 1024;
+constexpr size_t kResultImage = kHitsOffset + sizeof(pp_hit_record) * kFirstRows;
+constexpr size_t kQueueImage = 256 * 1024;
+// Pinned copies save a call 2 us of 42, and pinning takes a context 310 us: contexts in
+// steady use only.
+constexpr int kPinFrom = 64;
+
+// The host memory of a result's image, then a queue's.
+void need_image(pp_ctx* ctx) {
+  if (ctx->h_pinned) return;
+  if (++ctx->image_uses >= kPinFrom) {
+    if (cudaMallocHost(&ctx->h_pinned, kResultImage + kQueueImage) == cudaSuccess) {
+      ctx->h_image = ctx->h_pinned;
+      ctx->h_rows = 0;  // the last result's image is gone
+    } else {
+      cudaGetLastError();
+      ctx->h_pinned = nullptr;
+    }
+  }
+  if (!ctx->h_image) {
+    ctx->h_pageable.resize(kResultImage + kQueueImage);
+    ctx->h_image = ctx->h_pageable.data();
+  }
+}
 
 // Waits for an upload that is still in flight: launches on other streams are not
 // ordered after it.
@@ -223,12 +248,11 @@ int build_queue(pp_ctx* ctx, bool wait = true) {
     PP_CUDA(cudaMalloc(&ctx->d_queue, bytes), "cudaMalloc(sources)");
     ctx->queue_cap = bytes;
   }
-  // (pinning pays for small copies; an image is not touched while queue_in_flight)
-  const bool pinned = bytes <= kPinnedQueue;
-  if (pinned && !ctx->h_queue)
-    PP_CUDA(cudaMallocHost(&ctx->h_queue, kPinnedQueue), "cudaMallocHost(sources)");
-  if (!pinned) ctx->h_queue_big.resize(bytes);
-  unsigned char* image = pinned ? ctx->h_queue : ctx->h_queue_big.data();
+  // (an image is not touched while queue_in_flight)
+  const bool small = bytes <= kQueueImage;
+  if (small) need_image(ctx);
+  else ctx->h_queue_big.resize(bytes);
+  unsigned char* image = small ? ctx->h_image + kResultImage : ctx->h_queue_big.data();
   if (n > 0) memcpy(image, ctx->h_sources.data(), sizeof(pp_source) * n);
   unsigned long long* prefix = reinterpret_cast<unsigned long long*>(image + off_prefix);
   long long* nph = reinterpret_cast<long long*>(image + off_photons);
@@ -448,8 +472,6 @@ PP_API int pp_create(pp_ctx** out, int32_t device) {
   e = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->inflight, cudaEventDisableTiming);
-  if (e == cudaSuccess)
-    e = cudaMallocHost(&ctx->h_result, kHitsOffset + sizeof(pp_hit_record) * kFirstRows);
   if (e != cudaSuccess) {
     int rc = cuda_error(e, "pp_create");
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -477,9 +499,8 @@ PP_API int pp_destroy(pp_ctx* ctx) {
   cudaFree(ctx->d_blob);
   cudaFree(ctx->d_safety);
   cudaFree(ctx->d_queue);
-  if (ctx->h_queue) cudaFreeHost(ctx->h_queue);
+  if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
   cudaFree(ctx->d_result);
-  if (ctx->h_result) cudaFreeHost(ctx->h_result);
   if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->inflight) cudaEventDestroy(ctx->inflight);
@@ -933,6 +954,7 @@ PP_API int pp_propagate(pp_ctx* ctx, const pp_source* sources, int32_t n_src, in
   int rc = set_sources(ctx, sources, n_src, photon_scaling, false);
   if (rc == PP_OK) rc = check_ready(ctx);
   if (rc != PP_OK) return rc;
+  if (!ctx->h_image) need_image(ctx);
   // A photon hits at most once: the device buffer never needs more rows than
   // there are photons.
   const long long dev_cap = std::max<long long>(1, std::min<long long>(capacity, ctx->total_photons));
@@ -950,14 +972,14 @@ PP_API int pp_propagate(pp_ctx* ctx, const pp_source* sources, int32_t n_src, in
                ctx->stream);
   if (rc != PP_OK) return rc;
   const long long first = std::min<long long>(kFirstRows, ctx->d_hits_cap);
-  PP_CUDA(cudaMemcpyAsync(ctx->h_result, ctx->d_result,
+  PP_CUDA(cudaMemcpyAsync(ctx->h_image, ctx->d_result,
                           kHitsOffset + sizeof(pp_hit_record) * (size_t)first,
                           cudaMemcpyDeviceToHost, ctx->stream),
           "read counters");
   PP_CUDA(cudaStreamSynchronize(ctx->stream), "propagate");
   ctx->queue_in_flight = false;
   pp_counters c;
-  memcpy(&c, ctx->h_result, sizeof(c));
+  memcpy(&c, ctx->h_image, sizeof(c));
   *n_hits = (int64_t)c.n_hits;
   *n_ph_sim = (int64_t)c.n_ph_sim;
   if (c.err_flags & PP_FLAG_TIMEOUT)
@@ -1011,7 +1033,7 @@ int fetch_hits(pp_ctx* ctx, const pp_hits* out, long long n) {
     if (e != cudaSuccess) return cuda_error(e, "hits_to_columns");
     return PP_OK;
   }
-  const pp_hit_record* rows = reinterpret_cast<const pp_hit_record*>(ctx->h_result + kHitsOffset);
+  const pp_hit_record* rows = reinterpret_cast<const pp_hit_record*>(ctx->h_image + kHitsOffset);
   if (n > ctx->h_rows) {
     if (n > ctx->h_stage_cap) {
       if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
