@@ -120,7 +120,7 @@ inline double SafetyDev::auto_cell(const float* blo, const float* bhi, int n, bo
 // block_threads counts 1024 for all the warps an SM holds: that many, or the
 // same share of them, make a CTA.
 constexpr int kGroup = 64;     // photons a warp carries at a time
-// (16 warps of 104 registers: 24 of 80 issue 73% of the time against 68%, but
+// (16 warps of 128 registers: 24 of 80 issue 73% of the time against 68%, but
 // spill, and both take 13.6 ms per 1e8 photons; the FMA and ALU pipes bound both.)
 constexpr int kSmWarps = 16;
 constexpr int kMaxBlockThreads = 32 * kSmWarps;

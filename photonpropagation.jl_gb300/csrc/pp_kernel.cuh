@@ -10,16 +10,17 @@
 // (:927-943).  Design:
 //   * persistent CTAs; every warp pulls chunks of photons of one source from a
 //     device work queue, so one launch covers any number of sources with
-//     uneven photon counts;
+//     uneven photon counts, and sources of few photons share groups (kMixed);
 //   * photon i of source s draws its random numbers from Philox4x32-10 at
 //     counter (i, call, s) and key = seed: results do not depend on the launch
 //     shape and any photon range can be replayed;
 //   * two photons per lane.  The kernel is bound by instruction issue, and the
 //     packed f32x2 instructions do the two photons' sums and products in one
 //     issue slot; the 64 photons of a warp also fill its clip and walk passes
-//     twice as well.  16 warps of 104 registers replace 32 of 64: per photon step
+//     twice as well.  16 warps of 128 registers replace 32 of 64: per photon step
 //     8.7 warp instructions instead of 11.4 (1e8 photons, 400 modules: 16.66 ->
-//     15.75 ms; 256 emitters 5.51 -> 4.97; histogram tables 6.22 -> 5.37);
+//     15.75 ms; 256 emitters 5.51 -> 4.97; histogram tables 6.22 -> 5.37).  Tables too
+//     large for shared memory take 32 warps all the same (Tables);
 //   * speculative stepping with deferred hit tests.  Each lane runs all
 //     n_steps of its photons without waiting for the target test.  A step
 //     segment is cleared cheaply when the safety field proves that no target
@@ -32,7 +33,7 @@
 //     part only.  A photon's hit is the earliest step with an intersection
 //     and, within it, the lowest target index -- the reference's "first
 //     target in index order" (:497-506).  Steps after the hit were computed
-//     speculatively and are discarded;
+//     speculatively and are discarded, and not tested once the hit is known;
 //   * the target grid (cells, candidate lists, spheres) is staged once per CTA
 //     into shared memory with a TMA bulk copy completing on an mbarrier, waited
 //     on with a time bound;

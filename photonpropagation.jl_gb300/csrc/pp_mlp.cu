@@ -1447,9 +1447,9 @@ int check_err(pp_mlp* m, cudaStream_t s) {
 
 // ---- the three-kernel training step --------------------------------------------
 
-// The shapes rows_kernel takes: hidden widths that split into two halves of whole
-// 64-column chunks, one chunk of inputs, four 8-column blocks of outputs per
-// thread of the loss.  Others train layer by layer.
+// The shapes the step takes: hidden widths of whole 128-column tiles of dw_kernel (a
+// template parameter of rows_kernel), one chunk of inputs, four 8-column blocks of
+// outputs per thread of the loss.  Others train layer by layer.
 void rows_setup(pp_mlp* m) {
   m->rows_path = (m->hidden == 128 || m->hidden == 256) && m->in_pad <= pprows::kChunk &&
                  m->out_pad <= 128;

@@ -194,11 +194,11 @@ __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v 
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 
 // One CTA takes 64 rows of the batch through the forward pass, the loss and the
-// backward pass through the activations.  Two warps stream the weights into
-// slots of 32 KB, one thread issues the MMAs and stores the operands that
-// dw_kernel needs, 16 warps do the epilogues; two accumulators and two activation buffers alternate, and each
-// 64-column chunk of a layer's input starts its MMAs when its epilogue is done, so
-// that all but a layer's last chunk run under the epilogue before them.  Bound: the
+// backward pass through the activations.  One warp streams the weights into
+// slots of 32 KB, one issues the MMAs and stores the operands that dw_kernel needs,
+// 16 do the epilogues; two accumulators and two activation buffers alternate, and
+// each 64-column chunk of a layer's input starts its MMAs when its epilogue is done,
+// so that all but a layer's last chunk run under the epilogue before them.  Bound: the
 // serial chain of 2 L + 1 products, epilogue and MMA latency: 25 us for 4 x 256, at
 // batch 1024 (16 CTAs) as at 8192 (128).  With 128 rows per CTA, halves of a layer
 // and one thread's waits between the MMAs it took 40 us, on 64 SMs.
