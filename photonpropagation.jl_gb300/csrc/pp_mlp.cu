@@ -1503,6 +1503,13 @@ void forward_tiles(pp_mlp* m) {
   m->O = reinterpret_cast<float*>(m->tiles + t.total);
 }
 
+// A batch of up to this many rows is not split over CTAs: its weight gradients are then
+// sums in one order.  (Where it changes from run to run, an ulp of a gradient can turn the
+// rounding of a BF16 weight: after 11 steps of 256 rows, split four ways, two runs in ten
+// had over 1% of their parameters apart by more than 1e-6; now none differ by 2e-9.
+// The step takes as long.)
+constexpr int kUnsplitRows = 256;
+
 // Forward, loss and all gradients of a batch into m->G and m->loss_acc (which
 // are zero before): rows 0 .. B - 1 of the arrays, or B rows drawn from n_table.
 // `schedule`: also the captured step's step size.
@@ -1549,7 +1556,9 @@ int rows_gradients(pp_mlp* m, const float* x, const float* count, const float* h
       }
   }
   d.n_blocks = (int)grid.x;
-  const int splits = std::max(1, std::min(d.n_blocks, m->num_sms / d.n_tiles));
+  const int splits = d.n_blocks * pprows::kRows <= kUnsplitRows
+                         ? 1
+                         : std::max(1, std::min(d.n_blocks, m->num_sms / d.n_tiles));
   d.blocks_per_split = (d.n_blocks + splits - 1) / splits;
   d.err = m->err; d.wait_ns = kWaitNs;
   d.sched = schedule ? m->d_sched : nullptr; d.ctl = m->ctl; d.b1 = m->b1; d.b2 = m->b2;
