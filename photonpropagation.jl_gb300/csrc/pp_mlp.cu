@@ -1505,9 +1505,9 @@ void forward_tiles(pp_mlp* m) {
 
 // A batch of up to this many rows is not split over CTAs: its weight gradients are then
 // sums in one order.  (Where it changes from run to run, an ulp of a gradient can turn the
-// rounding of a BF16 weight: after 11 steps of 256 rows, split four ways, two runs in ten
-// had over 1% of their parameters apart by more than 1e-6; now none differ by 2e-9.
-// The step takes as long.)
+// rounding of a BF16 weight: after 11 steps of 256 rows, split four ways, one pair of runs
+// in eight had over 1% of their parameters apart by more than 1e-6; now none differ by
+// more than 2e-9.  The step takes as long.)
 constexpr int kUnsplitRows = 256;
 
 // Forward, loss and all gradients of a batch into m->G and m->loss_acc (which
