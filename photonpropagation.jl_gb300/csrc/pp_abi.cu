@@ -196,9 +196,9 @@ constexpr size_t kHitsOffset = 128;  // of the hits in the result buffer
 constexpr long long kFirstRows = 256;
 constexpr size_t kResultImage = kHitsOffset + sizeof(pp_hit_record) * kFirstRows;
 constexpr size_t kQueueImage = 256 * 1024;
-// Pinned copies save a call 2 us of 42, and pinning takes a context 310 us: contexts in
-// steady use only.
-constexpr int kPinFrom = 64;
+// Pinned copies save a call 2 us of 42, and pinning takes a context 310 us, a quarter of
+// its creation, tables and first launch: not for contexts of a few uploads.
+constexpr int kPinFrom = 4;
 
 // The host memory of a result's image, then a queue's.
 void need_image(pp_ctx* ctx) {

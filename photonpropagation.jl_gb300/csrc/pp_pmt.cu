@@ -30,8 +30,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <string>
-#include <vector>
 
 #include "pp_device.cuh"
 #include "pp_internal.h"
@@ -461,7 +461,7 @@ constexpr long long kManyHits = 1 << 20;
 // takes when it is made: the caller's structures, and the image they are gathered
 // in, are free when the call returns, also under stream capture and where a copy
 // from pageable memory is asynchronous.
-constexpr int kSmallImage = 250, kLargeImage = 2040;  // 16-byte words a launch carries
+constexpr int kImageWords[] = {250, 1020, 2040};  // 16-byte words that a launch carries
 template <int kWords>
 struct ImagePart {
   uint4 w[kWords];
@@ -472,23 +472,27 @@ __global__ void __launch_bounds__(256)
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dst[i] = part.w[i];
 }
-// Room for `bytes` and, after them, for what a launch reads past the last part.
-std::vector<unsigned char> host_image(size_t bytes) {
-  return std::vector<unsigned char>(bytes + sizeof(ImagePart<kLargeImage>));
+// Room for `bytes` (zeros) and, after them, for what a launch reads past the last part.
+using HostImage = std::unique_ptr<unsigned char[]>;
+HostImage host_image(size_t bytes) {
+  HostImage image(new unsigned char[bytes + sizeof(ImagePart<kImageWords[2]>)]);
+  memset(image.get(), 0, bytes);
+  return image;
 }
-// The first `bytes` (a multiple of 16) of a host_image to device memory.
-cudaError_t write_image(void* dst, std::vector<unsigned char>& image, size_t bytes,
-                        cudaStream_t s) {
+// The first `bytes` (a multiple of 16) of a host_image to device memory, in launches of
+// the smallest size that holds what is left.  (400 mixed modules, 15 KB: one of 16 KB.)
+cudaError_t write_image(void* dst, const HostImage& image, size_t bytes, cudaStream_t s) {
+  const void* kernels[] = {(const void*)write_kernel<kImageWords[0]>,
+                           (const void*)write_kernel<kImageWords[1]>,
+                           (const void*)write_kernel<kImageWords[2]>};
   cudaError_t e = cudaSuccess;
-  size_t words = bytes / 16, at = 0;
-  while (e == cudaSuccess && at < words) {
-    const bool small = words - at <= (size_t)kSmallImage;
-    int n = (int)std::min<size_t>(words - at, small ? kSmallImage : kLargeImage);
+  for (size_t words = bytes / 16, at = 0; e == cudaSuccess && at < words;) {
+    int size = 0;
+    while (size < 2 && words - at > (size_t)kImageWords[size]) ++size;
+    int n = (int)std::min<size_t>(words - at, kImageWords[size]);
     uint4* to = static_cast<uint4*>(dst) + at;
-    void* params[] = {&to, image.data() + 16 * at, &n};
-    e = cudaLaunchKernel(small ? (const void*)write_kernel<kSmallImage>
-                               : (const void*)write_kernel<kLargeImage>,
-                         dim3((unsigned)((n + 255) / 256)), dim3(256), params, 0, s);
+    void* params[] = {&to, image.get() + 16 * at, &n};
+    e = cudaLaunchKernel(kernels[size], dim3((unsigned)((n + 255) / 256)), dim3(256), params, 0, s);
     at += n;
   }
   return e;
@@ -574,13 +578,13 @@ PP_API int pp_make_hits_from_photons_models(const pp_hit_record* d_records, int6
   const bool many = pom && n >= kManyHits && bound_applies(*pom);
   const size_t total = ob_place + (many ? sizeof(float4) * (size_t)n_targets : 0);
   const size_t alloc = total + (many ? sizeof(float2) * kMapSize * kMapSize : 0);
-  std::vector<unsigned char> image = host_image(total);
-  if (n_targets > 0) memcpy(image.data(), targets, sizeof(pp_pmt_target) * n_targets);
-  if (pom) memcpy(image.data() + ob_pom, pom, sizeof(pp_pom_model));
-  if (dom) memcpy(image.data() + ob_dom, dom, sizeof(pp_dom_model));
-  if (mp) memcpy(image.data() + ob_mp, mp, sizeof(pp_multipmt_model));
+  const HostImage image = host_image(total);
+  if (n_targets > 0) memcpy(image.get(), targets, sizeof(pp_pmt_target) * n_targets);
+  if (pom) memcpy(image.get() + ob_pom, pom, sizeof(pp_pom_model));
+  if (dom) memcpy(image.get() + ob_dom, dom, sizeof(pp_dom_model));
+  if (mp) memcpy(image.get() + ob_mp, mp, sizeof(pp_multipmt_model));
   if (many) {  // centre and 1 / radius of the POMs, 0 for the others
-    float4* place = reinterpret_cast<float4*>(image.data() + ob_place);
+    float4* place = reinterpret_cast<float4*>(image.get() + ob_place);
     for (int i = 0; i < n_targets; ++i)
       place[i] = make_float4(targets[i].position[0], targets[i].position[1],
                              targets[i].position[2],
